@@ -1036,24 +1036,38 @@ void append_reserve(Instance& I, Binding& b, Tensor& past, const AppendPlan& ap)
     const bool ours = b.store.ptr && past.data == b.store.ptr && b.cap >= ap.tp;  // the view handed out by the previous run
     if (past.lazy && !ours) I.materialize(past);
     if (!(ours && b.cap >= ap.total)) {
-        // first run, a cache fed from outside, or out of room: move to a larger buffer (old rows copied once)
-        const int64_t ncap = ap.total + std::max<int64_t>(64, ap.total / 2);
-        void* np = nullptr;
-        check_cuda(cudaMalloc(&np, std::max<size_t>(static_cast<size_t>(ap.outer) * ncap * ap.row, 256)), "cache cudaMalloc");
+        // A cache fed from outside (a new sequence, a prompt's cache kept by the caller), the first run, or out of room.
+        // The buffer an earlier sequence left behind is taken over when it is large enough: everything that still reads
+        // it was enqueued before on the same stream.  Allocating one per sequence instead costs an allocation, a wait for
+        // the stream and a free per cache tensor - 57 ms instead of 27 ms for 16 one-request steps behind a fed cache.
+        const char* base = static_cast<const char*>(b.store.ptr);
+        const char* src = static_cast<const char*>(past.data);
+        const bool inside = base && src >= base && src < base + b.store.cap;  // rows that would be overwritten while they move
+        const size_t per_entry = static_cast<size_t>(ap.outer) * ap.row;
+        void* np = b.store.ptr;
+        int64_t ncap = static_cast<int64_t>(b.store.cap / per_entry);
+        const bool reuse = base && !inside && ncap >= ap.total;
+        if (!reuse) {
+            ncap = ap.total + std::max<int64_t>(64, ap.total / 2);
+            np = nullptr;
+            check_cuda(cudaMalloc(&np, std::max<size_t>(per_entry * ncap, 256)), "cache cudaMalloc");
+        }
         if (ap.tp > 0) {
             const size_t spitch = (ours ? static_cast<size_t>(b.cap) : static_cast<size_t>(ap.tp)) * ap.row;
             check_cuda(cudaMemcpy2DAsync(np, static_cast<size_t>(ncap) * ap.row, past.data, spitch, static_cast<size_t>(ap.tp) * ap.row,
                                          static_cast<size_t>(ap.outer), cudaMemcpyDeviceToDevice, I.stream), "cache move");
             I.launches++;
         }
-        if (b.store.ptr) {
-            check_cuda(cudaStreamSynchronize(I.stream), "cudaStreamSynchronize");  // the old buffer is still being read
-            cudaFree(b.store.ptr);
+        if (!reuse) {
+            if (b.store.ptr) {
+                check_cuda(cudaStreamSynchronize(I.stream), "cudaStreamSynchronize");  // the old buffer is still being read
+                cudaFree(b.store.ptr);
+            }
+            b.store.ptr = np;
+            b.store.cap = std::max<size_t>(per_entry * ncap, 256);
         }
-        b.store.ptr = np;
-        b.store.cap = static_cast<size_t>(ap.outer) * ncap * ap.row;
         b.cap = ncap;
-        // the old rows now live in the new buffer: later readers of `past` must not follow the freed pointer
+        // the old rows now live in the binding's buffer: later readers of `past` must not follow the freed pointer
         if (past.storage == nullptr) set_strided(past, np, past.shape, cache_strides(ap, past.shape, ncap));
     }
     b.reserved_run = I.run_counter;
