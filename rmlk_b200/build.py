@@ -31,7 +31,7 @@ def _sources():
 
 
 def _headers():
-    return (glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "runtime", "*.h")) +
+    return (glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.h")) + glob.glob(os.path.join(CSRC, "runtime", "*.h")) +
             glob.glob(os.path.join(INCLUDE, "*.h")))
 
 

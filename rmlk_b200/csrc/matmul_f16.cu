@@ -1,10 +1,11 @@
 // f16 MatMul: C[b] = A[b] x B[b], row-major, half in and out, products accumulated in fp32 and rounded to f16 once.
 // The reference runs cublasGemmStridedBatchedEx with CUBLAS_COMPUTE_16F for f16 (cuda/src/params.rs:24-31,
 // cuda/src/kernels/gemm.rs:206-231): same operands and result type, half-precision accumulation; this kernel's sums
-// are at least as accurate.  Shared-memory tiled SIMT kernel (64 x 64 x 16, 256 threads, 4 x 4 micro-tiles, guarded
-// edges, any M / N / K, batch strides may be 0 to broadcast an operand).  The benchmark path is fp32; a tensor-core
-// kind::f16 kernel is not built.
+// are at least as accurate.  A single product whose rows lie on 16-byte boundaries (N and K multiples of 8: what TMA can
+// fetch) runs on the tensor cores (umma_gemm.cu); what is left - batches and ragged rows - on the kernel here: shared-memory
+// tiled SIMT (64 x 64 x 16, 256 threads, 4 x 4 micro-tiles, guarded edges, any M / N / K, batch strides may be 0).
 #include "common.cuh"
+#include "umma_gemm.h"
 
 namespace rmlk {
 
@@ -66,12 +67,13 @@ __global__ void __launch_bounds__(256) gemm_f16_kernel(const __half* __restrict_
 }
 
 int matmul_f16(cudaStream_t st, int64_t batch, int64_t m, int64_t n, int64_t k, const void* a, int64_t sa, const void* b, int64_t sb, void* c,
-               int64_t sc) {
+               int64_t sc, int* status) {
     if (k == 0) {
         for (int64_t bi = 0; bi < batch; bi++)
             RMLK_CUDA(cudaMemsetAsync(static_cast<__half*>(c) + bi * sc, 0, static_cast<size_t>(m) * n * sizeof(__half), st));
         return RMLK_OK;
     }
+    if (batch == 1 && umma_f16_eligible(m, n, k, a, b)) return umma_f16(st, m, n, k, a, b, c, status);
     const int64_t gx = ceil_div64(n, HF_BN), gy = ceil_div64(m, HF_BM);
     if (gx > 0x7fffffffll || gy > 65535 || batch > 65535) return fail(RMLK_ERR_INVALID_ARG, "matmul f16: extent too large");
     launch_dep(gemm_f16_kernel, dim3(static_cast<unsigned>(gx), static_cast<unsigned>(gy), static_cast<unsigned>(batch)), dim3(256), 0, st,

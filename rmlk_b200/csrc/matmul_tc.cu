@@ -43,15 +43,12 @@
 #include <mutex>
 
 #include "matmul_tc_kernel.cuh"
+#include "umma_gemm.h"
 
 namespace rmlk {
 namespace tc {
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static EncodeTiledFn encode_fn() {
+EncodeTiledFn encode_fn() {
     // looked up once per process (function-local static: initialised exactly once, also under concurrent first calls)
     static const EncodeTiledFn fn = [] {
         void* p = nullptr;

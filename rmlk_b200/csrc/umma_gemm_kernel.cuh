@@ -1,0 +1,315 @@
+// gemm_kernel: out[m][n] = sum_k X[m][k] W[k][n] on tcgen05.mma kind::f16.
+#pragma once
+
+#include "umma_gemm.cuh"
+
+namespace rmlk {
+namespace umma {
+
+__device__ __forceinline__ void tmem_ld_x16(uint32_t taddr, uint32_t* r) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
+          "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_ld_x8(uint32_t taddr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
+}
+template <int W>
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t* r) {
+    if constexpr (W == 32) {
+        tmem_ld_x16(taddr, r);
+        tmem_ld_x16(taddr + 16, r + 16);
+    } else if constexpr (W == 16) {
+        tmem_ld_x16(taddr, r);
+    } else {
+        static_assert(W == 8, "");
+        tmem_ld_x8(taddr, r);
+    }
+}
+
+struct Item {
+    int n_tile, m_tile, split;
+};
+// Tile order: passes over all column tiles with `m_group` row tiles each, so that concurrently running tiles share weights and
+// activations in L2; the K splits of a tile come one after the other.
+__device__ __forceinline__ Item item_at(int w, const Params& p) {
+    Item it;
+    it.split = w % p.ksplit;
+    const int t = w / p.ksplit;
+    const int per_pass = p.m_group * p.n_tiles;
+    const int pass = t / per_pass, r = t - pass * per_pass;
+    const int m_first = pass * p.m_group;
+    const int rows = min(p.m_group, p.m_tiles - m_first);
+    it.n_tile = r / rows;
+    it.m_tile = m_first + r - it.n_tile * rows;
+    return it;
+}
+
+template <int CG, bool SPLIT, int MT, int ST, bool OUT16>
+__global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, Params p) {
+    using L = Layout<CG, SPLIT, MT, ST>;
+    dep_trigger();
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
+    const uint32_t bars = base + L::BAR_OFFSET;
+    auto full = [&](int s) { return bars + 8u * s; };
+    auto empty = [&](int s) { return bars + 8u * (ST + s); };
+    auto acc_full = [&](int b) { return bars + 8u * (2 * ST + b); };
+    auto acc_empty = [&](int b) { return bars + 8u * (2 * ST + L::NBUF + b); };
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(base_ptr + L::BAR_OFFSET + 8 * L::N_BARS);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(base_ptr + L::BAR_OFFSET + 8 * L::N_BARS + 8);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = CG == 2 ? cluster_ctarank() : 0;
+    const int first = CG == 2 ? blockIdx.x >> 1 : blockIdx.x, stride = CG == 2 ? gridDim.x >> 1 : gridDim.x;
+    const int items = p.n_tiles * p.m_tiles * p.ksplit;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < ST; s++) {
+            mbar_init(full(s), 1);
+            mbar_init(empty(s), 1);
+        }
+        for (int b = 0; b < L::NBUF; b++) {
+            mbar_init(acc_full(b), 1);
+            mbar_init(acc_empty(b), CG * EPI_WARPS);
+        }
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        if constexpr (CG == 1) {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(L::TMEM_COLS) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(L::TMEM_COLS) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        }
+    }
+    tc_fence_before();
+    if constexpr (CG == 2) cluster_sync_all();  // the pair's barriers exist and both have their TMEM
+    else __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp == 0) {
+        // ---------------- loads ----------------
+        if (lane == 0) {
+            const uint32_t pair_bar = CG == 2 ? mapa_shared(bars, 0) : bars;  // the pair's full barriers live in its first CTA
+            bool waited = false;
+            if (!p.w_static) {
+                dep_wait();
+                waited = true;
+            }
+            auto load_w = [&](int s, int n_tile, int kb) {
+                const uint32_t dst = base + s * L::STAGE, bar = pair_bar + 8u * s;
+                const int nb = n_tile * CG + static_cast<int>(rank);  // block of 128 columns
+                if constexpr (SPLIT) {  // packed: the high and the low tile of a block lie behind one another
+                    load_2d<CG>(dst, &tmW, 0, nb * p.w_rows_per_tile + kb * 256, bar);
+                } else {
+                    load_2d<CG>(dst, &tmW, nb * BN, kb * BK, bar);
+                    load_2d<CG>(dst + 8192, &tmW, nb * BN + 64, kb * BK, bar);
+                }
+            };
+            auto load_x = [&](int s, int m_tile, int kb) {
+                const uint32_t dst = base + s * L::STAGE + L::W_BYTES, bar = pair_bar + 8u * s;
+                const int row = m_tile * MT + static_cast<int>(rank) * L::XR;
+                load_2d<CG>(dst, &tmX, kb * BK, row, bar);
+                if constexpr (SPLIT) load_2d<CG>(dst + L::X_TILE, &tmX, kb * BK, row + p.x_lo_row, bar);
+            };
+            // The weights of the first stages do not depend on the kernel before this one: they are requested while it still
+            // runs (this grid may have been scheduled early), the activations behind its end.
+            int early = 0;
+            if (!waited && first < items) {
+                const Item it = item_at(first, p);
+                const int kb0 = it.split * p.k_per_split, nk = min(p.k_per_split, p.k_blocks - kb0);
+                early = min(ST, nk);
+                for (int s = 0; s < early; s++) {
+                    if (rank == 0) mbar_expect_tx(full(s), CG * L::STAGE);
+                    load_w(s, it.n_tile, kb0 + s);
+                }
+                dep_wait();
+                for (int s = 0; s < early; s++) load_x(s, it.m_tile, kb0 + s);
+            } else if (!waited) {
+                dep_wait();
+            }
+            int s = 0, done = 0;
+            uint32_t phase = 0;
+            bool ok = true;
+            for (int w = first; w < items && ok; w += stride) {
+                const Item it = item_at(w, p);
+                const int kb0 = it.split * p.k_per_split, nk = min(p.k_per_split, p.k_blocks - kb0);
+                for (int kb = 0; kb < nk && ok; kb++) {
+                    if (done >= early) {
+                        if (done >= ST) ok = mbar_wait(empty(s), phase ^ 1, abort_flag, p.status);
+                        if (!ok) break;
+                        if (rank == 0) mbar_expect_tx(full(s), CG * L::STAGE);
+                        load_w(s, it.n_tile, kb0 + kb);
+                        load_x(s, it.m_tile, kb0 + kb);
+                    }
+                    done++;
+                    if (++s == ST) {
+                        s = 0;
+                        phase ^= 1;
+                    }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        // ---------------- MMAs: one thread of the pair's first CTA ----------------
+        if (lane == 0 && rank == 0) {
+            constexpr uint32_t idesc = (1u << 4) | (1u << 15) | ((MT >> 3) << 17) | ((CG * BN >> 4) << 24);  // f16 x f16 -> f32, weights n-major
+            constexpr uint32_t idesc_wide = (1u << 4) | (1u << 15) | (((2 * MT) >> 3) << 17) | ((CG * BN >> 4) << 24);
+            const uint64_t w_desc0 = smem_desc_n128(base), x_desc0 = smem_desc_k128(base + L::W_BYTES);
+            int s = 0, buf = 0;
+            uint32_t phase = 0, acc_phase = 0;
+            bool ok = true;
+            for (int w = first; w < items && ok; w += stride) {
+                const Item it = item_at(w, p);
+                const int kb0 = it.split * p.k_per_split, nk = min(p.k_per_split, p.k_blocks - kb0);
+                for (int kb = 0; kb < nk && ok; kb++) {
+                    const int in_chunk = (kb0 + kb) % p.chunk_blocks;
+                    const bool fresh = kb == 0 || in_chunk == 0;
+                    if (fresh) {
+                        ok = mbar_wait(acc_empty(buf), acc_phase ^ 1, abort_flag, p.status);  // its first use passes at once
+                        if (!ok) break;
+                    }
+                    ok = mbar_wait(full(s), phase, abort_flag, p.status);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t d = tmem + buf * L::D_COLS;
+                    const uint64_t w_hi = w_desc0 + ((s * L::STAGE) >> 4), x_hi = x_desc0 + ((s * L::STAGE) >> 4);
+#pragma unroll
+                    for (int kk = 0; kk < 4; kk++) {
+                        const uint32_t acc = (fresh && kk == 0) ? 0u : 1u;
+                        const uint64_t wh = w_hi + kk * 128, xh = x_hi + kk * 2;  // 16 k: 2 KB of the weight tile, 32 bytes inside the activation rows
+                        if constexpr (!SPLIT) {
+                            mma_f16<CG>(d, wh, xh, idesc, acc);
+                        } else {
+                            // high x high in columns [0, MT), high x low and low x high in [MT, 2 MT): the small products stay out of the
+                            // large sums.  low x low (below 2^-22 of the product) is dropped.
+                            const uint64_t wl = wh + (W_TILE >> 4), xl = xh + (L::X_TILE >> 4);
+                            if constexpr (CG == 1) {  // the low activation tile follows the high one: one MMA of twice the width
+                                mma_f16<CG>(d, wh, xh, idesc_wide, acc);
+                            } else {
+                                mma_f16<CG>(d, wh, xh, idesc, acc);
+                                mma_f16<CG>(d + MT, wh, xl, idesc, acc);
+                            }
+                            mma_f16<CG>(d + MT, wl, xh, idesc, 1u);
+                        }
+                    }
+                    commit<CG>(empty(s));
+                    if (++s == ST) {
+                        s = 0;
+                        phase ^= 1;
+                    }
+                    if (kb + 1 == nk || in_chunk + 1 == p.chunk_blocks) {
+                        commit<CG>(acc_full(buf));
+                        if (++buf == L::NBUF) {
+                            buf = 0;
+                            acc_phase ^= 1;
+                        }
+                    }
+                }
+            }
+        }
+    } else {
+        // ---------------- epilogue ----------------
+        // Two warps per group of 32 TMEM lanes (= columns of the output), each with half of the tile's rows.  A chunk's sums move from
+        // TMEM to registers (scaled and added up there), the accumulator goes back to the MMA thread, and the stores follow under
+        // the next tile's MMAs.
+        constexpr int HM = MT / 2, STEP = HM < 32 ? HM : 32;
+        const int sub = warp & 3, half = (warp - 2) >> 2;
+        const uint32_t lane_field = static_cast<uint32_t>(sub * 32) << 16;
+        const uint32_t pair_empty = CG == 2 ? mapa_shared(acc_empty(0), 0) : acc_empty(0);
+        dep_wait();  // scales and outputs may belong to kernels before this one
+        int buf = 0;
+        uint32_t acc_phase = 0;
+        bool ok = true;
+        for (int w = first; w < items && ok; w += stride) {
+            const Item it = item_at(w, p);
+            const int kb0 = it.split * p.k_per_split, nk = min(p.k_per_split, p.k_blocks - kb0);
+            const int64_t n = (static_cast<int64_t>(it.n_tile) * CG + rank) * BN + sub * 32 + lane;
+            const int64_t m_base = static_cast<int64_t>(it.m_tile) * MT + half * HM;
+            float acc[HM];
+            const int c_first = kb0 / p.chunk_blocks, c_last = (kb0 + nk - 1) / p.chunk_blocks;
+            for (int c = c_first; c <= c_last && ok; c++) {
+                ok = mbar_wait(acc_full(buf), acc_phase, abort_flag, p.status);
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t d = tmem + lane_field + buf * L::D_COLS + half * HM;
+#pragma unroll
+                for (int j0 = 0; j0 < HM; j0 += STEP) {
+                    uint32_t r[STEP];
+                    tmem_ld<STEP>(d + j0, r);
+                    if constexpr (SPLIT) {
+                        uint32_t q[STEP];
+                        tmem_ld<STEP>(d + MT + j0, q);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                        const float* xs = p.x_scale + c * p.x_scale_pitch + m_base + j0;
+#pragma unroll
+                        for (int j = 0; j < STEP; j += 4) {
+                            const float4 s4 = __ldg(reinterpret_cast<const float4*>(xs + j));
+                            const float sc[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+                            for (int e = 0; e < 4; e++) {
+                                const float v = fmaf(__uint_as_float(q[j + e]), 1.f / LO_SCALE, __uint_as_float(r[j + e]));
+                                acc[j0 + j + e] = c == c_first ? v * sc[e] : fmaf(v, sc[e], acc[j0 + j + e]);
+                            }
+                        }
+                    } else {
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                        for (int j = 0; j < STEP; j++) acc[j0 + j] = __uint_as_float(r[j]);
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    if constexpr (CG == 2) arrive_cluster(pair_empty + 8u * buf);
+                    else mbar_arrive(acc_empty(buf));
+                }
+                if (++buf == L::NBUF) {
+                    buf = 0;
+                    acc_phase ^= 1;
+                }
+            }
+            if (!ok) break;
+            if (n < p.N) {
+                if constexpr (SPLIT) {
+                    const float ws = __ldg(p.w_scale + n);
+#pragma unroll
+                    for (int j = 0; j < HM; j++) acc[j] *= ws;
+                }
+                const int64_t slab = p.ksplit > 1 ? static_cast<int64_t>(it.split) * p.M * p.N : 0;
+#pragma unroll
+                for (int j = 0; j < HM; j++) {
+                    const int64_t m = m_base + j;
+                    if (m < p.M) {
+                        if constexpr (OUT16) static_cast<__half*>(p.out)[slab + m * p.ldc + n] = __float2half_rn(acc[j]);
+                        else static_cast<float*>(p.out)[slab + m * p.ldc + n] = acc[j];
+                    }
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    if constexpr (CG == 2) cluster_sync_all();  // no CTA of the pair leaves while the other may still signal its barriers or read its tiles
+    else __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        if constexpr (CG == 1)
+            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(L::TMEM_COLS) : "memory");
+        else
+            asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(L::TMEM_COLS) : "memory");
+    }
+}
+
+}  // namespace umma
+}  // namespace rmlk
