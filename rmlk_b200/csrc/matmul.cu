@@ -15,9 +15,11 @@
 //
 // The reference calls cublasGemmStridedBatchedEx with CUBLAS_COMPUTE_32F
 // (cuda/src/kernels/gemm.rs:206-231); both kernels accumulate in fp32 with FMA.
+#include <algorithm>
 #include <atomic>
 
 #include "common.cuh"
+#include "umma_gemm.h"
 
 namespace rmlk {
 
@@ -744,13 +746,27 @@ int tc_matmul_plan(int64_t m, int64_t n, int64_t k);
 // fewest rows of A the tensor-core path takes: from 5 rows on, one pass of the weight-streaming tensor-core kernel (its 64-row
 // tile mostly padding) beats the SIMT small-M kernels; up to 4 rows the wide-strip SIMT kernel is at the HBM stream's speed
 constexpr int64_t TC_MIN_ROWS = 5;
+constexpr int64_t SPLIT_MIN_ROWS = 256;
 bool tc_enabled();
 // matmul_f16.cu
 int matmul_f16(cudaStream_t st, int64_t batch, int64_t m, int64_t n, int64_t k, const void* a, int64_t sa, const void* b, int64_t sb, void* c,
                int64_t sc, int* status);
 }  // namespace rmlk
 
-extern "C" size_t rmlk_b200_matmul_workspace_bytes(int dtype, int64_t batch, int64_t m, int64_t n, int64_t k) {
+// The product on pairs of f16, both operands split into the workspace first.  Splitting moves 12 bytes per element of B and of A,
+// the product itself runs at twice the rate of the kernel that splits in flight: that pays from some hundred rows on.
+static bool split_pays(int64_t m, int64_t n, int64_t k) {
+    return tc_enabled() && m >= SPLIT_MIN_ROWS && n >= 64 && k >= 64 && ceil_div64(k, 64) <= 65535 && m < (1ll << 24) && n < (1ll << 28) && k < (1ll << 28) &&
+           ceil_div64(n, 128) * ceil_div64(k, 64) * 256 < (1ll << 31) && ceil_div64(n, 128) * ceil_div64(m, 16) < (1ll << 30) && tc::encode_fn() != nullptr;
+}
+static size_t round1k(size_t v) { return (v + 1023) & ~static_cast<size_t>(1023); }
+static size_t split_workspace(int64_t m, int64_t n, int64_t k) {
+    const int parts = umma_split_parts(m, n, k);
+    return 1024 + round1k(split_weights_bytes(n, k)) + round1k(split_rows_bytes(m, k, 0)) + (parts > 1 ? static_cast<size_t>(parts) * m * n * sizeof(float) : 0);
+}
+
+// Least scratch of a shape (what the kernels without a splitting pass need)
+static size_t matmul_least_scratch(int dtype, int64_t batch, int64_t m, int64_t n, int64_t k) {
     if (dtype != RMLK_F32 || batch <= 0 || m <= 0 || n <= 0 || k <= 0) return 0;
     if (batch == 1 && m >= TC_MIN_ROWS && tc_enabled() && n % 128 == 0 && k % 32 == 0 && k >= 32) return tc_matmul_workspace_bytes(m, n, k);
     if (m > 16) return 0;
@@ -762,6 +778,12 @@ extern "C" size_t rmlk_b200_matmul_workspace_bytes(int dtype, int64_t batch, int
         const size_t need_w = sw > 1 ? static_cast<size_t>(sw) * batch * m * n * sizeof(float) : 0;
         if (need_w > need) need = need_w;
     }
+    return need;
+}
+
+extern "C" size_t rmlk_b200_matmul_workspace_bytes(int dtype, int64_t batch, int64_t m, int64_t n, int64_t k) {
+    const size_t need = matmul_least_scratch(dtype, batch, m, n, k);
+    if (dtype == RMLK_F32 && batch == 1 && n > 0 && k > 0 && split_pays(m, n, k)) return std::max(need, split_workspace(m, n, k));
     return need;
 }
 
@@ -850,6 +872,25 @@ extern "C" int rmlk_b200_matmul_flags(rmlk_stream_t stream, int dtype, int64_t b
     if (!a || !b) return fail(RMLK_ERR_INVALID_ARG, "matmul: NULL operand");
     if (batch > 65535) return fail(RMLK_ERR_INVALID_ARG, "matmul: batch exceeds 65535");
     const bool b_rows_aligned = (n % 4 == 0) && aligned_to(b, 16) && (b_batch_stride % 4 == 0);
+    if (batch == 1 && split_pays(m, n, k) && workspace && workspace_bytes >= split_workspace(m, n, k)) {
+        char* ws = reinterpret_cast<char*>(round1k(reinterpret_cast<uintptr_t>(workspace)));
+        const SplitWeights w = split_weights_at(ws, n, k);
+        ws += round1k(split_weights_bytes(n, k));
+        const SplitRows x = split_rows_at(ws, m, k, 0);
+        ws += round1k(split_rows_bytes(m, k, 0));
+        WeightSources src = {};
+        src.count = 1;
+        src.w[0] = static_cast<const float*>(b);
+        src.n[0] = n;
+        src.vec[0] = n % 4 == 0 && aligned_to(b, 16);
+        if (int rc = split_weights_pack(st, src, w)) return rc;
+        if (int rc = split_rows_pack(st, static_cast<const float*>(a), k, x)) return rc;
+        int parts = 1;
+        const size_t left = workspace_bytes - static_cast<size_t>(ws - static_cast<char*>(workspace));
+        if (int rc = umma_split(st, x, w, static_cast<float*>(c), n, reinterpret_cast<float*>(ws), left, status, 0, &parts)) return rc;
+        if (parts > 1) return rmlk_b200_sum_parts(stream, dtype, parts, m * n, ws, c);
+        return RMLK_OK;
+    }
     if (batch == 1 && tc_matmul_eligible(m, n, k, a, b, c)) {
         int ksplit = 1;
         if (int rc = tc_matmul(st, m, n, k, static_cast<const float*>(a), static_cast<const float*>(b), static_cast<float*>(c), workspace,
@@ -1103,10 +1144,6 @@ static void* static_scratch_ptr(int* rc_out) {
 }
 
 extern "C" size_t rmlk_b200_matmul_static_scratch_bytes(void) { return RMLK_STATIC_SCRATCH_BYTES; }
-
-static size_t matmul_least_scratch(int dtype, int64_t batch, int64_t m, int64_t n, int64_t k) {
-    return rmlk_b200_matmul_workspace_bytes(dtype, batch, m, n, k);
-}
 
 extern "C" int rmlk_b200_matmul_static_supported(int dtype, int64_t batch, int64_t m, int64_t n, int64_t k) {
     return matmul_least_scratch(dtype, batch, m, n, k) <= RMLK_STATIC_SCRATCH_BYTES ? 1 : 0;

@@ -38,7 +38,7 @@ static int launch(cudaStream_t st, const CUtensorMap& tmW, const CUtensorMap& tm
     const int64_t items = static_cast<int64_t>(p.n_tiles) * p.m_tiles * p.ksplit;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(CG * std::min<int64_t>(items, sm_count() / CG)));
-    cfg.blockDim = dim3(THREADS);
+    cfg.blockDim = dim3(L::THREADS);
     cfg.dynamicSmemBytes = L::TOTAL;
     cfg.stream = st;
     cudaLaunchAttribute at[2];
@@ -68,13 +68,14 @@ struct Plan {
 
 // Tile shape for a product: the shape whose waves cost least, an item costing its k-blocks (the MMAs, or the bytes a CTA has to
 // bring in where those take longer) plus what starting and storing a tile takes.  `products`: MMAs per product (3 for split operands).
-static Plan plan_for(int64_t m, int64_t n, int64_t k, int products, bool may_split) {
+static Plan plan_for(int64_t m, int64_t n, int64_t k, int products, bool may_split, bool chunks = false) {
     static const int shapes[][2] = {{1, 16}, {1, 32}, {1, 64}, {1, 128}, {2, 128}, {2, 192}, {2, 256}};
     const int64_t sms = sm_count(), kb = ceil_div64(k, BK);
     Plan best = {1, 16, 1};
     double best_cost = 1e30;
     for (const auto& s : shapes) {
         const int cg = s[0], mt = s[1];
+        if (chunks && mt > 128) continue;  // the tall tiles take one scale per row
         const int64_t tiles = ceil_div64(n, BN * cg) * ceil_div64(m, mt), slots = sms / cg;
         int64_t ks = 1;
         if (may_split && tiles < slots) {
@@ -139,6 +140,33 @@ int umma_f16(cudaStream_t st, int64_t m, int64_t n, int64_t k, const void* a, co
     p.chunk_blocks = p.k_blocks;
     p.status = status;
     return dispatch<false, true>(st, pl, tmW, tmX, p);
+}
+
+int umma_split_parts(int64_t m, int64_t n, int64_t k) { return umma::plan_for(m, n, k, 3, true).ksplit; }
+
+int umma_split(cudaStream_t st, const SplitRows& x, const SplitWeights& w, float* out, int64_t ldc, float* slabs, size_t slab_bytes, int* status, int flags, int* parts) {
+    using namespace umma;
+    const bool chunks = static_cast<int64_t>(x.chunk_blocks) * BK < x.k_pad;
+    Plan pl = plan_for(x.m, w.n, x.k, 3, parts != nullptr, chunks);
+    if (pl.ksplit > 1 && slab_bytes < static_cast<size_t>(pl.ksplit) * x.m * w.n * sizeof(float)) pl = plan_for(x.m, w.n, x.k, 3, false, chunks);
+    CUtensorMap tmW, tmX;
+    if (!map_2d_f16(&tmW, w.tiles, 64, static_cast<uint64_t>(w.n_blocks) * w.k_blocks * 256, 64, 64, 256, CU_TENSOR_MAP_SWIZZLE_NONE) ||
+        !map_2d_f16(&tmX, x.data, x.k_pad, 2 * x.m_pad, x.k_pad, BK, pl.mt / pl.cg, CU_TENSOR_MAP_SWIZZLE_128B))
+        return fail(RMLK_ERR_INTERNAL, "matmul: cuTensorMapEncodeTiled failed");
+    Params p = {};
+    fill_tiles(p, pl, x.m, w.n, x.k);
+    p.out = p.ksplit > 1 ? slabs : out;
+    p.ldc = p.ksplit > 1 ? w.n : ldc;
+    p.w_rows_per_tile = static_cast<int>(w.k_blocks * 256);
+    p.x_lo_row = static_cast<int>(x.m_pad);
+    p.w_scale = w.scale;
+    p.x_scale = x.scale;
+    p.x_scale_pitch = x.scale_pitch;
+    p.chunk_blocks = x.chunk_blocks;
+    p.w_static = (flags & RMLK_MATMUL_B_STATIC) ? 1 : 0;
+    p.status = status;
+    if (parts) *parts = p.ksplit;
+    return dispatch<true, false>(st, pl, tmW, tmX, p);
 }
 
 }  // namespace rmlk

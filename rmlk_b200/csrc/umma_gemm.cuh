@@ -22,8 +22,6 @@ using tc::tmem_ld_x32;
 
 constexpr int BK = 64;     // f16 elements of K per block: one 128-byte row of an activation tile
 constexpr int BN = 128;    // weight columns per CTA = MMA M per CTA = TMEM lanes
-constexpr int EPI_WARPS = 8;
-constexpr int THREADS = 64 + 32 * EPI_WARPS;  // TMA warp, MMA warp, epilogue warps
 constexpr float LO_SCALE = 2048.f;            // the low parts are stored 2^11 times their size: their f16 exponent starts where the high part's ends
 
 // Weight tile: two [64 k][64 n] blocks of 8 KB, n contiguous, 128-byte swizzled (what a SWIZZLE_128B box of 64 x 64 leaves in shared
@@ -98,6 +96,9 @@ struct Params {
 // CG: CTAs per tile (a pair shares one tile of 256 columns); SPLIT: operands are (high, low) pairs of f16; MT: activation rows per tile; ST: stages
 template <int CG, bool SPLIT, int MT, int ST>
 struct Layout {
+    // Epilogue warps, two or four for each group of 32 TMEM lanes: at most 64 sums per thread, so that nothing spills.
+    static constexpr int EPI_WARPS = MT >= 192 ? 16 : 8;
+    static constexpr int THREADS = 64 + 32 * EPI_WARPS;  // TMA warp, MMA warp, epilogue warps
     static constexpr int XR = MT / CG;  // activation rows that this CTA loads
     static constexpr uint32_t W_BYTES = W_TILE * (SPLIT ? 2 : 1);
     static constexpr uint32_t X_TILE = XR * BK * 2;

@@ -18,4 +18,36 @@ bool tc_enabled();
 bool umma_f16_eligible(int64_t m, int64_t n, int64_t k, const void* a, const void* b);
 int umma_f16(cudaStream_t st, int64_t m, int64_t n, int64_t k, const void* a, const void* b, void* c, int* status);
 
+// ---- fp32 operands as pairs of f16 (umma_pack.cu) ----
+// Up to 4 row-major [k][n_j] matrices laid side by side.
+struct WeightSources {
+    int count;
+    const float* w[4];
+    int64_t n[4], col0[4];
+    int vec[4];  // rows are 16-byte aligned
+};
+struct SplitWeights {
+    void* tiles;   // [n_blocks][k_blocks][2][16 KB]
+    float* scale;  // per column, padded to whole blocks; behind it the scratch of the packing kernels
+    int64_t n, k, n_blocks, k_blocks;
+};
+size_t split_weights_bytes(int64_t n, int64_t k);
+SplitWeights split_weights_at(void* buf, int64_t n, int64_t k);  // buf: 1 KB aligned
+int split_weights_pack(cudaStream_t st, const WeightSources& src, const SplitWeights& w);
+
+struct SplitRows {
+    void* data;    // f16 [2][m_pad][k_pad]: high parts over low parts; rows behind m are never read into a result
+    float* scale;  // [chunks][scale_pitch]
+    int64_t m, k, m_pad, k_pad, scale_pitch;
+    int chunk_blocks;  // blocks of 64 k that share a scale
+};
+size_t split_rows_bytes(int64_t m, int64_t k, int chunk_blocks);  // chunk_blocks 0: one scale per row
+SplitRows split_rows_at(void* buf, int64_t m, int64_t k, int chunk_blocks);
+int split_rows_pack(cudaStream_t st, const float* x, int64_t ldx, const SplitRows& dst);  // one scale per row
+
+// out[m, n] = x w.  With `parts` the K splits may be left as f32 slabs [*parts][m][n] in `slabs` (*parts = 1: out holds the result);
+// without it, or without room for the slabs, K is not split.
+int umma_split(cudaStream_t st, const SplitRows& x, const SplitWeights& w, float* out, int64_t ldc, float* slabs, size_t slab_bytes, int* status, int flags, int* parts);
+int umma_split_parts(int64_t m, int64_t n, int64_t k);  // K splits that the plan would take
+
 }  // namespace rmlk

@@ -52,7 +52,7 @@ __device__ __forceinline__ Item item_at(int w, const Params& p) {
 }
 
 template <int CG, bool SPLIT, int MT, int ST, bool OUT16>
-__global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, Params p) {
+__global__ void __launch_bounds__(Layout<CG, SPLIT, MT, ST>::THREADS, 1) gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, Params p) {
     using L = Layout<CG, SPLIT, MT, ST>;
     dep_trigger();
     extern __shared__ uint8_t smem_raw[];
@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant_
         }
         for (int b = 0; b < L::NBUF; b++) {
             mbar_init(acc_full(b), 1);
-            mbar_init(acc_empty(b), CG * EPI_WARPS);
+            mbar_init(acc_empty(b), CG * L::EPI_WARPS);
         }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -221,11 +221,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant_
         }
     } else {
         // ---------------- epilogue ----------------
-        // Two warps per group of 32 TMEM lanes (= columns of the output), each with half of the tile's rows.  A chunk's sums move from
+        // Several warps per group of 32 TMEM lanes (= columns of the output), each with its part of the tile's rows.  A chunk's sums move from
         // TMEM to registers (scaled and added up there), the accumulator goes back to the MMA thread, and the stores follow under
         // the next tile's MMAs.
-        constexpr int HM = MT / 2, STEP = HM < 32 ? HM : 32;
-        const int sub = warp & 3, half = (warp - 2) >> 2;
+        constexpr int HM = MT / (L::EPI_WARPS / 4), STEP = HM < 16 ? HM : 16;
+        constexpr bool ONE_CHUNK = MT > 128;  // tall tiles take one scale per row
+        const int sub = warp & 3, part = (warp - 2) >> 2;
         const uint32_t lane_field = static_cast<uint32_t>(sub * 32) << 16;
         const uint32_t pair_empty = CG == 2 ? mapa_shared(acc_empty(0), 0) : acc_empty(0);
         dep_wait();  // scales and outputs may belong to kernels before this one
@@ -236,37 +237,49 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant_
             const Item it = item_at(w, p);
             const int kb0 = it.split * p.k_per_split, nk = min(p.k_per_split, p.k_blocks - kb0);
             const int64_t n = (static_cast<int64_t>(it.n_tile) * CG + rank) * BN + sub * 32 + lane;
-            const int64_t m_base = static_cast<int64_t>(it.m_tile) * MT + half * HM;
+            const int64_t m_base = static_cast<int64_t>(it.m_tile) * MT + part * HM;
             float acc[HM];
+            float4 s4 = make_float4(0.f, 0.f, 0.f, 0.f);
+            auto row_scale = [&](int j) {
+                return __shfl_sync(0xffffffffu, (j & 3) == 0 ? s4.x : (j & 3) == 1 ? s4.y : (j & 3) == 2 ? s4.z : s4.w, j >> 2);
+            };
             const int c_first = kb0 / p.chunk_blocks, c_last = (kb0 + nk - 1) / p.chunk_blocks;
             for (int c = c_first; c <= c_last && ok; c++) {
+                // the scales of this warp's rows, four per lane, handed round by shuffles when they are needed
+                if constexpr (SPLIT) {
+                    if (4 * lane < HM) s4 = __ldg(reinterpret_cast<const float4*>(p.x_scale + c * p.x_scale_pitch + m_base) + lane);
+                }
                 ok = mbar_wait(acc_full(buf), acc_phase, abort_flag, p.status);
                 if (!ok) break;
+                __syncwarp();
                 tc_fence_after();
-                const uint32_t d = tmem + lane_field + buf * L::D_COLS + half * HM;
+                const uint32_t d = tmem + lane_field + buf * L::D_COLS + part * HM;
+                if constexpr (!SPLIT || ONE_CHUNK) {
 #pragma unroll
-                for (int j0 = 0; j0 < HM; j0 += STEP) {
-                    uint32_t r[STEP];
-                    tmem_ld<STEP>(d + j0, r);
+                    for (int j0 = 0; j0 < HM; j0 += STEP) tmem_ld<STEP>(d + j0, reinterpret_cast<uint32_t*>(acc) + j0);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                     if constexpr (SPLIT) {
-                        uint32_t q[STEP];
+#pragma unroll
+                        for (int j0 = 0; j0 < HM; j0 += STEP) {
+                            uint32_t q[STEP];
+                            tmem_ld<STEP>(d + MT + j0, q);
+                            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                            for (int j = 0; j < STEP; j++) acc[j0 + j] = fmaf(__uint_as_float(q[j]), 1.f / LO_SCALE, acc[j0 + j]);
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int j0 = 0; j0 < HM; j0 += STEP) {
+                        uint32_t r[STEP], q[STEP];
+                        tmem_ld<STEP>(d + j0, r);
                         tmem_ld<STEP>(d + MT + j0, q);
                         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                        const float* xs = p.x_scale + c * p.x_scale_pitch + m_base + j0;
 #pragma unroll
-                        for (int j = 0; j < STEP; j += 4) {
-                            const float4 s4 = __ldg(reinterpret_cast<const float4*>(xs + j));
-                            const float sc[4] = {s4.x, s4.y, s4.z, s4.w};
-#pragma unroll
-                            for (int e = 0; e < 4; e++) {
-                                const float v = fmaf(__uint_as_float(q[j + e]), 1.f / LO_SCALE, __uint_as_float(r[j + e]));
-                                acc[j0 + j + e] = c == c_first ? v * sc[e] : fmaf(v, sc[e], acc[j0 + j + e]);
-                            }
+                        for (int j = 0; j < STEP; j++) {
+                            const float v = fmaf(__uint_as_float(q[j]), 1.f / LO_SCALE, __uint_as_float(r[j])), sc = row_scale(j0 + j);
+                            acc[j0 + j] = c == c_first ? v * sc : fmaf(v, sc, acc[j0 + j]);
                         }
-                    } else {
-                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                        for (int j = 0; j < STEP; j++) acc[j0 + j] = __uint_as_float(r[j]);
                     }
                 }
                 tc_fence_before();
@@ -281,21 +294,22 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant_
                 }
             }
             if (!ok) break;
-            if (n < p.N) {
-                if constexpr (SPLIT) {
-                    const float ws = __ldg(p.w_scale + n);
+            const bool in = n < p.N;
+            const float ws = SPLIT && in ? __ldg(p.w_scale + n) : 0.f;
+            using Out = typename std::conditional<OUT16, __half, float>::type;
+            Out* o = static_cast<Out*>(p.out) + (p.ksplit > 1 ? static_cast<int64_t>(it.split) * p.M * p.N : 0) + m_base * p.ldc + n;
+            const int64_t rows = in ? p.M - m_base : 0;
 #pragma unroll
-                    for (int j = 0; j < HM; j++) acc[j] *= ws;
+            for (int j = 0; j < HM; j++) {
+                float v = acc[j];
+                if constexpr (SPLIT) v *= ws;
+                if constexpr (SPLIT && ONE_CHUNK) v *= row_scale(j);
+                if (j < rows) {
+                    if constexpr (OUT16) *o = __float2half_rn(v);
+                    else *o = v;
                 }
-                const int64_t slab = p.ksplit > 1 ? static_cast<int64_t>(it.split) * p.M * p.N : 0;
-#pragma unroll
-                for (int j = 0; j < HM; j++) {
-                    const int64_t m = m_base + j;
-                    if (m < p.M) {
-                        if constexpr (OUT16) static_cast<__half*>(p.out)[slab + m * p.ldc + n] = __float2half_rn(acc[j]);
-                        else static_cast<float*>(p.out)[slab + m * p.ldc + n] = acc[j];
-                    }
-                }
+                o += p.ldc;
+                asm volatile("" : "+l"(o)::"memory");  // one row after the other: addresses and scales of all 128 rows would not fit in registers beside the sums
             }
         }
     }

@@ -31,3 +31,49 @@ def test_f16_large_tiles(cuda):
         want, mag = a.double() @ b.double(), a.double().abs() @ b.double().abs()
         bound = want.abs() * 2.0 ** -11 + mag * 2.0 ** -23 * (k / 16 + 1) + 2.0 ** -24
         assert bool(((got - want).abs() <= bound).all()), (m, n, k)
+
+
+def _check_f32(a, b, got):
+    import torch
+    want, mag = a.double() @ b.double(), a.double().abs() @ b.double().abs()
+    k = a.shape[1]
+    # the operands hold 22 bits (2^-22 for either one and for the dropped product of the low parts), sums lose one truncated fp32
+    # addition per 16 products
+    bound = mag * (3 * 2.0 ** -22 + 2.0 ** -23 * (k / 16 + 2))
+    assert bool(((got.double() - want).abs() <= bound).all()), float(((got.double() - want).abs() / bound).max())
+
+
+# what the splitting pass pads (K to 64, N to 128), row tiles, K splits; sizes that no other tensor-core kernel takes
+@pytest.mark.parametrize("m", [256, 300, 513])
+@pytest.mark.parametrize("n,k", [(64, 64), (100, 65), (129, 200), (512, 2048), (1000, 777), (3072, 2048)])
+def test_f32_split(cuda, m, n, k):
+    import torch
+    from rmlk_b200 import kernels as K
+    g = torch.Generator(device=cuda)
+    g.manual_seed(m + n + k)
+    a = torch.randn(m, k, device=cuda, generator=g)
+    b = torch.randn(k, n, device=cuda, generator=g) * 0.02
+    ws = torch.empty(K.matmul_workspace_bytes(1, m, n, k), dtype=torch.uint8, device=cuda)
+    _check_f32(a, b, K.matmul(a, b, workspace=ws))
+
+
+def test_f32_split_scales(cuda):
+    """Rows and columns of very different size, values far below their row's largest, zeros, the ends of the exponent range."""
+    import torch
+    from rmlk_b200 import kernels as K
+    m, n, k = 320, 256, 512
+    a = torch.randn(m, k, device=cuda) * torch.exp2(torch.randint(-60, 60, (m, 1), device=cuda).float())
+    b = torch.randn(k, n, device=cuda) * torch.exp2(torch.randint(-60, 60, (1, n), device=cuda).float())
+    a *= torch.exp2(-torch.rand(m, k, device=cuda) * 24)   # a range of 2^24 inside every row
+    b *= torch.exp2(-torch.rand(k, n, device=cuda) * 24)
+    a[5] = 0
+    b[:, 7] = 0
+    a[9] = 2.0 ** -120
+    a[11] = 2.0 ** 100
+    b[:, 13] = 2.0 ** -130   # denormal
+    ws = torch.empty(K.matmul_workspace_bytes(1, m, n, k), dtype=torch.uint8, device=cuda)
+    got = K.matmul(a, b, workspace=ws)
+    want, mag = a.double() @ b.double(), a.double().abs() @ b.double().abs()
+    bound = mag * (3 * 2.0 ** -22 + 2.0 ** -23 * (k / 16 + 2)) + 2.0 ** -125
+    fine = want.abs() < 2.0 ** 127
+    assert bool(((got.double() - want).abs() <= bound)[fine].all())
