@@ -23,6 +23,7 @@
 #include <cstdlib>
 #include <mutex>
 #include "common.cuh"
+#include "split_pair.cuh"
 
 namespace rmlk {
 
@@ -35,7 +36,9 @@ struct AttnParams {
     int64_t kb, vb;            // problem strides of K and V (elements)
     int64_t ms_b, ms_h;        // mask strides per batch entry and per head (elements; rows of T are dense)
     int rows, T, kv_heads;
+    int ctas;                  // CTAs that share a problem's keys (a cluster)
     float scale;
+    SplitRows pairs;           // gqa_decode_flash_kernel<.., PAIRS>: where the result goes as pairs of f16
 };
 
 template <int LPR>
@@ -393,7 +396,7 @@ struct FlashSmem {
     static constexpr uint32_t STATS_OFF = CORR_OFF + FL_WARPS * 4 * 4;       // m[warps][4], then l[warps][4]
     static constexpr uint32_t BAR_OFF = STATS_OFF + 2 * FL_WARPS * 4 * 4;    // full[FL_STAGES], empty[FL_STAGES] mbarriers, then a flag word
     static constexpr uint32_t TOTAL = BAR_OFF + 16 * FL_STAGES + 16;
-    static_assert(RING_BYTES >= FL_WARPS * 4 * D * 4, "the ring must hold the warps' partial outputs");
+    static_assert(RING_BYTES >= (FL_WARPS + 1) * 4 * D * 4 + 32, "the ring must hold the warps' partial outputs");
 };
 
 __device__ __forceinline__ uint32_t fl_smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
@@ -411,8 +414,12 @@ __device__ __forceinline__ bool fl_wait(uint32_t bar, uint32_t parity, volatile 
     return false;
 }
 
-template <int LPR>
-__global__ void __launch_bounds__(FL_THREADS, LPR <= 16 ? 4 : 2) gqa_decode_flash_kernel(AttnParams p) {
+// CLUSTER: the keys of a problem are shared out over the CTAs of a thread-block cluster (consecutive ranges of blocks); every CTA
+// leaves its maximum, sum and weighted values in its shared memory and the first one adds them up.  A decode step of one request
+// has 8 problems: one CTA each left 140 SMs idle for the whole walk over the keys.
+// PAIRS: the rows of a problem leave as pairs of f16 under one scale, for the tensor-core MatMul that reads them.
+template <int LPR, bool CLUSTER, bool PAIRS>
+__global__ void __launch_bounds__(FL_THREADS, LPR <= 16 ? 4 : 2) gqa_decode_flash_kernel(const __grid_constant__ AttnParams p) {
     using L = FlashSmem<LPR>;
     constexpr int D = 4 * LPR;
     constexpr int RPI = 32 / LPR;          // rows per warp-wide 16-byte-per-lane access
@@ -430,9 +437,13 @@ __global__ void __launch_bounds__(FL_THREADS, LPR <= 16 ? 4 : 2) gqa_decode_flas
     auto empty = [&](int st) { return bars + 8u * (FL_STAGES + st); };
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int sub = lane % LPR, rsel = lane / LPR;
-    const int64_t prob = blockIdx.x;
+    const int64_t prob = CLUSTER ? blockIdx.x / p.ctas : blockIdx.x;
+    const int rank = CLUSTER ? blockIdx.x % p.ctas : 0;
     const int T = p.T;
-    const int n_blocks = (T + FL_KEYS - 1) / FL_KEYS;
+    const int all_blocks = (T + FL_KEYS - 1) / FL_KEYS;
+    const int per_cta = CLUSTER ? (all_blocks + p.ctas - 1) / p.ctas : all_blocks;
+    const int first_block = rank * per_cta;
+    const int n_blocks = CLUSTER ? max(0, min(per_cta, all_blocks - first_block)) : all_blocks;
     const float* __restrict__ Kp = p.k + prob * p.kb;
     const float* __restrict__ Vp = p.v + prob * p.vb;
 
@@ -459,14 +470,15 @@ __global__ void __launch_bounds__(FL_THREADS, LPR <= 16 ? 4 : 2) gqa_decode_flas
             for (int blk = 0; blk < n_blocks; blk++) {
                 const int st = blk % FL_STAGES;
                 if (blk >= FL_STAGES && !fl_wait(empty(st), ((blk / FL_STAGES) - 1) & 1, s_bad)) break;
-                const int keys = T - blk * FL_KEYS < FL_KEYS ? T - blk * FL_KEYS : FL_KEYS;
+                const int key0 = (first_block + blk) * FL_KEYS;
+                const int keys = T - key0 < FL_KEYS ? T - key0 : FL_KEYS;
                 const uint32_t bytes = static_cast<uint32_t>(keys) * D * 4;
                 const uint32_t bar = full(st), dst = ring + st * L::STAGE_BYTES;
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(2 * bytes) : "memory");
                 asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                             ::"r"(dst), "l"(Kp + static_cast<int64_t>(blk) * FL_KEYS * D), "r"(bytes), "r"(bar) : "memory");
+                             ::"r"(dst), "l"(Kp + static_cast<int64_t>(key0) * D), "r"(bytes), "r"(bar) : "memory");
                 asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                             ::"r"(dst + L::BLOCK_BYTES), "l"(Vp + static_cast<int64_t>(blk) * FL_KEYS * D), "r"(bytes), "r"(bar) : "memory");
+                             ::"r"(dst + L::BLOCK_BYTES), "l"(Vp + static_cast<int64_t>(key0) * D), "r"(bytes), "r"(bar) : "memory");
             }
         }
     } else {
@@ -484,7 +496,7 @@ __global__ void __launch_bounds__(FL_THREADS, LPR <= 16 ? 4 : 2) gqa_decode_flas
 
         for (int blk = 0; blk < n_blocks; blk++) {
             const int st = blk % FL_STAGES;
-            const int t0 = blk * FL_KEYS;
+            const int t0 = (first_block + blk) * FL_KEYS;
             // the mask value of this lane's (key, row) of the softmax step is asked for now, before the wait for the block
             // and the dot products, and added there (the same two roundings, v * scale + mask, as in the kernels above)
             float mk = 0.f;
@@ -592,22 +604,108 @@ __global__ void __launch_bounds__(FL_THREADS, LPR <= 16 ? 4 : 2) gqa_decode_flas
         for (int m = 0; m < 4; m++) *reinterpret_cast<float4*>(s_a + (warp * 4 + m) * D + 4 * sub) = make_float4(acc[m][0], acc[m][1], acc[m][2], acc[m][3]);
     }
     __syncthreads();
-    const bool bad = *s_bad != 0;
-    for (int i = threadIdx.x; i < p.rows * D; i += FL_THREADS) {
-        const int m = i / D, d = i - m * D;
-        float M = -INFINITY;
+    // this CTA's values: s_a[0 .. 4 D) the weighted sums, s_m / s_l rows 0..3 the maxima and the sums (each thread rewrites what only it reads)
+    constexpr int PER = (4 * D + FL_THREADS - 1) / FL_THREADS;
+    float A[PER], M[PER], Ls[PER];
 #pragma unroll
-        for (int w = 0; w < FL_WARPS; w++) M = fmaxf(M, s_m[w * 4 + m]);
-        float A = 0.f, Lsum = 0.f;
+    for (int q = 0; q < PER; q++) {
+        const int i = threadIdx.x + q * FL_THREADS, m = i / D, d = i - m * D;
+        A[q] = Ls[q] = 0.f;
+        M[q] = -INFINITY;
+        if (i >= p.rows * D) continue;
+#pragma unroll
+        for (int w = 0; w < FL_WARPS; w++) M[q] = fmaxf(M[q], s_m[w * 4 + m]);
 #pragma unroll
         for (int w = 0; w < FL_WARPS; w++) {
             const float mw = s_m[w * 4 + m];
-            const float f = mw == -INFINITY ? 0.f : expf(mw - M);
-            Lsum = fmaf(s_l[w * 4 + m], f, Lsum);
-            A = fmaf(s_a[(w * 4 + m) * D + d], f, A);
+            const float f = mw == -INFINITY ? 0.f : expf(mw - M[q]);
+            Ls[q] = fmaf(s_l[w * 4 + m], f, Ls[q]);
+            A[q] = fmaf(s_a[(w * 4 + m) * D + d], f, A[q]);
         }
-        p.out[prob * p.rows * D + i] = bad ? __int_as_float(0x7fc00000) : A / Lsum;
     }
+    if constexpr (CLUSTER) {
+        // slots behind the warps' partial outputs in the ring: [0, 4 D) sums, then maxima and totals
+        float* mine = s_a + FL_WARPS * 4 * D;
+        if (*s_bad) {
+            for (int i = threadIdx.x; i < 4; i += FL_THREADS) mine[4 * D + 4 + i] = __int_as_float(0x7fc00000);
+        }
+#pragma unroll
+        for (int q = 0; q < PER; q++) {
+            const int i = threadIdx.x + q * FL_THREADS, m = i / D, d = i - m * D;
+            if (i >= p.rows * D) continue;
+            mine[i] = A[q];
+            if (d == 0) {
+                mine[4 * D + m] = M[q];
+                if (!*s_bad) mine[4 * D + 4 + m] = Ls[q];
+            }
+        }
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (rank == 0) {
+            const uint32_t local = fl_smem_u32(mine);
+            auto peer = [&](uint32_t rank, int at) {
+                uint32_t addr;
+                float v;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(local + 4u * at), "r"(rank));
+                asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+                return v;
+            };
+            const uint32_t n = p.ctas;
+#pragma unroll
+            for (int q = 0; q < PER; q++) {
+                const int i = threadIdx.x + q * FL_THREADS, m = i / D;
+                if (i >= p.rows * D) continue;
+                float top = M[q];
+                for (uint32_t r = 1; r < n; r++) top = fmaxf(top, peer(r, 4 * D + m));
+                float f = M[q] == -INFINITY ? 0.f : expf(M[q] - top);
+                float a2 = A[q] * f, l2 = Ls[q] * f;
+                for (uint32_t r = 1; r < n; r++) {  // in rank order: the same bits every time
+                    const float mr = peer(r, 4 * D + m);
+                    f = mr == -INFINITY ? 0.f : expf(mr - top);
+                    a2 = fmaf(peer(r, i), f, a2);
+                    l2 = fmaf(peer(r, 4 * D + 4 + m), f, l2);
+                }
+                A[q] = a2;
+                Ls[q] = l2;
+            }
+        }
+    }
+    if (rank == 0) {
+        const bool bad = *s_bad != 0;
+        uint32_t top = 0;
+#pragma unroll
+        for (int q = 0; q < PER; q++) {
+            const int i = threadIdx.x + q * FL_THREADS;
+            A[q] = bad ? __int_as_float(0x7fc00000) : A[q] / Ls[q];
+            if (i >= p.rows * D) continue;
+            if constexpr (PAIRS) top = max(top, finite_abs_bits(A[q]));
+            else p.out[prob * p.rows * D + i] = A[q];
+        }
+        if constexpr (PAIRS) {
+            uint32_t* s_top = reinterpret_cast<uint32_t*>(s_m);  // every thread has read the statistics
+            __syncthreads();
+            if (threadIdx.x == 0) *s_top = 0;
+            __syncthreads();
+            top = __reduce_max_sync(0xffffffffu, top);
+            if (lane == 0) atomicMax(s_top, top);
+            __syncthreads();
+            const int e = scale_exponent(*s_top);
+            const float up = exp2_int(e);
+            const int64_t b = prob / p.kv_heads, h = prob % p.kv_heads;
+            if (threadIdx.x == 0) p.pairs.scale[h * p.pairs.scale_pitch + b] = exp2_int(-e);
+            __half* o = static_cast<__half*>(p.pairs.data) + b * p.pairs.k_pad + h * p.rows * D;
+#pragma unroll
+            for (int q = 0; q < PER; q++) {
+                const int i = threadIdx.x + q * FL_THREADS;
+                if (i >= p.rows * D) continue;
+                const float x = A[q] * up;
+                const __half hi = __float2half_rn(x);
+                o[i] = hi;
+                o[p.pairs.m_pad * p.pairs.k_pad + i] = __float2half_rn((x - __half2float(hi)) * SPLIT_LO);
+            }
+        }
+    }
+    if constexpr (CLUSTER)  // no CTA leaves while the first one may still read its shared memory
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 constexpr int64_t ATTN_MAX_KEYS = 12288;  // 16 bytes of shared memory per key
@@ -630,21 +728,53 @@ static int attn_launch(cudaStream_t st, const AttnParams& p, int64_t problems) {
     return RMLK_OK;
 }
 
-template <int LPR>
-static int attn_flash_launch(cudaStream_t st, const AttnParams& p, int64_t problems) {
+template <int LPR, bool CLUSTER, bool PAIRS>
+static int attn_flash_launch_as(cudaStream_t st, AttnParams p, int64_t problems, int ctas) {
+    p.ctas = ctas;
     using L = FlashSmem<LPR>;
-    static std::once_flag configured[64];  // once per device; a concurrent first call waits for the attribute to be set
+    auto kernel = gqa_decode_flash_kernel<LPR, CLUSTER, PAIRS>;
+    static std::once_flag configured[64];
     int dev = 0;
     cudaGetDevice(&dev);
     cudaError_t cfg_err = cudaSuccess;
     if (dev >= 0 && dev < 64)
-        std::call_once(configured[dev], [&] {
-            cfg_err = cudaFuncSetAttribute(gqa_decode_flash_kernel<LPR>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(L::TOTAL));
-        });
+        std::call_once(configured[dev], [&] { cfg_err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(L::TOTAL)); });
     RMLK_CUDA(cfg_err);
-    launch_dep(gqa_decode_flash_kernel<LPR>, dim3(static_cast<unsigned>(problems)), dim3(FL_THREADS), L::TOTAL, st, p);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(problems * ctas));
+    cfg.blockDim = dim3(FL_THREADS);
+    cfg.dynamicSmemBytes = L::TOTAL;
+    cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    unsigned na = 0;
+    if (CLUSTER) {
+        at[na].id = cudaLaunchAttributeClusterDimension;
+        at[na].val.clusterDim.x = static_cast<unsigned>(ctas);
+        at[na].val.clusterDim.y = 1;
+        at[na].val.clusterDim.z = 1;
+        na++;
+    }
+    if (dep_launch_enabled()) {
+        at[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[na].val.programmaticStreamSerializationAllowed = 1;
+        na++;
+    }
+    cfg.attrs = at;
+    cfg.numAttrs = na;
+    RMLK_CUDA(cudaLaunchKernelEx(&cfg, kernel, p));
     RMLK_CHECK_LAUNCH("gqa_decode_flash_kernel");
     return RMLK_OK;
+}
+
+// CTAs per problem: as many as keep the whole launch resident at once (4 per SM for head sizes up to 64, else 2), at most 8 and at
+// least two blocks of keys each - below that the exchange at the end costs what the shorter walk saves.
+template <int LPR, bool PAIRS>
+static int attn_flash_launch(cudaStream_t st, const AttnParams& p, int64_t problems) {
+    const int64_t room = static_cast<int64_t>(sm_count()) * (LPR <= 16 ? 4 : 2), blocks = ceil_div64(p.T, FL_KEYS);
+    int ctas = 1;
+    while (ctas < 8 && problems * ctas * 2 <= room && blocks >= 4 * ctas) ctas *= 2;
+    if (ctas > 1) return attn_flash_launch_as<LPR, true, PAIRS>(st, p, problems, ctas);
+    return attn_flash_launch_as<LPR, false, PAIRS>(st, p, problems, 1);
 }
 
 // RMLK_B200_ATTENTION_FLASH=0: the one-launch attention falls back to the two-pass kernels (scores of all keys in shared
@@ -695,10 +825,10 @@ extern "C" int rmlk_b200_gqa_decode_attention(rmlk_stream_t stream, int dtype, i
     cudaStream_t st = as_stream(stream);
     if (attn_flash_enabled()) {
         switch (head_dim) {
-            case 16: return attn_flash_launch<4>(st, p, problems);
-            case 32: return attn_flash_launch<8>(st, p, problems);
-            case 64: return attn_flash_launch<16>(st, p, problems);
-            default: return attn_flash_launch<32>(st, p, problems);
+            case 16: return attn_flash_launch<4, false>(st, p, problems);
+            case 32: return attn_flash_launch<8, false>(st, p, problems);
+            case 64: return attn_flash_launch<16, false>(st, p, problems);
+            default: return attn_flash_launch<32, false>(st, p, problems);
         }
     }
     switch (head_dim) {
@@ -708,6 +838,33 @@ extern "C" int rmlk_b200_gqa_decode_attention(rmlk_stream_t stream, int dtype, i
         default: return attn_launch<32>(st, p, problems);
     }
 }
+
+namespace rmlk {
+int gqa_decode_attention_pairs(cudaStream_t st, int64_t problems, int64_t rows, int64_t head_dim, int64_t keys, int64_t kv_heads, const float* q, const float* k,
+                               int64_t kb, const float* v, int64_t vb, float scale, const float* mask, int64_t ms_b, int64_t ms_h, const SplitRows& out) {
+    if (out.chunk_blocks * 64 != rows * head_dim) return fail(RMLK_ERR_INTERNAL, "gqa_decode_attention: one scale per KV head needs rows x head_dim in multiples of 64");
+    AttnParams p = {};
+    p.q = q;
+    p.k = k;
+    p.v = v;
+    p.mask = mask;
+    p.kb = kb;
+    p.vb = vb;
+    p.ms_b = ms_b;
+    p.ms_h = ms_h;
+    p.rows = static_cast<int>(rows);
+    p.T = static_cast<int>(keys);
+    p.kv_heads = static_cast<int>(kv_heads);
+    p.scale = scale;
+    p.pairs = out;
+    switch (head_dim) {
+        case 16: return attn_flash_launch<4, true>(st, p, problems);
+        case 32: return attn_flash_launch<8, true>(st, p, problems);
+        case 64: return attn_flash_launch<16, true>(st, p, problems);
+        default: return attn_flash_launch<32, true>(st, p, problems);
+    }
+}
+}  // namespace rmlk
 
 extern "C" size_t rmlk_b200_gqa_decode_attention_workspace_bytes(int64_t problems, int64_t rows, int64_t head_dim, int64_t keys) {
     if (!rmlk_b200_gqa_decode_attention_supported(rows, head_dim, keys) || problems <= 0 || keys <= SPLIT_KEYS) return 0;

@@ -14,6 +14,7 @@
 // mul.rs, slice.rs (x2), neg.rs, concat.rs, add.rs; sigmoid.rs, mul.rs (x2); mul.rs, add.rs, softmax.rs
 // (all under runtime/src/providers/cuda/backend/).
 #include "common.cuh"
+#include "split_pair.cuh"
 
 namespace rmlk {
 
@@ -88,18 +89,24 @@ __global__ void __launch_bounds__(256) rmsnorm_f32_kernel(int64_t cols, float ex
 // Same, for rows of up to THREADS * 4 * NP elements with 16-byte alignment: the row is read once and held in registers.
 // A few rows (a decode step: 64) take 512 or 1024 threads with one pack each, so that the row, the residual and all
 // split-K slabs of a pack are requested at once - one trip to memory instead of several; many rows take 256 threads.
-template <int NP, int THREADS>
+// PAIRS: the normalised row goes out as pairs of f16 for the tensor-core MatMul that reads it (its scale from the largest
+// |x w| / sd, found in the same pass as the sum) instead of as fp32.
+template <int NP, int THREADS, bool PAIRS>
 __global__ void __launch_bounds__(THREADS) rmsnorm_f32_regs_kernel(int cols, float exponent, float eps, const float* __restrict__ x,
-                                                                  const float* __restrict__ w, float* __restrict__ out, RowAdd ra) {
-    dep_sync();
+                                                                  const float* __restrict__ w, float* __restrict__ out, SplitRows pairs, RowAdd ra) {
+    dep_trigger();
+    const float4* wv = reinterpret_cast<const float4*>(w);
+    const int packs = cols / 4;
+    dep_wait();
     __shared__ double part[THREADS / 32];
+    __shared__ uint32_t part_max[THREADS / 32];
     const int64_t r0 = static_cast<int64_t>(blockIdx.x) * cols;
     const float4* row = reinterpret_cast<const float4*>(x + r0);
     float4* dst = reinterpret_cast<float4*>(out + r0);
-    const float4* wv = reinterpret_cast<const float4*>(w);
-    const int packs = cols / 4;
     float4 v[NP];
     double acc = 0.0;
+    uint32_t mx = 0;
+    const bool square = exponent == 2.0f;  // powf(v, 2) is v * v rounded once; the product is a tenth of the instructions
 #pragma unroll
     for (int i = 0; i < NP; i++) {
         const int c = threadIdx.x + THREADS * i;
@@ -130,20 +137,45 @@ __global__ void __launch_bounds__(THREADS) rmsnorm_f32_regs_kernel(int cols, flo
                 v[i].w = __fadd_rn(v[i].w, y.w);
                 *reinterpret_cast<float4*>(ra.sum + r0 + 4 * c) = v[i];
             }
-            acc += static_cast<double>(powf(v[i].x, exponent));
-            acc += static_cast<double>(powf(v[i].y, exponent));
-            acc += static_cast<double>(powf(v[i].z, exponent));
-            acc += static_cast<double>(powf(v[i].w, exponent));
+            if (square) {
+                acc += static_cast<double>(__fmul_rn(v[i].x, v[i].x));
+                acc += static_cast<double>(__fmul_rn(v[i].y, v[i].y));
+                acc += static_cast<double>(__fmul_rn(v[i].z, v[i].z));
+                acc += static_cast<double>(__fmul_rn(v[i].w, v[i].w));
+            } else {
+                acc += static_cast<double>(powf(v[i].x, exponent));
+                acc += static_cast<double>(powf(v[i].y, exponent));
+                acc += static_cast<double>(powf(v[i].z, exponent));
+                acc += static_cast<double>(powf(v[i].w, exponent));
+            }
+            if constexpr (PAIRS) {
+                const float4 g = wv[c];
+                mx = max(max(mx, max(finite_abs_bits(v[i].x * g.x), finite_abs_bits(v[i].y * g.y))),
+                         max(finite_abs_bits(v[i].z * g.z), finite_abs_bits(v[i].w * g.w)));
+            }
         }
     }
     acc = warp_sum_d(acc);
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
+    if constexpr (PAIRS) mx = __reduce_max_sync(0xffffffffu, mx);
+    if ((threadIdx.x & 31) == 0) {
+        part[threadIdx.x >> 5] = acc;
+        if constexpr (PAIRS) part_max[threadIdx.x >> 5] = mx;
+    }
     __syncthreads();
     double total = 0.0;
 #pragma unroll
     for (int i = 0; i < THREADS / 32; i++) total += part[i];
     const float mean = static_cast<float>(total / static_cast<double>(cols));
     const float sd = sqrtf(__fadd_rn(mean, eps));
+    float scale = 1.f;
+    if constexpr (PAIRS) {
+        uint32_t top = 0;
+#pragma unroll
+        for (int i = 0; i < THREADS / 32; i++) top = max(top, part_max[i]);
+        const int e = scale_exponent(finite_abs_bits(__fdiv_rn(__uint_as_float(top), sd)));
+        scale = exp2_int(e);
+        if (threadIdx.x == 0) pairs.scale[blockIdx.x] = exp2_int(-e);
+    }
 #pragma unroll
     for (int i = 0; i < NP; i++) {
         const int c = threadIdx.x + THREADS * i;
@@ -154,7 +186,8 @@ __global__ void __launch_bounds__(THREADS) rmsnorm_f32_regs_kernel(int cols, flo
             r.y = __fmul_rn(__fdiv_rn(v[i].y, sd), g.y);
             r.z = __fmul_rn(__fdiv_rn(v[i].z, sd), g.z);
             r.w = __fmul_rn(__fdiv_rn(v[i].w, sd), g.w);
-            dst[c] = r;
+            if constexpr (PAIRS) store_pairs4(pairs, blockIdx.x, 4 * c, r, scale);
+            else dst[c] = r;
         }
     }
 }
@@ -376,6 +409,51 @@ __global__ void __launch_bounds__(256) swiglu_f32_pitched_kernel(int64_t rows, i
     *reinterpret_cast<float4*>(out + r * cols + c) = o;
 }
 
+template <int NP, int THREADS>
+__global__ void __launch_bounds__(THREADS) swiglu_pairs_kernel(int cols, const float* __restrict__ g, int64_t ldg, const float* __restrict__ u, int64_t ldu, SplitRows pairs) {
+    dep_sync();
+    __shared__ uint32_t part_max[THREADS / 32];
+    const int64_t row = blockIdx.x;
+    const float4* gr = reinterpret_cast<const float4*>(g + row * ldg);
+    const float4* ur = reinterpret_cast<const float4*>(u + row * ldu);
+    const int packs = cols / 4;
+    float4 a[NP], b[NP];
+#pragma unroll
+    for (int i = 0; i < NP; i++) {
+        const int c = threadIdx.x + THREADS * i;
+        if (c < packs) {
+            a[i] = gr[c];
+            b[i] = ur[c];
+        }
+    }
+    uint32_t mx = 0;
+#pragma unroll
+    for (int i = 0; i < NP; i++) {
+        if (threadIdx.x + THREADS * i < packs) {
+            float4& r = a[i];
+            r.x = __fmul_rn(__fmul_rn(r.x, 1.0f / (1.0f + expf(-r.x))), b[i].x);
+            r.y = __fmul_rn(__fmul_rn(r.y, 1.0f / (1.0f + expf(-r.y))), b[i].y);
+            r.z = __fmul_rn(__fmul_rn(r.z, 1.0f / (1.0f + expf(-r.z))), b[i].z);
+            r.w = __fmul_rn(__fmul_rn(r.w, 1.0f / (1.0f + expf(-r.w))), b[i].w);
+            mx = max(max(mx, max(finite_abs_bits(r.x), finite_abs_bits(r.y))), max(finite_abs_bits(r.z), finite_abs_bits(r.w)));
+        }
+    }
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if ((threadIdx.x & 31) == 0) part_max[threadIdx.x >> 5] = mx;
+    __syncthreads();
+    uint32_t top = 0;
+#pragma unroll
+    for (int i = 0; i < THREADS / 32; i++) top = max(top, part_max[i]);
+    const int e = scale_exponent(top);
+    const float scale = exp2_int(e);
+    if (threadIdx.x == 0) pairs.scale[row] = exp2_int(-e);
+#pragma unroll
+    for (int i = 0; i < NP; i++) {
+        const int c = threadIdx.x + THREADS * i;
+        if (c < packs) store_pairs4(pairs, row, 4 * c, a[i], scale);
+    }
+}
+
 struct MaskParams {
     int64_t d[3];   // leading dims of the scores [d0, d1, d2, cols]
     int64_t ms[3];  // mask element strides for those dims (0 = broadcast); mask rows are dense
@@ -430,28 +508,61 @@ __global__ void __launch_bounds__(256) scale_mask_softmax_f32_kernel(MaskParams 
 
 using namespace rmlk;
 
+template <bool PAIRS>
+static void launch_rmsnorm_regs(cudaStream_t st, int64_t rows, int c, float exponent, float eps, const float* x, const float* w, float* out, const SplitRows& pairs,
+                                const RowAdd& ra) {
+    const unsigned grid = static_cast<unsigned>(rows);
+    const bool few = rows <= 512;  // too few rows to fill the GPU with 256-thread CTAs: widen the CTA instead
+    if (c <= 1024) launch_dep(rmsnorm_f32_regs_kernel<1, 256, PAIRS>, dim3(grid), dim3(256), 0, st, c, exponent, eps, x, w, out, pairs, ra);
+    else if (c <= 2048 && few) launch_dep(rmsnorm_f32_regs_kernel<1, 512, PAIRS>, dim3(grid), dim3(512), 0, st, c, exponent, eps, x, w, out, pairs, ra);
+    else if (c <= 2048) launch_dep(rmsnorm_f32_regs_kernel<2, 256, PAIRS>, dim3(grid), dim3(256), 0, st, c, exponent, eps, x, w, out, pairs, ra);
+    else if (few) launch_dep(rmsnorm_f32_regs_kernel<1, 1024, PAIRS>, dim3(grid), dim3(1024), 0, st, c, exponent, eps, x, w, out, pairs, ra);
+    else launch_dep(rmsnorm_f32_regs_kernel<4, 256, PAIRS>, dim3(grid), dim3(256), 0, st, c, exponent, eps, x, w, out, pairs, ra);
+}
+
+static bool rmsnorm_in_registers(int64_t cols, const void* x, const void* weight, const void* out, const RowAdd& ra) {
+    const bool add_ok = !ra.b || (aligned_to(ra.b, 16) && aligned_to(ra.sum, 16) && ra.part_stride % 4 == 0);
+    return cols % 4 == 0 && cols <= 4096 && aligned_to(x, 16) && aligned_to(weight, 16) && aligned_to(out, 16) && add_ok;
+}
+
 static int launch_rmsnorm(rmlk_stream_t stream, int64_t rows, int64_t cols, const void* x, float exponent, float eps, const void* weight,
                           void* out, const RowAdd& ra) {
     const float* xp = static_cast<const float*>(x);
     const float* wp = static_cast<const float*>(weight);
     float* op = static_cast<float*>(out);
     cudaStream_t st = as_stream(stream);
-    const unsigned grid = static_cast<unsigned>(rows);
-    const bool add_ok = !ra.b || (aligned_to(ra.b, 16) && aligned_to(ra.sum, 16) && ra.part_stride % 4 == 0);
-    if (cols % 4 == 0 && cols <= 4096 && aligned_to(x, 16) && aligned_to(weight, 16) && aligned_to(out, 16) && add_ok) {
-        const int c = static_cast<int>(cols);
-        const bool few = rows <= 512;  // too few rows to fill the GPU with 256-thread CTAs: widen the CTA instead
-        if (cols <= 1024) launch_dep(rmsnorm_f32_regs_kernel<1, 256>, dim3(grid), dim3(256), 0, st, c, exponent, eps, xp, wp, op, ra);
-        else if (cols <= 2048 && few) launch_dep(rmsnorm_f32_regs_kernel<1, 512>, dim3(grid), dim3(512), 0, st, c, exponent, eps, xp, wp, op, ra);
-        else if (cols <= 2048) launch_dep(rmsnorm_f32_regs_kernel<2, 256>, dim3(grid), dim3(256), 0, st, c, exponent, eps, xp, wp, op, ra);
-        else if (few) launch_dep(rmsnorm_f32_regs_kernel<1, 1024>, dim3(grid), dim3(1024), 0, st, c, exponent, eps, xp, wp, op, ra);
-        else launch_dep(rmsnorm_f32_regs_kernel<4, 256>, dim3(grid), dim3(256), 0, st, c, exponent, eps, xp, wp, op, ra);
-    } else {
-        launch_dep(rmsnorm_f32_kernel, dim3(grid), dim3(256), 0, st, cols, exponent, eps, xp, wp, op, ra);
-    }
+    if (rmsnorm_in_registers(cols, x, weight, out, ra)) launch_rmsnorm_regs<false>(st, rows, static_cast<int>(cols), exponent, eps, xp, wp, op, SplitRows(), ra);
+    else launch_dep(rmsnorm_f32_kernel, dim3(static_cast<unsigned>(rows)), dim3(256), 0, st, cols, exponent, eps, xp, wp, op, ra);
     RMLK_CHECK_LAUNCH("rmsnorm_f32_kernel");
     return RMLK_OK;
 }
+
+namespace rmlk {
+bool rmsnorm_pairs_supported(int64_t rows, int64_t cols, const float* x, const float* b, int b_parts, const float* weight) {
+    const RowAdd ra = {b, nullptr, b_parts, b_parts > 1 ? rows * cols : 0};
+    return rows > 0 && rows <= 0x7fffffffll && cols % 64 == 0 && rmsnorm_in_registers(cols, x, weight, nullptr, ra);
+}
+int rmsnorm_pairs(cudaStream_t st, int64_t rows, int64_t cols, const float* x, const float* b, int b_parts, float exponent, float eps, const float* weight, float* sum,
+                  const SplitRows& out) {
+    const RowAdd ra = {b, sum, b_parts, rows * cols};
+    launch_rmsnorm_regs<true>(st, rows, static_cast<int>(cols), exponent, eps, x, weight, nullptr, out, ra);
+    RMLK_CHECK_LAUNCH("rmsnorm_f32_kernel");
+    return RMLK_OK;
+}
+
+// SwiGLU gate of [rows, cols] blocks (row pitches ldg, ldu), written as pairs of f16: one CTA per row, the row in registers
+// between the search for its largest value and the stores.  cols % 64 == 0 and at most 16384.
+bool swiglu_pairs_supported(int64_t rows, int64_t cols) { return rows > 0 && rows <= 0x7fffffffll && cols % 64 == 0 && cols <= 16384; }
+int swiglu_pairs(cudaStream_t st, int64_t rows, int64_t cols, const float* gate, int64_t ldg, const float* up, int64_t ldu, const SplitRows& out) {
+    const unsigned grid = static_cast<unsigned>(rows);
+    const int c = static_cast<int>(cols);
+    if (cols <= 2048) launch_dep(swiglu_pairs_kernel<2, 256>, dim3(grid), dim3(256), 0, st, c, gate, ldg, up, ldu, out);
+    else if (cols <= 8192) launch_dep(swiglu_pairs_kernel<2, 1024>, dim3(grid), dim3(1024), 0, st, c, gate, ldg, up, ldu, out);
+    else launch_dep(swiglu_pairs_kernel<4, 1024>, dim3(grid), dim3(1024), 0, st, c, gate, ldg, up, ldu, out);
+    RMLK_CHECK_LAUNCH("swiglu_pairs_kernel");
+    return RMLK_OK;
+}
+}  // namespace rmlk
 
 extern "C" int rmlk_b200_rmsnorm(rmlk_stream_t stream, int dtype, int64_t rows, int64_t cols, const void* x, float exponent, float eps,
                                  const void* weight, void* out) {

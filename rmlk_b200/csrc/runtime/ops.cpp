@@ -95,6 +95,7 @@ struct Ctx {
     // Input i as a dense tensor; a deferred view is copied out first.
     Tensor* in(size_t i) const {
         Tensor* t = raw(i);
+        if (t && t->pairs) raise(RMLK_ERR_INTERNAL, "value `" + I.g.values[n.inputs[i]].name + "` is only kept for packed MatMuls");
         if (t && t->lazy) I.materialize(*t);
         return t;
     }
@@ -130,6 +131,7 @@ struct Ctx {
         o.mf.clear();
         o.lazy = false;
         o.parts = 0;
+        o.pairs = false;
         I.alloc_output(n.outputs[i], o);
         o.present = true;
         return o;
@@ -145,6 +147,8 @@ struct Ctx {
         o.mi = src.mi;
         o.mf = src.mf;
         o.parts = 0;
+        o.pairs = src.pairs;
+        o.split = src.split;
         if (bound) {  // a carried output must own its storage
             I.alloc_output(vid, o);
             if (o.nbytes()) check_cuda(cudaMemcpyAsync(o.data, src.data, o.nbytes(), cudaMemcpyDeviceToDevice, I.stream), "view copy");
@@ -170,6 +174,8 @@ struct Ctx {
         o.mi.clear();
         o.mf.clear();
         o.parts = 0;
+        o.pairs = base.pairs;
+        o.split = base.split;
         o.data = base.data;
         o.storage = base.storage;
         if (o.storage) o.storage->refs++;
@@ -691,8 +697,81 @@ void op_gemm(const Ctx& c) {
     }
 }
 
+// An output the host is waiting for (logits): the product is issued in blocks of columns - one wave of 128-column tiles, then two
+// waves each - and every block goes to the host on the copy stream while the next is computed.
+std::vector<int64_t> host_output_blocks(const Ctx& c, int64_t n) {
+    int sm_attr = 148;
+    cudaDeviceGetAttribute(&sm_attr, cudaDevAttrMultiProcessorCount, c.I.device);
+    const int64_t sms = sm_attr > 0 ? sm_attr : 148, tiles = n / 128;
+    std::vector<int64_t> blocks;
+    for (int64_t left = tiles, first = 1; left > 0; first = 0) {
+        int64_t take = std::min<int64_t>(left, first ? sms : 2 * sms);
+        if (left - take < sms) take = left;  // a short tail joins the last block
+        blocks.push_back(take);
+        left -= take;
+    }
+    return blocks;
+}
+
+// Columns [n0, n0 + nc) of `o` (block i of the product) to the host behind what the stream holds so far.
+void send_columns(const Ctx& c, int hout, size_t i, const Tensor& o, int64_t rows, int64_t n, int64_t n0, int64_t nc) {
+    while (c.I.copy_events.size() <= i) {
+        cudaEvent_t e = nullptr;
+        check_cuda(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
+        c.I.copy_events.push_back(e);
+    }
+    check_cuda(cudaEventRecord(c.I.copy_events[i], c.I.stream), "cudaEventRecord");
+    check_cuda(cudaStreamWaitEvent(c.I.copy_stream, c.I.copy_events[i], 0), "cudaStreamWaitEvent");
+    check_cuda(cudaMemcpy2DAsync(static_cast<char*>(c.I.host_outputs[hout].dst) + n0 * 4, static_cast<size_t>(n) * 4, static_cast<const float*>(o.data) + n0,
+                                 static_cast<size_t>(n) * 4, static_cast<size_t>(nc) * 4, static_cast<size_t>(rows), cudaMemcpyDeviceToHost, c.I.copy_stream),
+               "host output D2H");
+}
+
+// MatMul against weights kept as pairs of f16.
+void matmul_packed(const Ctx& c, PackedWeights& pw, const Tensor& a, int64_t rows, int64_t n, Tensor& o) {
+    Instance& I = c.I;
+    const int ovid = c.n.outputs[0];
+    const SplitRows x = I.split_left_operand(a, rows, pw.k);
+    float* out = static_cast<float*>(o.data);
+    if (I.parts_owner < 0 && ovid < static_cast<int>(I.parts_ok_value.size()) && I.parts_ok_value[ovid]) {
+        // the only reader is a residual Add + RMSNorm chain whose kernel adds K splits itself
+        int parts = 1;
+        I.packed_product(pw, x, 0, n, out, n, &I.parts_ws, &parts);
+        if (parts > 1) {
+            I.release_value(ovid);  // the dense buffer is not needed unless the chain falls back (settle_parts)
+            o.data = I.parts_ws.ptr;
+            o.parts = parts;
+            I.parts_owner = ovid;
+        }
+        return;
+    }
+    const int hout = I.host_output_of(ovid);
+    if (hout >= 0 && n % 128 == 0 && I.host_outputs[hout].nbytes == o.nbytes()) {
+        const std::vector<int64_t> blocks = host_output_blocks(c, n);
+        if (blocks.size() > 1) {
+            int64_t n0 = 0;
+            for (size_t i = 0; i < blocks.size(); i++) {
+                const int64_t nc = blocks[i] * 128;
+                I.packed_product(pw, x, n0, nc, out + n0, n, nullptr, nullptr);
+                send_columns(c, hout, i, o, rows, n, n0, nc);
+                n0 += nc;
+            }
+            I.host_outputs[hout].delivered_run = I.run_counter;
+            I.copies_pending = true;
+            return;
+        }
+    }
+    int parts = 1;
+    I.packed_product(pw, x, 0, n, out, n, &I.matmul_ws, &parts);
+    if (parts > 1) {
+        check_rc(rmlk_b200_sum_parts(c.stream(), RMLK_F32, parts, rows * n, I.matmul_ws.ptr, out));
+        c.launched();
+    }
+}
+
 void op_matmul(const Ctx& c) {
-    Tensor& a = c.req(0);
+    Tensor* araw = c.raw(0);
+    Tensor& a = araw && araw->pairs ? *araw : c.req(0);  // pairs: its producer has made sure that packed_for takes this node
     Tensor* braw = c.raw(1);
     if (!braw) raise(RMLK_ERR_INVALID_ARG, "missing input 1");
     Tensor& b = *braw;  // may be a deferred view; made dense below unless the kernels can read it as it is
@@ -750,8 +829,16 @@ void op_matmul(const Ctx& c) {
         sa = sb = 0;
         sc = em * n;
     }
-    const size_t need = rmlk_b200_matmul_workspace_bytes(a.dtype, eb, em, n, ka);
     const int ovid = c.n.outputs[0];
+    if (a.dtype == RMLK_F32 && eb == 1)
+        if (PackedWeights* pw = c.I.packed_for(static_cast<int>(&c.n - c.I.g.nodes.data()), em)) {
+            if (pw->weight_values.size() == 1 && pw->n_total == n && pw->k == ka) {
+                matmul_packed(c, *pw, a, em, n, o);
+                return;
+            }
+        }
+    if (a.pairs) raise(RMLK_ERR_INTERNAL, "matmul: left operand kept as pairs, but the packed product does not apply");
+    const size_t need = rmlk_b200_matmul_workspace_bytes(a.dtype, eb, em, n, ka);
     // initializers were uploaded before the first run: nothing in flight writes them
     const int flags = c.I.g.values[c.n.inputs[1]].is_const ? RMLK_MATMUL_B_STATIC : 0;
     if (need && a.dtype == RMLK_F32 && eb == 1 && c.I.parts_owner < 0 && ovid < static_cast<int>(c.I.parts_ok_value.size()) && c.I.parts_ok_value[ovid]) {
@@ -772,40 +859,19 @@ void op_matmul(const Ctx& c) {
     }
     const int hout = c.I.host_output_of(ovid);
     if (hout >= 0 && !need && a.dtype == RMLK_F32 && eb == 1 && n % 128 == 0 && c.I.host_outputs[hout].nbytes == o.nbytes()) {
-        // An output the host is waiting for (logits): the product is issued in blocks of columns - one wave of tiles,
-        // then two waves each - and every block goes to the host on the copy stream while the next is computed.
-        int sm_attr = 148;
-        cudaDeviceGetAttribute(&sm_attr, cudaDevAttrMultiProcessorCount, c.I.device);
-        const int64_t sms = sm_attr > 0 ? sm_attr : 148, tiles = n / 128;
-        std::vector<int64_t> blocks;
-        for (int64_t left = tiles, first = 1; left > 0; first = 0) {
-            int64_t take = std::min<int64_t>(left, first ? sms : 2 * sms);
-            if (left - take < sms) take = left;  // a short tail joins the last block
-            blocks.push_back(take);
-            left -= take;
-        }
+        const std::vector<int64_t> blocks = host_output_blocks(c, n);
         bool ok = blocks.size() > 1;
         for (int64_t bt : blocks) ok = ok && rmlk_b200_matmul_window_supported(em, bt * 128, ka, n);
         if (ok) {
-            HostOutput& h = c.I.host_outputs[hout];
-            while (c.I.copy_events.size() < blocks.size()) {
-                cudaEvent_t e = nullptr;
-                check_cuda(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
-                c.I.copy_events.push_back(e);
-            }
             int64_t n0 = 0;
             for (size_t i = 0; i < blocks.size(); i++) {
                 const int64_t nc = blocks[i] * 128;
                 check_rc(rmlk_b200_matmul_window(c.stream(), a.dtype, em, nc, ka, a.data, static_cast<const float*>(b.data) + n0,
                                                  static_cast<float*>(o.data) + n0, n, static_cast<int*>(c.I.status_word.ptr), flags));
-                check_cuda(cudaEventRecord(c.I.copy_events[i], c.I.stream), "cudaEventRecord");
-                check_cuda(cudaStreamWaitEvent(c.I.copy_stream, c.I.copy_events[i], 0), "cudaStreamWaitEvent");
-                check_cuda(cudaMemcpy2DAsync(static_cast<char*>(h.dst) + n0 * 4, static_cast<size_t>(n) * 4, static_cast<const float*>(o.data) + n0,
-                                             static_cast<size_t>(n) * 4, static_cast<size_t>(nc) * 4, static_cast<size_t>(em), cudaMemcpyDeviceToHost,
-                                             c.I.copy_stream), "host output D2H");
+                send_columns(c, hout, i, o, em, n, n0, nc);
                 n0 += nc;
             }
-            h.delivered_run = c.I.run_counter;
+            c.I.host_outputs[hout].delivered_run = c.I.run_counter;
             c.I.copies_pending = true;
             c.I.status_dirty = true;
             c.launched(static_cast<int>(blocks.size()));
@@ -1897,7 +1963,17 @@ bool Instance::run_fused(const FusedGroup& fg) {
             if (x->lazy) materialize(*x);
             const Shape oshape = x->shape;
             const int64_t rows = x->numel() / cols;
+            const int ov = root.outputs[0];
+            const bool pairs = !x->pairs && rmsnorm_pairs_supported(rows, cols, static_cast<const float*>(x->data), with_add ? static_cast<const float*>(rb->data) : nullptr,
+                                                                    with_add && rb->parts > 1 ? rb->parts : 1, static_cast<const float*>(w->data)) &&
+                               !(with_add && rb->lazy) && pairs_wanted(ov, rows, cols, false);
             if (!with_add) {
+                if (pairs) {
+                    Tensor& o = make_pairs(ov, oshape, rows, cols, 0);
+                    check_rc(rmsnorm_pairs(stream, rows, cols, static_cast<const float*>(x->data), nullptr, 1, p, e, static_cast<const float*>(w->data), nullptr, o.split));
+                    launches++;
+                    return true;
+                }
                 Tensor& o = c.make(0, RMLK_F32, oshape);
                 check_rc(rmlk_b200_rmsnorm(st, RMLK_F32, rows, cols, x->data, p, e, w->data, o.data));
                 launches++;
@@ -1912,11 +1988,18 @@ bool Instance::run_fused(const FusedGroup& fg) {
             sum.mf.clear();
             sum.lazy = false;
             sum.parts = 0;
+            sum.pairs = false;
             alloc_output(fg.v[0], sum);
             sum.present = true;
-            Tensor& o = c.make(0, RMLK_F32, oshape);
             const int parts = rb->parts > 1 ? rb->parts : 1;
-            check_rc(rmlk_b200_add_rmsnorm(st, RMLK_F32, rows, cols, ra->data, rb->data, parts, rows * cols, p, e, w->data, sum.data, o.data));
+            if (pairs) {
+                Tensor& o = make_pairs(ov, oshape, rows, cols, 0);
+                check_rc(rmsnorm_pairs(stream, rows, cols, static_cast<const float*>(ra->data), static_cast<const float*>(rb->data), parts, p, e,
+                                       static_cast<const float*>(w->data), static_cast<float*>(sum.data), o.split));
+            } else {
+                Tensor& o = c.make(0, RMLK_F32, oshape);
+                check_rc(rmlk_b200_add_rmsnorm(st, RMLK_F32, rows, cols, ra->data, rb->data, parts, rows * cols, p, e, w->data, sum.data, o.data));
+            }
             launches++;
             if (rb->parts > 1) {  // the slabs have been consumed
                 rb->parts = 0;
@@ -1950,6 +2033,18 @@ bool Instance::run_fused(const FusedGroup& fg) {
             int64_t pg = 0, pu = 0;
             const bool pitched = (gt->lazy || up->lazy) && !gt->shape.empty() && gt->shape.back() % 4 == 0 && as_rows(*gt, pg) && as_rows(*up, pu) &&
                                  pg % 4 == 0 && pu % 4 == 0 && reinterpret_cast<uintptr_t>(gt->data) % 16 == 0 && reinterpret_cast<uintptr_t>(up->data) % 16 == 0;
+            if (!gt->shape.empty() && as_rows(*gt, pg) && as_rows(*up, pu) && pg % 4 == 0 && pu % 4 == 0 && reinterpret_cast<uintptr_t>(gt->data) % 16 == 0 &&
+                reinterpret_cast<uintptr_t>(up->data) % 16 == 0) {
+                const int64_t cols = gt->shape.back(), rows = cols ? gt->numel() / cols : 0;
+                if (swiglu_pairs_supported(rows, cols) && pairs_wanted(root.outputs[0], rows, cols, false)) {
+                    const Shape shape = gt->shape;
+                    const float *gd = static_cast<const float*>(gt->data), *ud = static_cast<const float*>(up->data);
+                    Tensor& o = make_pairs(root.outputs[0], shape, rows, cols, 0);
+                    check_rc(swiglu_pairs(stream, rows, cols, gd, pg, ud, pu, o.split));
+                    launches++;
+                    return true;
+                }
+            }
             if (!pitched) {
                 if (gt->lazy) materialize(*gt);
                 if (up->lazy) materialize(*up);
@@ -2020,6 +2115,14 @@ bool Instance::run_fused(const FusedGroup& fg) {
             if (mk->shape.size() > 4 || mk->shape.empty() || mk->shape.back() != T || !bcast_strides(*mk, sshape, ms) || (T > 1 && ms[3] != 1)) return false;
             if (q->lazy) materialize(*q);
             const void *kdata = kt->data, *vdata = vh->data;
+            if (!attention_split && (lk.fold * D) % 64 == 0 && pairs_wanted(root.outputs[0], B, H * D, true)) {
+                const float* qd = static_cast<const float*>(q->data);
+                Tensor& o = make_pairs(root.outputs[0], Shape({B, H, 1, D}), B, H * D, static_cast<int>(lk.fold * D / 64));
+                check_rc(gqa_decode_attention_pairs(stream, lk.outer, lk.fold, D, T, H / lk.fold, qd, static_cast<const float*>(kdata), lk.sb,
+                                                    static_cast<const float*>(vdata), lv.sb, scale, static_cast<const float*>(mk->data), ms[0], ms[1], o.split));
+                launches++;
+                return true;
+            }
             Tensor& o = c.make(0, RMLK_F32, Shape({B, H, 1, D}));
             // one CTA per problem in one pass over K and V by default; RMLK_B200_ATTENTION=split: keys split over CTAs, merged through a workspace
             const size_t ws_need = attention_split ? rmlk_b200_gqa_decode_attention_workspace_bytes(lk.outer, lk.fold, D, T) : 0;
@@ -2244,6 +2347,26 @@ bool Instance::run_merged_matmul(int node_index) {
         if (!w.present || w.lazy || w.dtype != RMLK_F32 || w.shape.size() != 2 || w.shape[0] != mm.k || w.shape[1] != mm.n[j]) return false;
     }
     if (a.lazy) materialize(a);
+    const int64_t rows = a.numel() / mm.k;
+    Storage* y = arena->alloc(static_cast<size_t>(rows) * mm.n_total * sizeof(float));
+    if (PackedWeights* pw = packed_for(node_index, rows)) {
+        const SplitRows x = split_left_operand(a, rows, mm.k);
+        int parts = 1;
+        packed_product(*pw, x, 0, mm.n_total, static_cast<float*>(y->ptr), mm.n_total, &matmul_ws, &parts);
+        if (parts > 1 && batch_jobs && rows <= 64) {
+            // decode-sized product: the K splits stay unsummed for the placements that read them (Instance::unsummed)
+            unsummed.y = y;
+            unsummed.slabs = static_cast<const float*>(matmul_ws.ptr);
+            unsummed.parts = parts;
+            unsummed.part_stride = rows * mm.n_total;
+            y->refs++;
+        } else if (parts > 1) {
+            check_rc(rmlk_b200_sum_parts(reinterpret_cast<rmlk_stream_t>(stream), RMLK_F32, parts, rows * mm.n_total, matmul_ws.ptr, y->ptr));
+            launches++;
+        }
+        hand_out_merged(mm, a, rows, y);
+        return true;
+    }
     const int flags = mm.ready ? RMLK_MATMUL_B_STATIC : 0;  // from the second run on nothing in flight writes the weights
     if (!mm.ready) {
         char* dst = static_cast<char*>(mm.w.ensure(static_cast<size_t>(mm.k) * mm.n_total * sizeof(float)));
@@ -2254,8 +2377,6 @@ bool Instance::run_merged_matmul(int node_index) {
         }
         mm.ready = true;
     }
-    const int64_t rows = a.numel() / mm.k;
-    Storage* y = arena->alloc(static_cast<size_t>(rows) * mm.n_total * sizeof(float));
     const size_t need = rmlk_b200_matmul_workspace_bytes(RMLK_F32, 1, rows, mm.n_total, mm.k);
     void* ws = need ? matmul_ws.ensure(need) : nullptr;
     if (batch_jobs && rows <= 64) {
@@ -2277,6 +2398,12 @@ bool Instance::run_merged_matmul(int node_index) {
         launches += need ? 2 : 1;
     }
     status_dirty = true;
+    hand_out_merged(mm, a, rows, y);
+    return true;
+}
+
+// Every member's output: its block of columns of the product in `y`, as a view.
+void Instance::hand_out_merged(MergedMatMul& mm, const Tensor& a, int64_t rows, Storage* y) {
     for (size_t j = 0; j < mm.nodes.size(); j++) {
         Tensor& o = values[g.nodes[mm.nodes[j]].outputs[0]];
         o.dtype = RMLK_F32;
@@ -2298,7 +2425,180 @@ bool Instance::run_merged_matmul(int node_index) {
         o.present = true;
     }
     mm.done_in_run = run_counter;
+}
+
+// ---------------------------------------------------------------------------------------------
+// MatMul against weights kept as pairs of f16
+// ---------------------------------------------------------------------------------------------
+void Instance::find_packable() {
+    packed.clear();
+    packed_of_node.assign(g.nodes.size(), -1);
+    std::map<int, int> by_weight;
+    std::vector<int> of_group(merged.size(), -1);
+    for (size_t i = 0; i < g.nodes.size(); i++) {
+        const NodeDef& n = g.nodes[i];
+        if (n.op != RMLK_OP_MATMUL || n.inputs.size() < 2 || n.outputs.empty() || n.inputs[0] < 0 || n.inputs[1] < 0) continue;
+        const int gi = merged_of_node.empty() ? -1 : merged_of_node[i];
+        if (gi >= 0 && of_group[gi] >= 0) {
+            packed_of_node[i] = of_group[gi];
+            continue;
+        }
+        PackedWeights pw;
+        if (gi >= 0) {
+            if (merged[gi].nodes.size() > 4) continue;
+            for (int m : merged[gi].nodes) pw.weight_values.push_back(g.nodes[m].inputs[1]);
+        } else {
+            pw.weight_values.push_back(n.inputs[1]);
+        }
+        bool ok = true;
+        for (int v : pw.weight_values) {
+            const ValueDef& w = g.values[v];
+            ok = ok && w.is_const && w.dtype == RMLK_F32 && w.dims.size() == 2 && w.dims[0] >= 64 && w.dims[1] >= 64;
+            if (!ok) break;
+            pw.k = w.dims[0];
+            pw.n.push_back(w.dims[1]);
+            pw.col0.push_back(pw.n_total);
+            pw.n_total += w.dims[1];
+        }
+        if (!ok || ceil_div64(pw.n_total, 128) * ceil_div64(pw.k, 64) * 256 >= (1ll << 31) || ceil_div64(pw.k, 64) > 65535) continue;
+        if (gi < 0) {
+            auto it = by_weight.find(n.inputs[1]);
+            if (it != by_weight.end()) {
+                packed_of_node[i] = it->second;
+                continue;
+            }
+            by_weight[n.inputs[1]] = static_cast<int>(packed.size());
+        } else {
+            of_group[gi] = static_cast<int>(packed.size());
+        }
+        packed_of_node[i] = static_cast<int>(packed.size());
+        packed.push_back(std::move(pw));
+    }
+}
+
+// The node's weights as pairs of f16 if this many rows are to be multiplied that way, laid out now if they have not been.
+PackedWeights* Instance::packed_for(int node_index, int64_t rows) {
+    if (rows < PACKED_MIN_ROWS || node_index < 0 || node_index >= static_cast<int>(packed_of_node.size()) || packed_of_node[node_index] < 0 || packed_state < 0 ||
+        rows >= (1ll << 24) || !tc_enabled() || !tc::encode_fn())
+        return nullptr;
+    PackedWeights& pw = packed[packed_of_node[node_index]];
+    if (packed_state == 0) {
+        size_t total = 0;
+        for (PackedWeights& p : packed) {
+            p.offset = total;
+            total += (split_weights_bytes(p.n_total, p.k) + 1023) & ~size_t(1023);
+        }
+        void* ptr = nullptr;
+        if ((flush_deferred(), cudaMalloc(&ptr, total)) != cudaSuccess) {
+            cudaGetLastError();
+            packed_state = -1;
+            return nullptr;
+        }
+        packed_store.ptr = ptr;
+        packed_store.cap = total;
+        packed_state = 1;
+    }
+    if (pw.packed_run < 0) {
+        pw.w = split_weights_at(static_cast<char*>(packed_store.ptr) + pw.offset, pw.n_total, pw.k);
+        WeightSources src = {};
+        src.count = static_cast<int>(pw.weight_values.size());
+        for (int j = 0; j < src.count; j++) {
+            const Tensor& w = values[pw.weight_values[j]];
+            if (!w.present || w.lazy || w.numel() != pw.k * pw.n[j]) return nullptr;
+            src.w[j] = static_cast<const float*>(w.data);
+            src.n[j] = pw.n[j];
+            src.col0[j] = pw.col0[j];
+            src.vec[j] = pw.n[j] % 4 == 0 && pw.col0[j] % 4 == 0 && reinterpret_cast<uintptr_t>(w.data) % 16 == 0;
+        }
+        check_rc(split_weights_pack(stream, src, pw.w));
+        launches += 2;
+        pw.packed_run = run_counter;
+    }
+    return &pw;
+}
+
+// Who reads which value as the left operand of packable MatMuls and nothing else.
+void Instance::find_pairs() {
+    pairs_readers.assign(g.values.size(), {});
+    pairs_through.assign(g.values.size(), 0);
+    if (!fusion) return;
+    std::vector<std::vector<int>> readers(g.values.size());
+    for (size_t i = 0; i < g.nodes.size(); i++)
+        for (int v : g.nodes[i].inputs)
+            if (v >= 0) readers[v].push_back(static_cast<int>(i));
+    auto plain = [&](int v) { return !g.values[v].is_output && !g.values[v].is_input && !g.values[v].is_const && binding_of_out[v] < 0; };
+    for (size_t v = 0; v < g.values.size(); v++) {
+        int at = static_cast<int>(v);
+        bool through = false;
+        // [B, heads, 1, D] -> Transpose -> Reshape -> [B, 1, heads D]
+        while (plain(at) && readers[at].size() == 1) {
+            const NodeDef& n = g.nodes[readers[at][0]];
+            if ((n.op != RMLK_OP_TRANSPOSE && n.op != RMLK_OP_RESHAPE) || n.inputs[0] != at || n.outputs.empty()) break;
+            at = n.outputs[0];
+            through = true;
+        }
+        bool ok = plain(static_cast<int>(v)) && plain(at) && !readers[at].empty();
+        for (int r : readers[at]) {
+            const NodeDef& n = g.nodes[r];
+            ok = ok && n.op == RMLK_OP_MATMUL && n.inputs.size() == 2 && n.inputs[0] == at && n.inputs[1] != at && packed_of_node[r] >= 0 && group_of_node[r] < 0;
+        }
+        if (!ok) continue;
+        pairs_readers[v] = readers[at];
+        pairs_through[v] = through;
+    }
+}
+
+// May this run's producer of `value_id` ([rows, k] as MatMul sees it) write pairs instead of fp32?
+bool Instance::pairs_wanted(int value_id, int64_t rows, int64_t k, bool through) {
+    if (value_id < 0 || value_id >= static_cast<int>(pairs_readers.size()) || pairs_readers[value_id].empty() || (pairs_through[value_id] != 0) != through) return false;
+    for (int r : pairs_readers[value_id]) {
+        const PackedWeights* pw = packed_for(r, rows);
+        if (!pw || pw->k != k) return false;
+    }
     return true;
+}
+
+Tensor& Instance::make_pairs(int value_id, const std::vector<int64_t>& shape, int64_t rows, int64_t k, int chunk_blocks) {
+    Tensor& o = values[value_id];
+    o = Tensor();
+    o.dtype = RMLK_F32;
+    o.shape = shape;
+    o.storage = arena->alloc(split_rows_bytes(rows, k, chunk_blocks));
+    o.data = o.storage->ptr;
+    o.split = split_rows_at(o.data, rows, k, chunk_blocks);
+    o.pairs = true;
+    o.present = true;
+    return o;
+}
+
+SplitRows Instance::split_left_operand(const Tensor& t, int64_t rows, int64_t k) {
+    if (t.pairs) {
+        if (t.split.m != rows || t.split.k != k) raise(RMLK_ERR_INTERNAL, "matmul: left operand kept as pairs of another shape");
+        return t.split;
+    }
+    const float* a = static_cast<const float*>(t.data);
+    const SplitRows x = split_rows_at(x_split.ensure(split_rows_bytes(rows, k, 0)), rows, k, 0);
+    check_rc(split_rows_pack(stream, a, k, x));
+    launches++;
+    return x;
+}
+
+void Instance::packed_product(PackedWeights& pw, const SplitRows& x, int64_t n0, int64_t n, float* out, int64_t ldc, DeviceBuffer* slabs, int* parts) {
+    const SplitWeights w = n0 == 0 && n == pw.n_total ? pw.w : split_weights_window(pw.w, n0, n);
+    float* sp = nullptr;
+    size_t bytes = 0;
+    if (parts) {
+        const int want = umma_split_parts(x.m, n, x.k);
+        if (want > 1) {
+            bytes = static_cast<size_t>(want) * x.m * n * sizeof(float);
+            sp = static_cast<float*>(slabs->ensure(bytes));
+        }
+    }
+    // from the run after the one that laid them out nothing in flight writes the weights
+    const int flags = pw.packed_run < run_counter ? RMLK_MATMUL_B_STATIC : 0;
+    check_rc(umma_split(stream, x, w, out, ldc, sp, bytes, static_cast<int*>(status_word.ptr), flags, parts));
+    status_dirty = true;
+    launches++;
 }
 
 void Instance::run_node(const NodeDef& n) {

@@ -328,6 +328,8 @@ Instance::~Instance() {
     status_word.release();
     matmul_ws.release();
     parts_ws.release();
+    packed_store.release();
+    x_split.release();
     attn_ws.release();
     read_staging.release();
     if (copy_stream) {
@@ -503,6 +505,7 @@ void Instance::run() {
         values[i].data = nullptr;
         values[i].lazy = false;
         values[i].parts = 0;
+        values[i].pairs = false;
     }
     parts_owner = -1;
     if (copies_pending) {
@@ -837,6 +840,8 @@ extern "C" rmlk_instance* rmlk_instance_create(const rmlk_graph* g, int device, 
         }
         I.find_fusions();  // recognise RMSNorm / rotary / SwiGLU / scale-mask-softmax chains; re-derives last_use
         I.find_merged_matmuls();  // q / k / v and gate / up projections: one MatMul per shared left operand
+        I.find_packable();        // weights that the tensor-core MatMul reads in its own layout
+        I.find_pairs();           // values that only such MatMuls read
         I.find_foldable();        // nodes that depend on initializers only: computed in the first run, kept afterwards
         // one weight arena, one pass of uploads (the reference allocates and copies per tensor through a
         // 4 KiB bump allocator, runtime/src/providers/cuda/store.rs:95-262)

@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "../../../include/rmlk_b200_runtime.h"
+#include "../umma_gemm.h"
 
 namespace rmlk {
 namespace rt {
@@ -88,6 +89,10 @@ struct Tensor {
     // order); only ever set on a value whose single reader is the residual Add in front of an RMSNorm chain, which
     // adds the slabs itself.  Any other access goes through Instance::settle_parts first.
     int parts = 0;
+    // The value exists only as pairs of f16 (`split`, rows x last dims), written that way by its producer because every reader is a
+    // MatMul against packed weights.  Transpose / Reshape of one decoded token in between keep it so.
+    bool pairs = false;
+    SplitRows split = {};
     bool mirror_valid = false;
     std::vector<int64_t> mi;  // integer / bool mirror
     std::vector<double> mf;   // float mirror
@@ -184,6 +189,17 @@ struct MergedMatMul {
     int64_t done_in_run = -1;   // run counter of the run in which the first member produced every output
 };
 
+// Constant [K, N] right operands of MatMul laid out for the tensor cores as pairs of f16 (umma_pack.cu): a single node's weights,
+// or those of a merged group side by side.  Laid out on the device the first time a run brings enough rows, kept afterwards.
+struct PackedWeights {
+    std::vector<int> weight_values;
+    std::vector<int64_t> n, col0;
+    int64_t k = 0, n_total = 0;
+    size_t offset = 0;         // in Instance::packed_store
+    SplitWeights w = {};
+    int64_t packed_run = -1;   // run that laid them out
+};
+
 // A graph output that every run delivers to (pinned) host memory without being asked: the copy is enqueued as soon
 // as the value exists - for a wide MatMul (the logits) block of columns by block of columns on a second stream, so
 // that most of the transfer overlaps the rest of the product.  The reference copies outputs after the run
@@ -213,7 +229,27 @@ struct Instance {
     std::vector<int> merged_of_node;  // per node: index into `merged`, or -1
     int64_t run_counter = 0;
     void find_merged_matmuls();
+    std::vector<PackedWeights> packed;
+    std::vector<int> packed_of_node;   // per MatMul node: index into `packed`, or -1
+    DeviceBuffer packed_store;         // all of them, one allocation
+    int packed_state = 0;              // 0: not tried yet, 1: allocated, -1: no memory for them (the fp32 weights are used)
+    DeviceBuffer x_split;              // the left operand's pairs
+    // fewer rows stream the fp32 weights through the SIMT kernels at the HBM's speed
+    static constexpr int64_t PACKED_MIN_ROWS = 5;
+    void find_packable();
+    PackedWeights* packed_for(int node_index, int64_t rows);
+    // out[rows, n] = a x columns [n0, n0 + n) of the weights; with `parts`, K splits may be left in `slabs` (grown as needed)
+    void packed_product(PackedWeights& pw, const SplitRows& x, int64_t n0, int64_t n, float* out, int64_t ldc, DeviceBuffer* slabs, int* parts);
+    // Per value: the MatMul nodes that are its only readers, all against packable weights (empty: has other readers).  Where the value
+    // passes through Transpose and Reshape on its way, `pairs_through` is set and it may hold one row per batch entry only.
+    std::vector<std::vector<int>> pairs_readers;
+    std::vector<uint8_t> pairs_through;
+    void find_pairs();
+    bool pairs_wanted(int value_id, int64_t rows, int64_t k, bool through);
+    Tensor& make_pairs(int value_id, const std::vector<int64_t>& shape, int64_t rows, int64_t k, int chunk_blocks);
+    SplitRows split_left_operand(const Tensor& a, int64_t rows, int64_t k);
     bool run_merged_matmul(int node_index);
+    void hand_out_merged(MergedMatMul& mm, const Tensor& a, int64_t rows, Storage* y);
     std::vector<FusedGroup> groups;
     std::vector<int> group_of_node;  // per node: index into `groups`, or -1
     bool fusion = true;              // RMLK_B200_NO_FUSION=1 turns the substitution off

@@ -78,7 +78,8 @@ static Plan plan_for(int64_t m, int64_t n, int64_t k, int products, bool may_spl
         if (chunks && mt > 128) continue;  // the tall tiles take one scale per row
         const int64_t tiles = ceil_div64(n, BN * cg) * ceil_div64(m, mt), slots = sms / cg;
         int64_t ks = 1;
-        if (may_split && tiles < slots) {
+        // fewer than 16 k-blocks (K up to 960) are not split: adding up the parts costs more than the shorter loop saves
+        if (may_split && tiles < slots && kb >= 16) {
             ks = std::min<int64_t>(slots / tiles, std::max<int64_t>(1, kb / 4));
             ks = ceil_div64(kb, ceil_div64(kb, ks));
         }

@@ -33,6 +33,7 @@ struct SplitWeights {
 };
 size_t split_weights_bytes(int64_t n, int64_t k);
 SplitWeights split_weights_at(void* buf, int64_t n, int64_t k);  // buf: 1 KB aligned
+SplitWeights split_weights_window(const SplitWeights& w, int64_t n0, int64_t n);  // columns [n0, n0 + n), n0 a multiple of 128
 int split_weights_pack(cudaStream_t st, const WeightSources& src, const SplitWeights& w);
 
 struct SplitRows {
@@ -49,5 +50,17 @@ int split_rows_pack(cudaStream_t st, const float* x, int64_t ldx, const SplitRow
 // without it, or without room for the slabs, K is not split.
 int umma_split(cudaStream_t st, const SplitRows& x, const SplitWeights& w, float* out, int64_t ldc, float* slabs, size_t slab_bytes, int* status, int flags, int* parts);
 int umma_split_parts(int64_t m, int64_t n, int64_t k);  // K splits that the plan would take
+
+// ---- producers that write their result as pairs (fused.cu, attention.cu) ----
+// RMSNorm of x, or of x + b (b: b_parts split-K slabs [b_parts][rows][cols]; the sum goes to `sum`)
+bool rmsnorm_pairs_supported(int64_t rows, int64_t cols, const float* x, const float* b, int b_parts, const float* weight);
+int rmsnorm_pairs(cudaStream_t st, int64_t rows, int64_t cols, const float* x, const float* b, int b_parts, float exponent, float eps, const float* weight, float* sum,
+                  const SplitRows& out);
+bool swiglu_pairs_supported(int64_t rows, int64_t cols);
+int swiglu_pairs(cudaStream_t st, int64_t rows, int64_t cols, const float* gate, int64_t ldg, const float* up, int64_t ldu, const SplitRows& out);
+// Decode attention (rmlk_b200_gqa_decode_attention) whose result is row b, columns [h rows D, (h + 1) rows D) of `out` for KV head h of batch
+// entry b: one scale per KV head (out.chunk_blocks * 64 == rows * D)
+int gqa_decode_attention_pairs(cudaStream_t st, int64_t problems, int64_t rows, int64_t head_dim, int64_t keys, int64_t kv_heads, const float* q, const float* k,
+                               int64_t kb, const float* v, int64_t vb, float scale, const float* mask, int64_t ms_b, int64_t ms_h, const SplitRows& out);
 
 }  // namespace rmlk

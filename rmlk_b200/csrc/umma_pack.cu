@@ -11,37 +11,10 @@
 // Rows go into two plain row-major f16 matrices (high over low) that TMA swizzles on its way in.
 #include <algorithm>
 
-#include "umma_gemm.h"
+#include "split_pair.cuh"
 
 namespace rmlk {
 namespace umma {
-
-constexpr float LO = 2048.f;
-
-__device__ __forceinline__ uint32_t finite_abs_bits(float x) {
-    const uint32_t b = __float_as_uint(x) & 0x7fffffffu;
-    return b < 0x7f800000u ? b : 0u;  // infinities and NaNs stay what they are in the high part and do not set the scale
-}
-// 2^e with max * 2^e in [2^14, 2^15), from the bits of the largest magnitude; e in [-113, 126]
-__device__ __forceinline__ int scale_exponent(uint32_t max_bits) {
-    if (max_bits == 0) return 0;
-    const int e = 14 - (static_cast<int>(max_bits >> 23) - 127);
-    return e > 126 ? 126 : e;
-}
-__device__ __forceinline__ float exp2_int(int e) { return __int_as_float((e + 127) << 23); }
-
-__device__ __forceinline__ void split8(const float (&x)[8], float scale, uint4& hi, uint4& lo) {
-    __half2 h[4], l[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const float a = x[2 * i] * scale, b = x[2 * i + 1] * scale;
-        h[i] = __floats2half2_rn(a, b);
-        const float2 f = __half22float2(h[i]);
-        l[i] = __floats2half2_rn((a - f.x) * LO, (b - f.y) * LO);
-    }
-    hi = *reinterpret_cast<uint4*>(h);
-    lo = *reinterpret_cast<uint4*>(l);
-}
 
 // Eight consecutive columns of row k of the matrices laid side by side
 __device__ __forceinline__ void load8(const WeightSources& s, int64_t k, int64_t n0, float (&x)[8]) {
@@ -186,6 +159,15 @@ SplitWeights split_weights_at(void* buf, int64_t n, int64_t k) {
     w.tiles = buf;
     w.scale = reinterpret_cast<float*>(static_cast<char*>(buf) + static_cast<size_t>(w.n_blocks) * w.k_blocks * 32768);
     return w;
+}
+
+SplitWeights split_weights_window(const SplitWeights& w, int64_t n0, int64_t n) {
+    SplitWeights r = w;
+    r.n = n;
+    r.n_blocks = ceil_div64(n, 128);
+    r.tiles = static_cast<char*>(w.tiles) + (n0 / 128) * w.k_blocks * 32768;
+    r.scale = w.scale + n0;
+    return r;
 }
 
 int split_weights_pack(cudaStream_t st, const WeightSources& src, const SplitWeights& w) {
