@@ -192,6 +192,23 @@ __global__ void __launch_bounds__(THREADS) rmsnorm_f32_regs_kernel(int cols, flo
     }
 }
 
+// 0.f + slab 0 + slab 1 + ... of four consecutive elements: up to eight slabs are asked for at a time, added in slab order
+__device__ __forceinline__ float4 sum_slabs4(const float* p, int parts, int64_t stride) {
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int k0 = 0; k0 < parts; k0 += 8) {
+        float4 v[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+            if (k0 + j < parts) v[j] = *reinterpret_cast<const float4*>(p + (k0 + j) * stride);
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+            if (k0 + j < parts) {
+                s.x += v[j].x; s.y += v[j].y; s.z += v[j].z; s.w += v[j].w;
+            }
+    }
+    return s;
+}
+
 struct RopeParams {
     int64_t d[4];         // output dims, row-major; d[3] = head dim D
     int64_t xs[4], cs[4], ss[4];  // element strides of x, cos, sin per output dim (0 = broadcast)
@@ -246,12 +263,7 @@ __device__ __forceinline__ float batch_load(const BatchJob& j, int64_t off) {
 // four consecutive elements at element offset `off` (16-byte aligned), slabs added in order from 0.f per component
 __device__ __forceinline__ float4 batch_load4(const BatchJob& j, int64_t off) {
     if (j.parts <= 1) return *reinterpret_cast<const float4*>(j.in + off);
-    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int k = 0; k < j.parts; k++) {
-        const float4 v = *reinterpret_cast<const float4*>(j.in + k * j.part_stride + off);
-        s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
-    }
-    return s;
+    return sum_slabs4(j.in + off, j.parts, j.part_stride);
 }
 
 __global__ void __launch_bounds__(256) rope_copy_batch_kernel(const __grid_constant__ BatchParams bp) {
@@ -409,6 +421,23 @@ __global__ void __launch_bounds__(256) swiglu_f32_pitched_kernel(int64_t rows, i
     *reinterpret_cast<float4*>(out + r * cols + c) = o;
 }
 
+// gate and up as K slabs of the product that makes both (row pitches ldg, ldu, slabs part_stride apart), out dense
+__global__ void __launch_bounds__(128) swiglu_slabs_kernel(int64_t rows, int64_t cols, const float* __restrict__ g, int64_t ldg, const float* __restrict__ u, int64_t ldu,
+                                                           int parts, int64_t part_stride, float* __restrict__ out) {
+    dep_sync();
+    const int64_t i = static_cast<int64_t>(blockIdx.x) * 128 + threadIdx.x;
+    const int64_t packs = cols / 4;
+    if (i >= rows * packs) return;
+    const int64_t r = i / packs, c = (i - r * packs) * 4;
+    const float4 a = sum_slabs4(g + r * ldg + c, parts, part_stride), b = sum_slabs4(u + r * ldu + c, parts, part_stride);
+    float4 o;
+    o.x = __fmul_rn(__fmul_rn(a.x, 1.0f / (1.0f + expf(-a.x))), b.x);
+    o.y = __fmul_rn(__fmul_rn(a.y, 1.0f / (1.0f + expf(-a.y))), b.y);
+    o.z = __fmul_rn(__fmul_rn(a.z, 1.0f / (1.0f + expf(-a.z))), b.z);
+    o.w = __fmul_rn(__fmul_rn(a.w, 1.0f / (1.0f + expf(-a.w))), b.w);
+    *reinterpret_cast<float4*>(out + r * cols + c) = o;
+}
+
 template <int NP, int THREADS>
 __global__ void __launch_bounds__(THREADS) swiglu_pairs_kernel(int cols, const float* __restrict__ g, int64_t ldg, const float* __restrict__ u, int64_t ldu, SplitRows pairs) {
     dep_sync();
@@ -547,6 +576,14 @@ int rmsnorm_pairs(cudaStream_t st, int64_t rows, int64_t cols, const float* x, c
     const RowAdd ra = {b, sum, b_parts, rows * cols};
     launch_rmsnorm_regs<true>(st, rows, static_cast<int>(cols), exponent, eps, x, weight, nullptr, out, ra);
     RMLK_CHECK_LAUNCH("rmsnorm_f32_kernel");
+    return RMLK_OK;
+}
+
+int swiglu_slabs(cudaStream_t st, int64_t rows, int64_t cols, const float* gate, int64_t ldg, const float* up, int64_t ldu, int parts, int64_t part_stride, float* out) {
+    const int64_t blocks = ceil_div64(rows * (cols / 4), 128);
+    if (blocks > 0x7fffffffll) return fail(RMLK_ERR_INVALID_ARG, "swiglu: tensor too large");
+    launch_dep(swiglu_slabs_kernel, dim3(static_cast<unsigned>(blocks)), dim3(128), 0, st, rows, cols, gate, ldg, up, ldu, parts, part_stride, out);
+    RMLK_CHECK_LAUNCH("swiglu_slabs_kernel");
     return RMLK_OK;
 }
 

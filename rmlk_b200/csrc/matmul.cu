@@ -39,6 +39,7 @@ struct SkinnyParams {
     int64_t k_per_split;
     int ksplit;
     int vec_b;           // B rows are 16-byte aligned (N % 4 == 0 and base aligned)
+    int b_static = 0;    // nothing in flight writes B: its first loads need not wait for the kernel before this one
 };
 
 template <int MB>
@@ -152,21 +153,25 @@ __global__ void __launch_bounds__(SK_THREADS) skinny_kernel(SkinnyParams p) {
 // wide-strip small-M MatMul (M <= 16, rows of B 16-byte aligned): the decode GEMV
 // ---------------------------------------------------------------------------------------------
 // Memory-bound: B is read exactly once.  A CTA owns a strip of 128 columns (a warp-wide load is one 512-byte piece
-// of a row of B; 128-byte pieces stream a fifth slower) and a range of K; its 8 warps take rows k, k + 8, ... of the
-// range, each thread holding 8 independent 128-bit loads in flight.  A round covers 64 rows of B: the loads go
-// out first, then the 64 x MB block of A is staged in shared memory as [k][m] under them, then the FMAs.  K is split
-// over enough CTAs to keep several per SM in flight (the partial sums go through the caller's scratch and the
-// fixed-order split-K sum); a thread's 8 k-lanes are added by a three-step tree through shared memory.
+// of a row of B; 128-byte pieces stream a fifth slower) and a range of K; its 16 warps take rows k, k + 16, ... of the
+// range, each thread holding 8 independent 128-bit loads in flight (64 KB per CTA, two CTAs per SM).  A round covers 128 rows
+// of B: the loads go out first, then the 128 x MB block of A is staged in shared memory as [k][m] under them, then the FMAs.
+// Weights that nothing in flight writes (b_static) are requested for the first round before the kernel waits for its
+// predecessor: the stream starts while that one drains.  K is split until the grid has about two CTAs per SM (the partial sums go
+// through the caller's scratch and a fixed-order sum); the 16 k-lanes are added by a tree through shared memory.
+// 8 warps and six CTAs per SM streamed as fast, but cut K into two to three times as many slabs for the reader to add.
 constexpr int GW_COLS = 128;
 constexpr int GW_U = 8;                 // loads in flight per thread
-constexpr int GW_KR = 8 * GW_U;         // rows of B per round
-constexpr int GW_THREADS = 256;
+constexpr int GW_WARPS = 16;
+constexpr int GW_KR = GW_WARPS * GW_U;  // rows of B per round
+constexpr int GW_THREADS = 32 * GW_WARPS;
 
 template <int MB>
-__global__ void __launch_bounds__(GW_THREADS) gemv_wide_kernel(SkinnyParams p) {
-    dep_sync();
+__global__ void __launch_bounds__(GW_THREADS, MB <= 4 ? 2 : 1) gemv_wide_kernel(SkinnyParams p) {
+    dep_trigger();
     __shared__ __align__(16) float sA[GW_KR * MB];
-    __shared__ __align__(16) float sRed[4 * MB * GW_COLS];
+    constexpr int SLOTS = MB <= 8 ? GW_WARPS / 2 : GW_WARPS / 4;  // warps whose sums are in shared memory at a time
+    __shared__ __align__(16) float sRed[SLOTS * MB * GW_COLS];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t batch = blockIdx.z;
     const int split = blockIdx.y;
@@ -183,16 +188,24 @@ __global__ void __launch_bounds__(GW_THREADS) gemv_wide_kernel(SkinnyParams p) {
 #pragma unroll
         for (int j = 0; j < 4; j++) acc[m][j] = 0.f;
 
-    for (int64_t kc = kbeg; kc < kend; kc += GW_KR) {
-        const int kn = static_cast<int>(kend - kc < GW_KR ? kend - kc : GW_KR);
-        uint4 bv[GW_U];
+    uint4 bv[GW_U];
+    auto load_b = [&](int64_t kc) {
 #pragma unroll
         for (int u = 0; u < GW_U; u++) {
-            const int k = warp + u * 8;
+            const int64_t k = kc + warp + u * GW_WARPS;
             bv[u] = make_uint4(0u, 0u, 0u, 0u);
-            if (k < kn && in_cols) bv[u] = ld_stream_u4(B + (kc + k) * p.N + n0);
+            if (k < kend && in_cols) bv[u] = ld_stream_u4(B + k * p.N + n0);
         }
-        __syncthreads();  // the previous round's FMAs have read sA
+    };
+    if (!p.b_static) dep_wait();
+    load_b(kbeg);
+    if (p.b_static) dep_wait();
+    for (int64_t kc = kbeg; kc < kend; kc += GW_KR) {
+        const int kn = static_cast<int>(kend - kc < GW_KR ? kend - kc : GW_KR);
+        if (kc > kbeg) {
+            load_b(kc);
+            __syncthreads();  // the previous round's FMAs have read sA
+        }
         for (int i = threadIdx.x; i < GW_KR * MB; i += GW_THREADS) {
             const int m = i / GW_KR, k = i - m * GW_KR;  // consecutive threads -> consecutive k (coalesced)
             float v = 0.f;
@@ -202,7 +215,7 @@ __global__ void __launch_bounds__(GW_THREADS) gemv_wide_kernel(SkinnyParams p) {
         __syncthreads();
 #pragma unroll
         for (int u = 0; u < GW_U; u++) {
-            const float* arow = sA + (warp + u * 8) * MB;  // the same address across a warp: a broadcast
+            const float* arow = sA + (warp + u * GW_WARPS) * MB;  // the same address across a warp: a broadcast
             float av[MB];
             if constexpr (MB % 4 == 0) {
 #pragma unroll
@@ -224,21 +237,25 @@ __global__ void __launch_bounds__(GW_THREADS) gemv_wide_kernel(SkinnyParams p) {
             }
         }
     }
-    // add the 8 warps (k lanes): 4..7 into 0..3, 2..3 into 0..1, 1 into 0
+    // add the warps (k lanes): the upper half into the lower one until one is left
 #pragma unroll
-    for (int half = 4; half >= 1; half >>= 1) {
-        __syncthreads();
-        if (warp >= half && warp < 2 * half) {
+    for (int half = GW_WARPS / 2; half >= 1; half >>= 1) {
 #pragma unroll
-            for (int m = 0; m < MB; m++)
-                *reinterpret_cast<float4*>(sRed + ((warp - half) * MB + m) * GW_COLS + lane * 4) = make_float4(acc[m][0], acc[m][1], acc[m][2], acc[m][3]);
-        }
-        __syncthreads();
-        if (warp < half) {
+        for (int base = 0; base < half; base += SLOTS) {
+            const int n = half < SLOTS ? half : SLOTS, from = warp - half - base, to = warp - base;
+            __syncthreads();
+            if (from >= 0 && from < n) {
 #pragma unroll
-            for (int m = 0; m < MB; m++) {
-                const float4 t = *reinterpret_cast<const float4*>(sRed + (warp * MB + m) * GW_COLS + lane * 4);
-                acc[m][0] += t.x; acc[m][1] += t.y; acc[m][2] += t.z; acc[m][3] += t.w;
+                for (int m = 0; m < MB; m++)
+                    *reinterpret_cast<float4*>(sRed + (from * MB + m) * GW_COLS + lane * 4) = make_float4(acc[m][0], acc[m][1], acc[m][2], acc[m][3]);
+            }
+            __syncthreads();
+            if (to >= 0 && to < n) {
+#pragma unroll
+                for (int m = 0; m < MB; m++) {
+                    const float4 t = *reinterpret_cast<const float4*>(sRed + (to * MB + m) * GW_COLS + lane * 4);
+                    acc[m][0] += t.x; acc[m][1] += t.y; acc[m][2] += t.z; acc[m][3] += t.w;
+                }
             }
         }
     }
@@ -250,14 +267,11 @@ __global__ void __launch_bounds__(GW_THREADS) gemv_wide_kernel(SkinnyParams p) {
     }
 }
 
-// K split of the wide-strip kernel: about six CTAs per SM, ranges that are multiples of a round, and partial sums that
-// stay below a tenth of the bytes of B.
+// K split of the wide-strip kernel: about two CTAs per SM, ranges that are multiples of a round.
 static int gemv_wide_plan(int64_t batch, int64_t m, int64_t n, int64_t k, int64_t* k_per_split) {
     const int64_t strips = ceil_div64(n, GW_COLS) * batch;
-    int64_t s = ceil_div64(6ll * sm_count(), strips);
-    const int64_t by_traffic = k / (20 * m) > 0 ? k / (20 * m) : 1;
-    if (s > by_traffic) s = by_traffic;
     const int64_t rounds = ceil_div64(k, GW_KR);
+    int64_t s = (m <= 4 ? 2ll : 1ll) * sm_count() / strips;
     if (s > rounds) s = rounds;
     if (s < 1) s = 1;
     if (s > 64) s = 64;
@@ -825,6 +839,40 @@ extern "C" int rmlk_b200_matmul_window(rmlk_stream_t stream, int dtype, int64_t 
                      status, &ksplit, flags, ld);
 }
 
+// The wide-strip kernel takes up to 16 rows against rows of B on 16-byte boundaries.
+static bool gemv_wide_takes(int64_t batch, int64_t m, int64_t n, int64_t k, const void* a, const void* b, int64_t b_batch_stride, const void* c, int64_t c_batch_stride) {
+    return gemv_wide_enabled() && batch > 0 && m >= 1 && m <= 16 && k >= 1 && a && b && c && n >= GW_COLS && n % 4 == 0 && aligned_to(b, 16) && b_batch_stride % 4 == 0 &&
+           aligned_to(c, 16) && c_batch_stride % 4 == 0;
+}
+// Returns the number of K slabs left in `workspace` (1: c holds the result).
+static int gemv_wide(cudaStream_t st, int64_t batch, int64_t m, int64_t n, int64_t k, const void* a, int64_t sa, const void* b, int64_t sb, void* c, int64_t sc,
+                     void* workspace, size_t workspace_bytes, int flags) {
+    SkinnyParams p;
+    p.a = static_cast<const float*>(a);
+    p.b = static_cast<const float*>(b);
+    p.M = m; p.N = n; p.K = k;
+    p.sa = sa; p.sb = sb; p.sc = sc;
+    p.vec_b = 1;
+    p.b_static = (flags & RMLK_MATMUL_B_STATIC) ? 1 : 0;
+    int64_t kps = k;
+    int ksplit = gemv_wide_plan(batch, m, n, k, &kps);
+    const size_t need = static_cast<size_t>(ksplit) * batch * m * n * sizeof(float);
+    if (ksplit > 1 && (!workspace || workspace_bytes < need || !aligned_to(workspace, 16))) {
+        ksplit = 1;
+        kps = k;
+    }
+    p.ksplit = ksplit;
+    p.k_per_split = kps;
+    p.c = ksplit > 1 ? static_cast<float*>(workspace) : static_cast<float*>(c);
+    const dim3 grid(static_cast<unsigned>(ceil_div64(n, GW_COLS)), ksplit, static_cast<unsigned>(batch));
+    if (m == 1) launch_dep(gemv_wide_kernel<1>, grid, dim3(GW_THREADS), 0, st, p);
+    else if (m == 2) launch_dep(gemv_wide_kernel<2>, grid, dim3(GW_THREADS), 0, st, p);
+    else if (m <= 4) launch_dep(gemv_wide_kernel<4>, grid, dim3(GW_THREADS), 0, st, p);
+    else if (m <= 8) launch_dep(gemv_wide_kernel<8>, grid, dim3(GW_THREADS), 0, st, p);
+    else launch_dep(gemv_wide_kernel<16>, grid, dim3(GW_THREADS), 0, st, p);
+    return ksplit;
+}
+
 // C[m,n] = A x B for a caller that adds the split-K partial sums itself (in its next kernel): when the plan for this
 // shape splits K through the workspace, the slabs are left there ([*parts][m*n] floats, to be added in slab order
 // starting from 0.f) and C is not written; otherwise C is complete and *parts = 1.
@@ -838,6 +886,11 @@ extern "C" int rmlk_b200_matmul_parts(rmlk_stream_t stream, int dtype, int64_t m
                                workspace, workspace_bytes, status, &ksplit, flags, 0))
             return rc;
         *parts = ksplit;
+        return RMLK_OK;
+    }
+    if (dtype == RMLK_F32 && gemv_wide_takes(1, m, n, k, a, b, 0, c, 0)) {
+        *parts = gemv_wide(as_stream(stream), 1, m, n, k, a, 0, b, 0, c, 0, workspace, workspace_bytes, flags);
+        RMLK_CHECK_LAUNCH("gemv_wide_kernel");
         return RMLK_OK;
     }
     return rmlk_b200_matmul_flags(stream, dtype, 1, m, n, k, a, 0, b, 0, c, 0, workspace, workspace_bytes, status, flags);
@@ -950,23 +1003,8 @@ extern "C" int rmlk_b200_matmul_flags(rmlk_stream_t stream, int dtype, int64_t b
             RMLK_CHECK_LAUNCH("nn_narrow_kernel");
             return RMLK_OK;
         }
-        if (b_rows_aligned && aligned_to(c, 16) && c_batch_stride % 4 == 0 && n >= GW_COLS && gemv_wide_enabled()) {
-            int64_t kps = k;
-            int ksplit = gemv_wide_plan(batch, m, n, k, &kps);
-            const size_t need = static_cast<size_t>(ksplit) * batch * m * n * sizeof(float);
-            if (ksplit > 1 && (!workspace || workspace_bytes < need || !aligned_to(workspace, 16))) {
-                ksplit = 1;
-                kps = k;
-            }
-            p.ksplit = ksplit;
-            p.k_per_split = kps;
-            p.c = ksplit > 1 ? static_cast<float*>(workspace) : static_cast<float*>(c);
-            dim3 grid(static_cast<unsigned>(ceil_div64(n, GW_COLS)), ksplit, static_cast<unsigned>(batch));
-            if (m == 1) launch_dep(gemv_wide_kernel<1>, grid, dim3(GW_THREADS), 0, st, p);
-            else if (m == 2) launch_dep(gemv_wide_kernel<2>, grid, dim3(GW_THREADS), 0, st, p);
-            else if (m <= 4) launch_dep(gemv_wide_kernel<4>, grid, dim3(GW_THREADS), 0, st, p);
-            else if (m <= 8) launch_dep(gemv_wide_kernel<8>, grid, dim3(GW_THREADS), 0, st, p);
-            else launch_dep(gemv_wide_kernel<16>, grid, dim3(GW_THREADS), 0, st, p);
+        if (gemv_wide_takes(batch, m, n, k, a, b, b_batch_stride, c, c_batch_stride)) {
+            const int ksplit = gemv_wide(st, batch, m, n, k, a, a_batch_stride, b, b_batch_stride, c, c_batch_stride, workspace, workspace_bytes, flags);
             RMLK_CHECK_LAUNCH("gemv_wide_kernel");
             if (ksplit > 1) {
                 const int64_t total = batch * m * n;

@@ -92,9 +92,34 @@ struct Ctx {
         if (t.parts > 1) I.settle_parts(n.inputs[i]);
         return &t;
     }
+    // Input i for an op that only looks at its host mirror or its shape.
+    Tensor* peek(size_t i) const {
+        Tensor* t = raw(i);
+        return t && (t->host_only || t->mirror_valid) ? t : in(i);
+    }
+    Tensor& peek_req(size_t i) const {
+        Tensor* t = peek(i);
+        if (!t) raise(RMLK_ERR_INVALID_ARG, "missing input " + std::to_string(i));
+        return *t;
+    }
+    // Output i whose values the host knows and no kernel may ever ask for.  False: it leaves the graph, so it needs device memory.
+    bool host_result(size_t i, int dtype, const Shape& shape, const std::vector<int64_t>& v) const {
+        const int vid = n.outputs[i];
+        if (static_cast<int64_t>(v.size()) > HOST_MIRROR_MAX || I.g.values[vid].is_output || I.binding_of_out[vid] >= 0) return false;
+        Tensor& o = I.values[vid];
+        o = Tensor();
+        o.dtype = dtype;
+        o.shape = shape;
+        o.mi = v;
+        o.mirror_valid = true;
+        o.host_only = true;
+        o.present = true;
+        return true;
+    }
     // Input i as a dense tensor; a deferred view is copied out first.
     Tensor* in(size_t i) const {
         Tensor* t = raw(i);
+        if (t && t->host_only) I.settle_host_only(*t);
         if (t && t->pairs) raise(RMLK_ERR_INTERNAL, "value `" + I.g.values[n.inputs[i]].name + "` is only kept for packed MatMuls");
         if (t && t->lazy) I.materialize(*t);
         return t;
@@ -132,6 +157,7 @@ struct Ctx {
         o.lazy = false;
         o.parts = 0;
         o.pairs = false;
+        o.host_only = false;
         I.alloc_output(n.outputs[i], o);
         o.present = true;
         return o;
@@ -149,7 +175,9 @@ struct Ctx {
         o.parts = 0;
         o.pairs = src.pairs;
         o.split = src.split;
+        o.host_only = src.host_only && !bound;
         if (bound) {  // a carried output must own its storage
+            if (src.host_only) raise(RMLK_ERR_INTERNAL, "view of a host-only tensor as a carried output");
             I.alloc_output(vid, o);
             if (o.nbytes()) check_cuda(cudaMemcpyAsync(o.data, src.data, o.nbytes(), cudaMemcpyDeviceToDevice, I.stream), "view copy");
             I.launches++;
@@ -176,6 +204,7 @@ struct Ctx {
         o.parts = 0;
         o.pairs = base.pairs;
         o.split = base.split;
+        o.host_only = false;
         o.data = base.data;
         o.storage = base.storage;
         if (o.storage) o.storage->refs++;
@@ -377,14 +406,33 @@ bool analyze_lazy_b(const Tensor& b, int64_t k, int64_t n, LazyB& r) {
 // ---------------------------------------------------------------------------------------------
 // backend/binary.rs:18-162 with backend/{add,sub,mul,div,equal,greater}.rs
 void op_binary(const Ctx& c, int bop) {
-    Tensor& a = c.req(0);
-    Tensor& b = c.req(1);
+    Tensor& a = c.peek_req(0);
+    Tensor& b = c.peek_req(1);
     if (!in_set(a.dtype, {RMLK_F16, RMLK_F32, RMLK_F64, RMLK_I32, RMLK_I64})) unsupported_dtype(a.dtype, "binary op");
     if (a.dtype != b.dtype) raise(RMLK_ERR_INVALID_ARG, "binary op: operand data types differ (" + dtype_name(a.dtype) + " vs " + dtype_name(b.dtype) + ")");
     Shape oshape;
     if (!broadcast_shape(a.shape, b.shape, oshape))
         raise(RMLK_ERR_INVALID_ARG, "incompatible tensor shapes: " + shape_str(a.shape) + " " + shape_str(b.shape));
     const bool cmp = bop == RMLK_BIN_EQUAL || bop == RMLK_BIN_GREATER;
+    // Index arithmetic on shapes: the host has the operands, so it has the result; no kernel unless one is asked for it later.
+    auto int_value = [&](int64_t x, int64_t y) -> int64_t {
+        auto wrap = [&](int64_t v) { return a.dtype == RMLK_I32 ? static_cast<int64_t>(static_cast<int32_t>(v)) : v; };
+        switch (bop) {
+            case RMLK_BIN_ADD: return wrap(static_cast<int64_t>(static_cast<uint64_t>(x) + static_cast<uint64_t>(y)));
+            case RMLK_BIN_SUB: return wrap(static_cast<int64_t>(static_cast<uint64_t>(x) - static_cast<uint64_t>(y)));
+            case RMLK_BIN_MUL: return wrap(static_cast<int64_t>(static_cast<uint64_t>(x) * static_cast<uint64_t>(y)));
+            case RMLK_BIN_DIV: return (y == 0 || (x == std::numeric_limits<int64_t>::min() && y == -1)) ? 0 : wrap(x / y);
+            case RMLK_BIN_EQUAL: return x == y;
+            default: return x > y;
+        }
+    };
+    if (!is_float_dtype(a.dtype) && !cmp && small_mirrored(a) && small_mirrored(b) && prod(oshape) <= HOST_MIRROR_MAX) {
+        std::vector<int64_t> r(prod(oshape));
+        for (size_t i = 0; i < r.size(); i++) r[i] = int_value(a.mi[bindex(a.shape, oshape, i)], b.mi[bindex(b.shape, oshape, i)]);
+        if (c.host_result(0, a.dtype, oshape, r)) return;
+    }
+    c.req(0);
+    c.req(1);
     Tensor& o = c.make(0, cmp ? RMLK_BOOL : a.dtype, oshape);
     const Shape ks = (a.is_scalar() && b.is_scalar()) ? Shape{1} : oshape;
     const Shape as = broadcast_strides(kshape(a), ks), bs = broadcast_strides(kshape(b), ks);
@@ -408,16 +456,7 @@ void op_binary(const Ctx& c, int bop) {
                     default: ri[i] = x > y; break;
                 }
             } else {
-                const int64_t x = a.mi[ia], y = b.mi[ib];
-                auto wrap = [&](int64_t v) { return a.dtype == RMLK_I32 ? static_cast<int64_t>(static_cast<int32_t>(v)) : v; };
-                switch (bop) {
-                    case RMLK_BIN_ADD: ri[i] = wrap(static_cast<int64_t>(static_cast<uint64_t>(x) + static_cast<uint64_t>(y))); break;
-                    case RMLK_BIN_SUB: ri[i] = wrap(static_cast<int64_t>(static_cast<uint64_t>(x) - static_cast<uint64_t>(y))); break;
-                    case RMLK_BIN_MUL: ri[i] = wrap(static_cast<int64_t>(static_cast<uint64_t>(x) * static_cast<uint64_t>(y))); break;
-                    case RMLK_BIN_DIV: ri[i] = (y == 0 || (x == std::numeric_limits<int64_t>::min() && y == -1)) ? 0 : wrap(x / y); break;
-                    case RMLK_BIN_EQUAL: ri[i] = x == y; break;
-                    default: ri[i] = x > y; break;
-                }
+                ri[i] = int_value(a.mi[ia], b.mi[ib]);
             }
         }
         if (isf && !cmp) set_mirror_f(o, rf); else set_mirror_i(o, ri);
@@ -566,7 +605,7 @@ void op_reduce_mean(const Ctx& c) {
     const bool keepdims = c.attr_int("keepdims", 1) > 0;
     bool have_axes = false;
     std::vector<int64_t> axes;
-    if (Tensor* at = c.in(1)) {
+    if (Tensor* at = c.peek(1)) {
         if (at->numel() > 0) {
             for (int64_t v : c.I.host_i64(*at)) axes.push_back(normalize_index(v, rank));
             have_axes = true;
@@ -685,7 +724,7 @@ void op_gemm(const Ctx& c) {
         const size_t need = rmlk_b200_matmul_workspace_bytes(a.dtype, 1, m, n, k);
         void* ws = need ? c.I.matmul_ws.ensure(need) : nullptr;
         const int flags = (!tb && c.I.g.values[c.n.inputs[1]].is_const) ? RMLK_MATMUL_B_STATIC : 0;
-        check_rc(rmlk_b200_matmul_flags(c.stream(), a.dtype, 1, m, n, k, ap, 0, bp, 0, y.data, 0, ws, need, static_cast<int*>(c.I.status_word.ptr), flags));
+        check_rc(rmlk_b200_matmul_flags(c.stream(), a.dtype, 1, m, n, k, ap, 0, bp, 0, y.data, 0, ws, need, c.I.status_ptr(), flags));
         c.I.status_dirty = true;
         c.launched();
     }
@@ -812,7 +851,7 @@ void op_matmul(const Ctx& c) {
                 const size_t need = rmlk_b200_matmul_workspace_bytes(a.dtype, lb.outer, em, n, ka);
                 void* ws = need ? c.I.matmul_ws.ensure(need) : nullptr;
                 check_rc(rmlk_b200_matmul_ex(c.stream(), a.dtype, lb.outer, em, n, ka, a.data, em * ka, b.data, lb.sb, o.data, em * n, ws, need,
-                                             static_cast<int*>(c.I.status_word.ptr)));
+                                             c.I.status_ptr()));
                 c.I.status_dirty = true;
                 c.launched(need ? 2 : 1);
             }
@@ -845,7 +884,7 @@ void op_matmul(const Ctx& c) {
         // The only reader is a residual Add + RMSNorm chain whose kernel adds split-K slabs itself: leave them unreduced.
         void* slabs = c.I.parts_ws.ensure(need);
         int parts = 1;
-        check_rc(rmlk_b200_matmul_parts(c.stream(), a.dtype, em, n, ka, a.data, b.data, o.data, slabs, need, static_cast<int*>(c.I.status_word.ptr),
+        check_rc(rmlk_b200_matmul_parts(c.stream(), a.dtype, em, n, ka, a.data, b.data, o.data, slabs, need, c.I.status_ptr(),
                                         flags, &parts));
         c.I.status_dirty = true;
         c.launched();
@@ -867,7 +906,7 @@ void op_matmul(const Ctx& c) {
             for (size_t i = 0; i < blocks.size(); i++) {
                 const int64_t nc = blocks[i] * 128;
                 check_rc(rmlk_b200_matmul_window(c.stream(), a.dtype, em, nc, ka, a.data, static_cast<const float*>(b.data) + n0,
-                                                 static_cast<float*>(o.data) + n0, n, static_cast<int*>(c.I.status_word.ptr), flags));
+                                                 static_cast<float*>(o.data) + n0, n, c.I.status_ptr(), flags));
                 send_columns(c, hout, i, o, em, n, n0, nc);
                 n0 += nc;
             }
@@ -880,7 +919,7 @@ void op_matmul(const Ctx& c) {
     }
     void* ws = need ? c.I.matmul_ws.ensure(need) : nullptr;
     check_rc(rmlk_b200_matmul_flags(c.stream(), a.dtype, eb, em, n, ka, a.data, sa, b.data, sb, o.data, sc, ws, need,
-                                    static_cast<int*>(c.I.status_word.ptr), flags));
+                                    c.I.status_ptr(), flags));
     c.I.status_dirty = true;
     c.launched(need ? 2 : 1);
 }
@@ -890,8 +929,8 @@ void op_matmul(const Ctx& c) {
 // ---------------------------------------------------------------------------------------------
 // backend/gather.rs:28-258
 void op_gather(const Ctx& c) {
-    Tensor& data = c.req(0);
-    Tensor& idx = c.req(1);
+    Tensor& data = c.peek_req(0);
+    Tensor& idx = c.peek_req(1);
     if (!in_set(data.dtype, {RMLK_F16, RMLK_F32, RMLK_F64, RMLK_I32, RMLK_U32, RMLK_I64, RMLK_U64})) unsupported_dtype(data.dtype, "gather");
     if (!in_set(idx.dtype, {RMLK_I32, RMLK_I64})) unsupported_dtype(idx.dtype, "gather indices");
     if (data.is_scalar()) raise(RMLK_ERR_INVALID_ARG, "scalar input data not allowed");
@@ -906,16 +945,13 @@ void op_gather(const Ctx& c) {
         for (int64_t v : idx.mi)
             if (v < -axis_dim || v >= axis_dim) raise(RMLK_ERR_INVALID_ARG, "axis out of bound " + std::to_string(v));
     }
-    Tensor& o = c.make(0, data.dtype, oshape);
     const int64_t outer = prod(data.shape, 0, axis), inner = prod(data.shape, axis + 1);
-    check_rc(rmlk_b200_gather(c.stream(), static_cast<int>(dtype_size_of(data.dtype)), idx.dtype, outer, axis_dim, inner, idx.numel(), data.data,
-                              idx.data, o.data, static_cast<int*>(c.I.status_word.ptr)));
-    c.launched();
-    if (small_mirrored(data) && small_mirrored(idx) && o.numel() <= HOST_MIRROR_MAX && data.dtype != RMLK_F16) {
+    std::vector<int64_t> ri;
+    std::vector<double> rf;
+    const bool on_host = small_mirrored(data) && small_mirrored(idx) && prod(oshape) <= HOST_MIRROR_MAX && data.dtype != RMLK_F16;
+    const bool isf = is_float_dtype(data.dtype);
+    if (on_host) {
         const int64_t n_idx = idx.numel();
-        const bool isf = is_float_dtype(data.dtype);
-        std::vector<int64_t> ri;
-        std::vector<double> rf;
         for (int64_t ou = 0; ou < outer; ou++)
             for (int64_t j = 0; j < n_idx; j++) {
                 int64_t ix = idx.mi[j];
@@ -925,6 +961,16 @@ void op_gather(const Ctx& c) {
                     if (isf) rf.push_back(data.mf[src]); else ri.push_back(data.mi[src]);
                 }
             }
+        if (in_set(data.dtype, {RMLK_I32, RMLK_I64}) && c.host_result(0, data.dtype, oshape, ri)) return;
+    }
+    c.req(0);
+    c.req(1);
+    Tensor& o = c.make(0, data.dtype, oshape);
+    check_rc(rmlk_b200_gather(c.stream(), static_cast<int>(dtype_size_of(data.dtype)), idx.dtype, outer, axis_dim, inner, idx.numel(), data.data,
+                              idx.data, o.data, c.I.status_ptr()));
+    c.launched();
+    c.I.status_dirty = true;
+    if (on_host) {
         if (isf) set_mirror_f(o, rf); else set_mirror_i(o, ri);
     }
 }
@@ -957,17 +1003,17 @@ void op_scatter_nd(const Ctx& c) {
     if (upd.numel() != n_tuples * slice_len) raise(RMLK_ERR_INVALID_ARG, "scatter_nd: updates shape does not match indices and data");
     Tensor& o = c.make(0, data.dtype, data.shape);
     check_rc(rmlk_b200_scatter_nd(c.stream(), red, data.dtype, static_cast<int>(data.shape.size()), data.shape.data(), n_tuples, static_cast<int>(k),
-                                  data.data, idx.data, upd.data, o.data, static_cast<int*>(c.I.status_word.ptr)));
+                                  data.data, idx.data, upd.data, o.data, c.I.status_ptr()));
     c.launched(2);
 }
 
 // backend/slice.rs:49-464
 void op_slice(const Ctx& c) {
     Tensor& x = c.req(0);
-    Tensor& starts = c.req(1);
-    Tensor& ends = c.req(2);
-    Tensor* axes = c.in(3);
-    Tensor* steps = c.in(4);
+    Tensor& starts = c.peek_req(1);
+    Tensor& ends = c.peek_req(2);
+    Tensor* axes = c.peek(3);
+    Tensor* steps = c.peek(4);
     if (starts.dtype != ends.dtype) raise(RMLK_ERR_INVALID_ARG, "StartAndEndDataTypeMismatch");
     if (!in_set(x.dtype, {RMLK_F16, RMLK_F32, RMLK_F64, RMLK_I32, RMLK_I64}) || !in_set(starts.dtype, {RMLK_I32, RMLK_I64}))
         unsupported_dtype(x.dtype, "slice");
@@ -1197,6 +1243,8 @@ bool concat_append(const Ctx& c) {
     Binding& b = c.I.bindings[bi];
     Tensor* past = c.raw(0);
     Tensor* add = c.raw(1);
+    if (past && past->host_only) c.I.settle_host_only(*past);
+    if (add && add->host_only) c.I.settle_host_only(*add);
     AppendPlan ap;
     if (!past || !add || !append_plan(b, *past, add->dtype, add->shape, ap)) return false;
     append_reserve(c.I, b, *past, ap);
@@ -1244,7 +1292,21 @@ bool concat_append(const Ctx& c) {
                 c.I.materialize(*add);
             }
         }
-        if (!add->lazy && add->data != slot) {
+        if (!add->lazy && add->data != slot && c.I.inplace_append_to && ap.elem == 4 && ap.rank <= 5 && add->numel() <= (1 << 20)) {
+            // a few dense rows (one decoded token): collected with the rotary embeddings of the layer as well
+            const Shape st = dense_strides(add->shape);
+            rmlk_batch_job j = {};
+            j.kind = RMLK_BATCH_COPY4;
+            j.rank = static_cast<int>(ap.rank);
+            for (int64_t d = 0; d < 5; d++) {
+                j.shape[d] = d < ap.rank ? add->shape[d] : 1;
+                j.in_strides[d] = d < ap.rank ? st[d] : 0;
+                j.out_strides[d] = d < ap.rank ? dst[d] : 0;
+            }
+            j.in = add->data;
+            j.out = slot;
+            c.I.defer_job(j);
+        } else if (!add->lazy && add->data != slot) {
             check_cuda(cudaMemcpy2DAsync(slot, static_cast<size_t>(b.cap) * ap.row, add->data, static_cast<size_t>(ap.tn) * ap.row,
                                          static_cast<size_t>(ap.tn) * ap.row, static_cast<size_t>(ap.outer), cudaMemcpyDeviceToDevice, c.I.stream),
                        "cache append");
@@ -1267,7 +1329,7 @@ bool concat_append(const Ctx& c) {
 // backend/concat.rs:28-198
 void op_concat(const Ctx& c) {
     if (concat_append(c)) return;
-    Tensor& first = c.req(0);
+    Tensor& first = c.peek_req(0);
     if (!in_set(first.dtype, {RMLK_F16, RMLK_F32, RMLK_F64, RMLK_I32, RMLK_U32, RMLK_I64, RMLK_U64})) unsupported_dtype(first.dtype, "concat");
     if (first.is_scalar()) raise(RMLK_ERR_INVALID_ARG, "scalars are not allowed");
     const Attr* ax = c.attr("axis");
@@ -1281,7 +1343,7 @@ void op_concat(const Ctx& c) {
     Shape oshape = first.shape;
     int64_t total = 0;
     for (size_t i = 0; i < c.n.inputs.size(); i++) {
-        Tensor* t = c.in(i);
+        Tensor* t = c.peek(i);
         if (!t) break;
         if (static_cast<int64_t>(t->shape.size()) != rank)
             raise(RMLK_ERR_INVALID_ARG, "ShapeMismatch { index: " + std::to_string(i) + ", base_rank: " + std::to_string(rank) + ", found_rank: " + std::to_string(t->shape.size()) + " }");
@@ -1290,11 +1352,20 @@ void op_concat(const Ctx& c) {
             if (d != axis && t->shape[d] != first.shape[d])
                 raise(RMLK_ERR_INVALID_ARG, "DimensionMismatch { axis: " + std::to_string(d) + ", dim: " + std::to_string(t->shape[d]) + ", expected_dim: " + std::to_string(first.shape[d]) + " }");
         total += t->shape[axis];
-        ptrs.push_back(t->data);
         dims.push_back(t->shape[axis]);
         ins.push_back(t);
     }
     oshape[axis] = total;
+    if (rank == 1 && in_set(first.dtype, {RMLK_I32, RMLK_I64}) && total <= HOST_MIRROR_MAX) {
+        bool known = true;
+        std::vector<int64_t> r;
+        for (Tensor* t : ins) {
+            known = known && small_mirrored(*t);
+            if (known) r.insert(r.end(), t->mi.begin(), t->mi.end());
+        }
+        if (known && c.host_result(0, first.dtype, oshape, r)) return;
+    }
+    for (size_t i = 0; i < ins.size(); i++) ptrs.push_back(c.in(i)->data);
     Tensor& o = c.make(0, first.dtype, oshape);
     if (o.numel() == 0) return;
     check_rc(rmlk_b200_concat(c.stream(), static_cast<int>(dtype_size_of(first.dtype)), static_cast<int>(ptrs.size()), prod(first.shape, 0, axis),
@@ -1319,7 +1390,8 @@ void op_concat(const Ctx& c) {
 void op_expand(const Ctx& c) {
     Tensor* xr = c.raw(0);
     if (!xr) raise(RMLK_ERR_INVALID_ARG, "missing input 0");
-    Tensor& sh = c.req(1);
+    if (xr->host_only) c.I.settle_host_only(*xr);
+    Tensor& sh = c.peek_req(1);
     if (!in_set(xr->dtype, {RMLK_F16, RMLK_F32, RMLK_F64, RMLK_I32, RMLK_U32, RMLK_I64, RMLK_U64})) unsupported_dtype(xr->dtype, "expand");
     if (sh.dtype != RMLK_I64) unsupported_dtype(sh.dtype, "expand shape");
     const std::vector<int64_t> target = c.I.host_i64(sh);
@@ -1381,7 +1453,7 @@ void op_trilu(const Ctx& c) {
     if (!in_set(x.dtype, {RMLK_F16, RMLK_F32, RMLK_F64, RMLK_I32, RMLK_U32, RMLK_I64, RMLK_U64})) unsupported_dtype(x.dtype, "trilu");
     const bool upper = c.attr_int("upper", 1) != 0;
     int64_t k = 0;
-    if (Tensor* kt = c.in(1)) {
+    if (Tensor* kt = c.peek(1)) {
         if (!kt->is_scalar()) raise(RMLK_ERR_INVALID_ARG, "InvalidKTensor");
         if (kt->dtype != RMLK_I64) unsupported_dtype(kt->dtype, "trilu k");
         k = c.I.host_i64(*kt)[0];
@@ -1399,9 +1471,9 @@ void op_trilu(const Ctx& c) {
 
 // backend/range.rs:28-205
 void op_range(const Ctx& c) {
-    Tensor& s = c.req(0);
-    Tensor& l = c.req(1);
-    Tensor& d = c.req(2);
+    Tensor& s = c.peek_req(0);
+    Tensor& l = c.peek_req(1);
+    Tensor& d = c.peek_req(2);
     if (!in_set(s.dtype, {RMLK_F16, RMLK_F32, RMLK_F64, RMLK_I32, RMLK_I64})) unsupported_dtype(s.dtype, "range");
     if (l.dtype != s.dtype || d.dtype != s.dtype) raise(RMLK_ERR_INVALID_ARG, "range: start, limit and delta must share a data type");
     if (s.numel() != 1 || l.numel() != 1 || d.numel() != 1) raise(RMLK_ERR_INVALID_ARG, "range: inputs must be scalars");
@@ -1461,7 +1533,7 @@ void op_range(const Ctx& c) {
 void op_reshape(const Ctx& c) {
     // a deferred view keeps its element order under Reshape, so it can stay deferred
     Tensor& x = c.may_defer(0) && c.raw(0) ? *c.raw(0) : c.req(0);
-    Tensor& sh = c.req(1);
+    Tensor& sh = c.peek_req(1);
     if (sh.dtype != RMLK_I64) unsupported_dtype(sh.dtype, "reshape shape");
     const bool allow_zero = c.attr_int("allowzero", 0) != 0;
     std::vector<int64_t> dims = sh.shape.empty() ? std::vector<int64_t>{} : c.I.host_i64(sh);
@@ -1505,7 +1577,7 @@ void op_unsqueeze(const Ctx& c) {
     // inserting size-1 dims does not change the element order: a deferred view stays deferred
     Tensor& x = c.may_defer(0) && c.raw(0) ? *c.raw(0) : c.req(0);
     std::vector<int64_t> axes;
-    if (Tensor* at = c.in(1)) {
+    if (Tensor* at = c.peek(1)) {
         if (at->shape.size() != 1) raise(RMLK_ERR_INVALID_ARG, "InvalidAxesRank");
         axes = c.I.host_i64(*at);
     } else if (const Attr* a = c.attr("axes")) {
@@ -1564,6 +1636,7 @@ void op_shape(const Ctx& c) {
     end = std::min(std::max<int64_t>(end, 0), rank);
     std::vector<int64_t> vals;
     for (int64_t i = start; i < end; i++) vals.push_back(x.shape[i]);
+    if (c.host_result(0, RMLK_I64, Shape{static_cast<int64_t>(vals.size())}, vals)) return;
     Tensor& o = c.make(0, RMLK_I64, Shape{static_cast<int64_t>(vals.size())});
     store_small_i64(c, o, vals);
     set_mirror_i(o, vals);
@@ -1571,7 +1644,7 @@ void op_shape(const Ctx& c) {
 
 // backend/constant_of_shape.rs:30-70
 void op_constant_of_shape(const Ctx& c) {
-    Tensor& sh = c.req(0);
+    Tensor& sh = c.peek_req(0);
     if (sh.dtype != RMLK_I64) unsupported_dtype(sh.dtype, "constant_of_shape shape");
     const std::vector<int64_t> dims = c.I.host_i64(sh);
     for (int64_t v : dims)
@@ -2033,6 +2106,24 @@ bool Instance::run_fused(const FusedGroup& fg) {
             int64_t pg = 0, pu = 0;
             const bool pitched = (gt->lazy || up->lazy) && !gt->shape.empty() && gt->shape.back() % 4 == 0 && as_rows(*gt, pg) && as_rows(*up, pu) &&
                                  pg % 4 == 0 && pu % 4 == 0 && reinterpret_cast<uintptr_t>(gt->data) % 16 == 0 && reinterpret_cast<uintptr_t>(up->data) % 16 == 0;
+            if (unsummed.y && gt->storage == unsummed.y && up->storage == unsummed.y && last_use[fg.v[0]] == fg.root && last_use[fg.v[1]] == fg.root &&
+                pending_jobs.empty() && !gt->shape.empty() && gt->shape.back() % 4 == 0 && as_rows(*gt, pg) && as_rows(*up, pu) && pg % 4 == 0 && pu % 4 == 0 &&
+                unsummed.part_stride % 4 == 0) {
+                // the product's K slabs have not been added up and nothing else reads them: added here, as they are read
+                const Unsummed u = unsummed;
+                const ptrdiff_t og = static_cast<const char*>(gt->data) - static_cast<const char*>(u.y->ptr), ou = static_cast<const char*>(up->data) - static_cast<const char*>(u.y->ptr);
+                if (og % 16 == 0 && ou % 16 == 0) {
+                    unsummed = Unsummed();
+                    const Shape shape = gt->shape;
+                    const int64_t cols = shape.back();
+                    Tensor& o = c.make(0, RMLK_F32, shape);
+                    check_rc(swiglu_slabs(stream, o.numel() / cols, cols, reinterpret_cast<const float*>(reinterpret_cast<const char*>(u.slabs) + og), pg,
+                                          reinterpret_cast<const float*>(reinterpret_cast<const char*>(u.slabs) + ou), pu, u.parts, u.part_stride, static_cast<float*>(o.data)));
+                    launches++;
+                    arena->release(u.y);
+                    return true;
+                }
+            }
             if (!gt->shape.empty() && as_rows(*gt, pg) && as_rows(*up, pu) && pg % 4 == 0 && pu % 4 == 0 && reinterpret_cast<uintptr_t>(gt->data) % 16 == 0 &&
                 reinterpret_cast<uintptr_t>(up->data) % 16 == 0) {
                 const int64_t cols = gt->shape.back(), rows = cols ? gt->numel() / cols : 0;
@@ -2175,7 +2266,7 @@ bool Instance::run_fused(const FusedGroup& fg) {
             auto axes_are = [&](int node, int64_t a0, int64_t a1) {
                 const Ctx cu{*this, g.nodes[node]};
                 std::vector<int64_t> axes;
-                if (Tensor* at = cu.in(1)) axes = host_i64(*at);
+                if (Tensor* at = cu.peek(1)) axes = host_i64(*at);
                 else if (const Attr* a = cu.attr("axes")) axes = a->ints;
                 return axes.size() == 2 && axes[0] == a0 && axes[1] == a1;
             };
@@ -2183,6 +2274,7 @@ bool Instance::run_fused(const FusedGroup& fg) {
             const std::vector<int64_t> dims = host_i64(*shp);
             if (dims.size() != 2 || dims[0] < 0 || dims[1] < 0 || dims[1] != am->shape[1]) return false;
             const int64_t k = kt ? host_i64(*kt)[0] : 0;
+            if (am->host_only) settle_host_only(*am);
             if (am->lazy) materialize(*am);
             const int64_t B = am->shape[0], S = dims[0], T = dims[1];
             const void* amd = am->data;
@@ -2383,7 +2475,7 @@ bool Instance::run_merged_matmul(int node_index) {
         // decode-sized product: the split-K slabs stay unsummed for the placements that read them (Instance::unsummed)
         int parts = 1;
         check_rc(rmlk_b200_matmul_parts(reinterpret_cast<rmlk_stream_t>(stream), RMLK_F32, rows, mm.n_total, mm.k, a.data, mm.w.ptr, y->ptr, ws, need,
-                                        static_cast<int*>(status_word.ptr), flags, &parts));
+                                        status_ptr(), flags, &parts));
         launches++;
         if (parts > 1) {
             unsummed.y = y;
@@ -2394,7 +2486,7 @@ bool Instance::run_merged_matmul(int node_index) {
         }
     } else {
         check_rc(rmlk_b200_matmul_flags(reinterpret_cast<rmlk_stream_t>(stream), RMLK_F32, 1, rows, mm.n_total, mm.k, a.data, 0, mm.w.ptr, 0, y->ptr,
-                                        rows * mm.n_total, ws, need, static_cast<int*>(status_word.ptr), flags));
+                                        rows * mm.n_total, ws, need, status_ptr(), flags));
         launches += need ? 2 : 1;
     }
     status_dirty = true;
@@ -2596,7 +2688,7 @@ void Instance::packed_product(PackedWeights& pw, const SplitRows& x, int64_t n0,
     }
     // from the run after the one that laid them out nothing in flight writes the weights
     const int flags = pw.packed_run < run_counter ? RMLK_MATMUL_B_STATIC : 0;
-    check_rc(umma_split(stream, x, w, out, ldc, sp, bytes, static_cast<int*>(status_word.ptr), flags, parts));
+    check_rc(umma_split(stream, x, w, out, ldc, sp, bytes, status_ptr(), flags, parts));
     status_dirty = true;
     launches++;
 }

@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "../../../include/rmlk_b200_runtime.h"
+#include "../hostio.h"
 #include "../umma_gemm.h"
 
 namespace rmlk {
@@ -85,6 +86,9 @@ struct Tensor {
     // (backend/expand.rs:49-216, backend/transpose.rs:44-178, backend/reshape.rs:27-73).
     bool lazy = false;
     std::vector<int64_t> pshape, pstride;
+    // Only the host mirror exists (shapes and index arithmetic on them): written to device memory when a kernel asks for it, which in
+    // an exported decoder never happens - eight launches of a step that no kernel waited for.
+    bool host_only = false;
     // > 1: a MatMul result still in `parts` split-K slabs ([parts][numel] floats at `data`, to be added in slab
     // order); only ever set on a value whose single reader is the residual Add in front of an RMSNorm chain, which
     // adds the slabs itself.  Any other access goes through Instance::settle_parts first.
@@ -142,6 +146,17 @@ struct DeviceBuffer {
     void* ptr = nullptr;
     size_t cap = 0;
     void* ensure(size_t bytes);
+    void release();
+};
+
+// Pinned, device-visible host memory of an instance: the status word, the arrival flags of a download, and the staging areas of small
+// inputs and outputs.  Blocks come from a process-wide list that keeps a few released ones (pinning memory takes as long as many runs).
+struct HostBlock {
+    static constexpr size_t STATUS = 0, FLAGS = 4096, UP = 8192, UP_BYTES = size_t(2) << 20, DOWN = UP + UP_BYTES, DOWN_BYTES = size_t(4) << 20,
+                            BYTES = DOWN + DOWN_BYTES;
+    static_assert(FLAGS + 4 * (DOWN_BYTES / DOWNLOAD_CHUNK) <= UP, "one flag per chunk");
+    char* base = nullptr;
+    void acquire();
     void release();
 };
 
@@ -263,7 +278,16 @@ struct Instance {
     std::vector<DeviceBuffer> input_bufs;  // per value id (only inputs use theirs)
     DeviceBuffer weights;
     std::unique_ptr<Arena> arena;
-    DeviceBuffer status_word;   // device int for gather / scatter_nd diagnostics
+    HostBlock host;
+    int* status_ptr() const { return reinterpret_cast<int*>(host.base + HostBlock::STATUS); }  // device-visible word for kernel diagnostics
+    std::vector<UploadJob> uploads;  // small inputs fed since the last run, fetched by one kernel at its start
+    size_t up_used = 0;              // bytes of the staging area that uploads not known to be finished occupy
+    cudaEvent_t up_done = nullptr;   // behind the last upload
+    uint32_t down_seq = 0;
+    void feed_host(void* dst, const void* src, size_t bytes);
+    void flush_uploads();
+    void read_to_host(void* dst, const void* src, size_t bytes);
+    void settle_host_only(Tensor& t);  // gives a host-only tensor its device data
     DeviceBuffer matmul_ws;     // split-K scratch
     DeviceBuffer attn_ws;       // partial results + arrival counters of the split-keys attention kernel (kept zeroed)
     size_t attn_ws_zeroed = 0;  // capacity that has been zero-filled
@@ -339,6 +363,8 @@ struct Instance {
 };
 
 size_t dtype_size_of(int dt);
+void* host_result_alloc(size_t bytes);
+void host_result_free(void* p, size_t bytes);
 
 std::string status_word_message(int word);  // text for a non-zero device status word
 void check_cuda_fn(cudaError_t e, const char* what);

@@ -56,6 +56,8 @@ int umma_split_parts(int64_t m, int64_t n, int64_t k);  // K splits that the pla
 bool rmsnorm_pairs_supported(int64_t rows, int64_t cols, const float* x, const float* b, int b_parts, const float* weight);
 int rmsnorm_pairs(cudaStream_t st, int64_t rows, int64_t cols, const float* x, const float* b, int b_parts, float exponent, float eps, const float* weight, float* sum,
                   const SplitRows& out);
+// SwiGLU gate read from K slabs (cols, pitches and part_stride multiples of 4, 16-byte aligned)
+int swiglu_slabs(cudaStream_t st, int64_t rows, int64_t cols, const float* gate, int64_t ldg, const float* up, int64_t ldu, int parts, int64_t part_stride, float* out);
 bool swiglu_pairs_supported(int64_t rows, int64_t cols);
 int swiglu_pairs(cudaStream_t st, int64_t rows, int64_t cols, const float* gate, int64_t ldg, const float* up, int64_t ldu, const SplitRows& out);
 // Decode attention (rmlk_b200_gqa_decode_attention) whose result is row b, columns [h rows D, (h + 1) rows D) of `out` for KV head h of batch

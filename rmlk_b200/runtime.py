@@ -17,6 +17,7 @@ from __future__ import annotations
 
 import ctypes
 import enum
+import weakref
 from typing import Dict, Optional, Sequence
 
 import numpy as np
@@ -100,8 +101,15 @@ class AttributeType:
             self.array = np.require(array, requirements="C")
 
 
+_DIMS = [ctypes.c_int64 * max(n, 1) for n in range(9)]  # array types, made once: a type expression costs as much as the call it serves
+
+
 def _i64(vals: Sequence[int]):
-    return (ctypes.c_int64 * max(len(vals), 1))(*[int(v) for v in vals])
+    n = len(vals)
+    return (_DIMS[n] if n < 9 else ctypes.c_int64 * n)(*vals)
+
+
+_NP_CODES = {np.dtype(dt.to_numpy(c)): c for c in dt.NAMES}  # dtype object -> code
 
 
 def _setup(l):
@@ -142,12 +150,34 @@ def _setup(l):
     l.rmlk_instance_value_info.argtypes = [ctypes.c_void_p, ctypes.c_char_p, ctypes.c_void_p, ctypes.c_void_p,
                                            ctypes.c_void_p, ctypes.c_void_p]
     l.rmlk_instance_read.argtypes = [ctypes.c_void_p, ctypes.c_char_p, ctypes.c_void_p, ctypes.c_size_t]
+    l.rmlk_host_alloc.restype = ctypes.c_void_p
+    l.rmlk_host_alloc.argtypes = [ctypes.c_size_t]
+    l.rmlk_host_free.restype = None
+    l.rmlk_host_free.argtypes = [ctypes.c_void_p, ctypes.c_size_t]
     l._rt_ready = True
     return l
 
 
 def _rt():
     return _setup(lib())
+
+
+_PINNED_FROM, _PINNED_TO = 32 << 10, 8 << 20
+
+
+def _result_array(l, shape, dtype) -> np.ndarray:
+    """An uninitialised array for a result.  From 32 KB on its memory is pinned, so that the device writes into it directly; it goes back
+    to the library's pool with the array.  (The pool is bounded: an ordinary array when it is used up.)"""
+    n = dtype.itemsize
+    for v in shape:
+        n *= v
+    if _PINNED_FROM <= n <= _PINNED_TO:
+        ptr = l.rmlk_host_alloc(n)
+        if ptr:
+            buf = (ctypes.c_char * n).from_address(ptr)
+            weakref.finalize(buf, l.rmlk_host_free, ptr, n).atexit = False
+            return np.frombuffer(buf, dtype=dtype).reshape(shape)
+    return np.empty(shape, dtype=dtype)
 
 
 class OpHandle:
@@ -240,6 +270,16 @@ class ModelInstance:
         if not self._h:
             raise InferenceError(1, last_error())
         self._keep = []
+        self._l = _rt()
+        self._names = {}           # name -> encoded, for the names used so far
+        self._info = (ctypes.c_int(), ctypes.c_int(), (ctypes.c_int64 * 8)(), ctypes.c_void_p())
+        self._info_refs = tuple(ctypes.byref(x) if i != 2 else x for i, x in enumerate(self._info))
+
+    def _key(self, name: str) -> bytes:
+        k = self._names.get(name)
+        if k is None:
+            k = self._names[name] = name.encode()
+        return k
 
     def __del__(self):
         h = getattr(self, "_h", None)
@@ -255,13 +295,15 @@ class ModelInstance:
     # -- feeding ---------------------------------------------------------------------------------
     def set_input(self, name: str, array: np.ndarray):
         """Host input: copied H2D on the instance's stream (load_inputs, instance.rs:33-56)."""
-        a = np.require(array, requirements="C")
+        a = array if type(array) is np.ndarray and array.flags.c_contiguous else np.require(array, requirements="C")
         self._keep.append(a)
-        _check(_rt().rmlk_instance_set_input(self._h, name.encode(), dt.from_numpy(a.dtype), a.ndim, _i64(a.shape), a.ctypes.data, 0))
+        code = _NP_CODES.get(a.dtype)
+        _check(self._l.rmlk_instance_set_input(self._h, self._key(name), dt.from_numpy(a.dtype) if code is None else code, a.ndim, _i64(a.shape),
+                                               a.__array_interface__["data"][0], 0))
 
     def set_input_ptr(self, name: str, dtype: int, dims: Sequence[int], ptr: int, on_device: bool):
         """Raw pointer input: pinned host memory (on_device=False) or a device buffer used in place."""
-        _check(_rt().rmlk_instance_set_input(self._h, name.encode(), dtype, len(dims), _i64(dims), ctypes.c_void_p(ptr), 1 if on_device else 0))
+        _check(self._l.rmlk_instance_set_input(self._h, self._key(name), dtype, len(dims), _i64(dims), ptr, 1 if on_device else 0))
 
     def bind(self, output: str, input_: str):
         """Carry `output` of one run into `input_` of the next on the device (no host round trip)."""
@@ -270,24 +312,24 @@ class ModelInstance:
     # -- running ---------------------------------------------------------------------------------
     def launch(self):
         """Enqueue one forward pass (the op loop of instance.rs:100-112); does not wait."""
-        _check(_rt().rmlk_instance_run(self._h))
+        _check(self._l.rmlk_instance_run(self._h))
         self._keep.clear()
 
     def synchronize(self):
         _check(_rt().rmlk_instance_synchronize(self._h))
 
     def value_info(self, name: str):
-        d = ctypes.c_int()
-        r = ctypes.c_int()
-        dims = (ctypes.c_int64 * 8)()
-        p = ctypes.c_void_p()
-        _check(_rt().rmlk_instance_value_info(self._h, name.encode(), ctypes.byref(d), ctypes.byref(r), dims, ctypes.byref(p)))
-        return d.value, list(dims)[: r.value], p.value or 0
+        d, r, dims, p = self._info
+        _check(self._l.rmlk_instance_value_info(self._h, self._key(name), *self._info_refs))
+        return d.value, dims[: r.value], p.value or 0
 
     def read(self, name: str) -> np.ndarray:
-        d, shape, _ = self.value_info(name)
-        out = np.empty(shape, dtype=dt.to_numpy(d))
-        _check(_rt().rmlk_instance_read(self._h, name.encode(), out.ctypes.data, out.nbytes))
+        d, r, dims, _ = self._info
+        key = self._key(name)
+        # (no device address: asking for one would give a value that only the host knows device memory)
+        _check(self._l.rmlk_instance_value_info(self._h, key, self._info_refs[0], self._info_refs[1], dims, None))
+        out = _result_array(self._l, dims[: r.value], dt.to_numpy(d.value))
+        _check(self._l.rmlk_instance_read(self._h, key, out.__array_interface__["data"][0], out.nbytes))
         return out
 
     def stream_output(self, name: str, ptr: int, nbytes: int):
