@@ -33,6 +33,18 @@ __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t* r) {
     }
 }
 
+// high x high + 2^-11 (high x low + low x high).  Where an operand is infinite or NaN its low part is NaN, and an infinity times a low
+// part of zero is one too: the high product alone then says what the fp32 product is.
+__device__ __forceinline__ float add_low(float high, float low) {
+    return fabsf(high) < INFINITY ? fmaf(low, 1.f / LO_SCALE, high) : high;
+}
+// v 2^a 2^b for the scales of a row and a column.  Their product is formed first where it is a normal number - v times one of them alone
+// may overflow although the result does not; where it is not, both have the same sign of exponent and the order does not matter.
+__device__ __forceinline__ float unscale(float v, float a, float b) {
+    const float t = a * b;
+    return t >= 1.17549435e-38f && t < INFINITY ? v * t : v * a * b;
+}
+
 struct Item {
     int n_tile, m_tile, split;
 };
@@ -237,6 +249,9 @@ __global__ void __launch_bounds__(Layout<CG, SPLIT, MT, ST>::THREADS, 1) gemm_ke
             const Item it = item_at(w, p);
             const int kb0 = it.split * p.k_per_split, nk = min(p.k_per_split, p.k_blocks - kb0);
             const int64_t n = (static_cast<int64_t>(it.n_tile) * CG + rank) * BN + sub * 32 + lane;
+            const bool in = n < p.N;
+            float ws = 0.f;
+            if constexpr (SPLIT && !ONE_CHUNK) ws = in ? __ldg(p.w_scale + n) : 0.f;
             const int64_t m_base = static_cast<int64_t>(it.m_tile) * MT + part * HM;
             float acc[HM];
             float4 s4 = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -265,7 +280,7 @@ __global__ void __launch_bounds__(Layout<CG, SPLIT, MT, ST>::THREADS, 1) gemm_ke
                             tmem_ld<STEP>(d + MT + j0, q);
                             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                            for (int j = 0; j < STEP; j++) acc[j0 + j] = fmaf(__uint_as_float(q[j]), 1.f / LO_SCALE, acc[j0 + j]);
+                            for (int j = 0; j < STEP; j++) acc[j0 + j] = add_low(acc[j0 + j], __uint_as_float(q[j]));
                         }
                     }
                 } else {
@@ -277,8 +292,8 @@ __global__ void __launch_bounds__(Layout<CG, SPLIT, MT, ST>::THREADS, 1) gemm_ke
                         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
                         for (int j = 0; j < STEP; j++) {
-                            const float v = fmaf(__uint_as_float(q[j]), 1.f / LO_SCALE, __uint_as_float(r[j])), sc = row_scale(j0 + j);
-                            acc[j0 + j] = c == c_first ? v * sc : fmaf(v, sc, acc[j0 + j]);
+                            const float v = unscale(add_low(__uint_as_float(r[j]), __uint_as_float(q[j])), row_scale(j0 + j), ws);
+                            acc[j0 + j] = c == c_first ? v : acc[j0 + j] + v;
                         }
                     }
                 }
@@ -294,16 +309,14 @@ __global__ void __launch_bounds__(Layout<CG, SPLIT, MT, ST>::THREADS, 1) gemm_ke
                 }
             }
             if (!ok) break;
-            const bool in = n < p.N;
-            const float ws = SPLIT && in ? __ldg(p.w_scale + n) : 0.f;
+            if constexpr (SPLIT && ONE_CHUNK) ws = in ? __ldg(p.w_scale + n) : 0.f;
             using Out = typename std::conditional<OUT16, __half, float>::type;
             Out* o = static_cast<Out*>(p.out) + (p.ksplit > 1 ? static_cast<int64_t>(it.split) * p.M * p.N : 0) + m_base * p.ldc + n;
             const int64_t rows = in ? p.M - m_base : 0;
 #pragma unroll
             for (int j = 0; j < HM; j++) {
                 float v = acc[j];
-                if constexpr (SPLIT) v *= ws;
-                if constexpr (SPLIT && ONE_CHUNK) v *= row_scale(j);
+                if constexpr (SPLIT && ONE_CHUNK) v = unscale(v, row_scale(j), ws);
                 if (j < rows) {
                     if constexpr (OUT16) *o = __float2half_rn(v);
                     else *o = v;

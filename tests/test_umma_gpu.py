@@ -77,3 +77,35 @@ def test_f32_split_scales(cuda):
     bound = mag * (3 * 2.0 ** -22 + 2.0 ** -23 * (k / 16 + 2)) + 2.0 ** -125
     fine = want.abs() < 2.0 ** 127
     assert bool(((got.double() - want).abs() <= bound)[fine].all())
+
+
+@pytest.mark.parametrize("n,k", [(200, 100), (256, 512)])
+def test_f32_split_non_finite_and_extreme(cuda, n, k):
+    """Infinities and NaNs come out where fp32 puts them; scales whose product is in range although one alone takes the sum out of it."""
+    import torch
+    from rmlk_b200 import kernels as K
+    m = 300
+    a, b = torch.randn(m, k, device=cuda), torch.randn(k, n, device=cuda)
+    a[:, 3] = a[:, 3].abs() + 1.0
+    b[3] = 1.0                    # exact in f16: its low part is zero
+    a[4, 3] = float("inf")
+    a[5, 3] = float("-inf")
+    a[6, 9] = float("nan")
+    a[7, 3], a[7, 8] = float("inf"), float("-inf")
+    b[8] = 2.0
+    b[11, 17] = float("-inf")
+    a[:, 11] = 1.0
+    a[20] *= 2.0 ** -120
+    b[:, 30] *= 2.0 ** 118
+    a[21] *= 2.0 ** 110
+    b[:, 31] *= 2.0 ** -122
+    ws = torch.empty(K.matmul_workspace_bytes(1, m, n, k), dtype=torch.uint8, device=cuda)
+    got = K.matmul(a, b, workspace=ws).double()
+    want = a.double() @ b.double()
+    assert torch.equal(torch.isnan(got), torch.isnan(want))
+    inf = torch.isinf(want)
+    assert bool((got[inf] == want[inf]).all())
+    fine = torch.isfinite(want) & (want.abs() < 2.0 ** 127)
+    mag = torch.nan_to_num(a.double().abs(), posinf=0.0) @ torch.nan_to_num(b.double().abs(), posinf=0.0)
+    bound = mag * (3 * 2.0 ** -22 + 2.0 ** -23 * (k / 16 + 2)) + 2.0 ** -125
+    assert bool(((got - want).abs() <= bound)[fine].all())
