@@ -2603,6 +2603,9 @@ PackedWeights* Instance::packed_for(int node_index, int64_t rows) {
             src.vec[j] = pw.n[j] % 4 == 0 && pw.col0[j] % 4 == 0 && reinterpret_cast<uintptr_t>(w.data) % 16 == 0;
         }
         check_rc(split_weights_pack(stream, src, pw.w));
+        // Later runs ask for these weights before they wait for the kernel in front of them.  A memset has no early start: it waits for the
+        // packing, whatever comes behind it waits for it, so no kernel that starts early can be ahead of the packing.
+        check_cuda(cudaMemsetAsync(pw.w.scale + pw.w.n_blocks * 128, 0, 4, stream), "packing barrier");
         launches += 2;
         pw.packed_run = run_counter;
     }
