@@ -477,45 +477,74 @@ void HostBlock::release() {
     base = nullptr;
 }
 
-// Pinned buffers for results (rmlk_host_alloc): carved from slabs of 8 MB, reused by size, at most 64 MB in all.  The slabs stay until the
-// process ends - pinning takes a millisecond, a result is wanted every step.
+// Pinned buffers for results (rmlk_host_alloc): carved from slabs of 8 MB, reused by size, at most 64 MB in all.  A slab with nothing
+// handed out starts anew; one such slab is kept, any further one is given back.  (Pinning takes a millisecond, a result is wanted
+// every step.)
 namespace {
 struct ResultPool {
-    static constexpr size_t SLAB = size_t(8) << 20, MOST = size_t(64) << 20, UNIT = size_t(32) << 10;
+    static constexpr size_t SLAB = size_t(8) << 20, SLABS_MOST = 8, UNIT = size_t(32) << 10;
+    struct Slab {
+        char* base;
+        size_t used = 0;  // carved so far
+        int live = 0;     // pieces handed out
+        std::multimap<size_t, char*> free_;
+    };
     std::mutex mutex;
-    std::multimap<size_t, char*> free_;
-    char* slab = nullptr;
-    size_t left = 0, total = 0;
+    std::vector<Slab> slabs;
+    static size_t rounded(size_t bytes) { return round_up(std::max<size_t>(bytes, 1), UNIT); }
     void* alloc(size_t bytes) {
-        const size_t n = round_up(std::max<size_t>(bytes, 1), UNIT);
+        if (bytes > SLAB) return nullptr;
+        const size_t n = rounded(bytes);
         std::lock_guard<std::mutex> lock(mutex);
-        auto it = free_.lower_bound(n);
-        if (it != free_.end() && it->first == n) {
+        for (Slab& s : slabs) {
+            auto it = s.free_.find(n);
+            if (it == s.free_.end()) continue;
             char* p = it->second;
-            free_.erase(it);
+            s.free_.erase(it);
+            s.live++;
             return p;
         }
-        if (n > SLAB) return nullptr;
-        if (left < n) {
-            if (total + SLAB > MOST) return nullptr;
+        Slab* room = nullptr;
+        for (Slab& s : slabs)
+            if (SLAB - s.used >= n) room = &s;
+        if (!room) {
+            if (slabs.size() >= SLABS_MOST) return nullptr;
+            slabs.reserve(slabs.size() + 1);
             void* p = nullptr;
             if (cudaHostAlloc(&p, SLAB, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
                 cudaGetLastError();
                 return nullptr;
             }
-            for (; left >= UNIT; left -= UNIT, slab += UNIT) free_.emplace(UNIT, slab);  // the rest of the old slab
-            slab = static_cast<char*>(p);
-            left = SLAB;
-            total += SLAB;
+            slabs.emplace_back();
+            room = &slabs.back();
+            room->base = static_cast<char*>(p);
         }
-        char* p = slab;
-        slab += n;
-        left -= n;
+        char* p = room->base + room->used;
+        room->used += n;
+        room->live++;
         return p;
     }
-    void release(void* p, size_t bytes) {
+    void release(void* ptr, size_t bytes) {
+        char* p = static_cast<char*>(ptr);
         std::lock_guard<std::mutex> lock(mutex);
-        free_.emplace(round_up(std::max<size_t>(bytes, 1), UNIT), static_cast<char*>(p));
+        size_t idle = 0, at = slabs.size();
+        for (size_t i = 0; i < slabs.size(); i++) {
+            Slab& s = slabs[i];
+            if (p >= s.base && p < s.base + SLAB) {
+                at = i;
+                if (--s.live == 0) {
+                    s.free_.clear();
+                    s.used = 0;
+                } else {
+                    s.free_.emplace(rounded(bytes), p);
+                }
+            }
+            idle += s.live == 0;
+        }
+        if (at < slabs.size() && slabs[at].live == 0 && idle > 1) {
+            cudaFreeHost(slabs[at].base);
+            slabs.erase(slabs.begin() + static_cast<ptrdiff_t>(at));
+        }
     }
 };
 ResultPool& result_pool() {
@@ -523,9 +552,19 @@ ResultPool& result_pool() {
     return *pool;
 }
 }  // namespace
-void* host_result_alloc(size_t bytes) { return result_pool().alloc(bytes); }
+void* host_result_alloc(size_t bytes) {
+    try {
+        return result_pool().alloc(bytes);
+    } catch (...) {  // no memory for the bookkeeping: as if the pool were used up
+        return nullptr;
+    }
+}
 void host_result_free(void* p, size_t bytes) {
-    if (p) result_pool().release(p, bytes);
+    if (!p) return;
+    try {
+        result_pool().release(p, bytes);
+    } catch (...) {  // the piece is reused when its slab starts anew
+    }
 }
 
 // Feeds host data to a device buffer of the instance (16-byte aligned).  Inputs up to 1 MB are copied to pinned memory and fetched by a
