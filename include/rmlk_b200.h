@@ -455,6 +455,14 @@ RMLK_API int rmlk_b200_gqa_decode_attention_ws(rmlk_stream_t stream, int dtype, 
                                       int64_t kv_heads, const void* q, const void* k, int64_t k_problem_stride, const void* v,
                                       int64_t v_problem_stride, float scale, const void* mask, int64_t mask_batch_stride,
                                       int64_t mask_head_stride, void* out, void* workspace, size_t workspace_bytes);
+/* Attention of `queries` tokens per request over the same kind of cache, one launch: query row (r, s) of a problem is token s of query head r
+ * of its KV head.  q: [problems, rows, queries, head_dim] dense; mask: rows of `keys` floats at b * mask_strides[0] + h * mask_strides[1] +
+ * s * mask_strides[2] (b, h as above), or NULL; out: rows of head_dim floats at b * out_strides[0] + h * out_strides[1] + s * out_strides[2].
+ * head_dim 64 (rmlk_b200_gqa_prefill_attention_supported).  `status`: device-visible word set when a bounded wait expires, or NULL. */
+RMLK_API int rmlk_b200_gqa_prefill_attention(rmlk_stream_t stream, int dtype, int64_t problems, int64_t rows, int64_t queries, int64_t head_dim, int64_t keys,
+                                    int64_t kv_heads, const void* q, const void* k, int64_t k_problem_stride, const void* v, int64_t v_problem_stride,
+                                    float scale, const void* mask, const int64_t* mask_strides, void* out, const int64_t* out_strides, int* status);
+RMLK_API int rmlk_b200_gqa_prefill_attention_supported(int64_t queries, int64_t rows, int64_t head_dim, int64_t keys);
 RMLK_API size_t rmlk_b200_gqa_decode_attention_workspace_bytes(int64_t problems, int64_t rows, int64_t head_dim, int64_t keys);
 
 /* SwiGLU gate as exported: Mul(Mul(gate, Sigmoid(gate)), up), n elements each.  Replaces backend/sigmoid.rs (cuDNN

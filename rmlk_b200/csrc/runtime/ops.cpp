@@ -2187,7 +2187,7 @@ bool Instance::run_fused(const FusedGroup& fg) {
                 return false;
             if (q->shape.size() != 4 || kt->shape.size() != 4 || vh->shape.size() != 4 || q->parts > 1) return false;
             const int64_t B = q->shape[0], H = q->shape[1], S = q->shape[2], D = q->shape[3], T = kt->shape[3];
-            if (S != 1 || B <= 0 || H <= 0 || kt->shape[0] != B || kt->shape[1] != H || kt->shape[2] != D || vh->shape != Shape({B, H, T, D})) return false;
+            if (S < 1 || B <= 0 || H <= 0 || kt->shape[0] != B || kt->shape[1] != H || kt->shape[2] != D || vh->shape != Shape({B, H, T, D})) return false;
             {
                 const NodeDef& smn = g.nodes[groups[fg.sub].root];
                 const int64_t axis = Ctx{*this, smn}.attr_int("axis", -1);
@@ -2197,15 +2197,33 @@ bool Instance::run_fused(const FusedGroup& fg) {
             LazyB lk, lv;
             if (!analyze_lazy_b(*kt, D, T, lk) || !lk.transposed || !analyze_lazy_b(*vh, T, D, lv) || lv.transposed) return false;
             if (lk.fold != lv.fold || lk.outer != lv.outer || lk.outer * lk.fold != B * H || H % lk.fold) return false;
-            if (!rmlk_b200_gqa_decode_attention_supported(lk.fold, D, T)) return false;
+            if (S == 1 ? !rmlk_b200_gqa_decode_attention_supported(lk.fold, D, T) : !rmlk_b200_gqa_prefill_attention_supported(S, lk.fold, D, T)) return false;
             if (lk.outer > 1 && (lk.sb % 4 || lv.sb % 4)) return false;
             if (reinterpret_cast<uintptr_t>(kt->data) % 16 || reinterpret_cast<uintptr_t>(vh->data) % 16) return false;
             if (mk->lazy) materialize(*mk);
             int64_t ms[4];
-            const Shape sshape = {B, H, 1, T};
+            const Shape sshape = {B, H, S, T};
             if (mk->shape.size() > 4 || mk->shape.empty() || mk->shape.back() != T || !bcast_strides(*mk, sshape, ms) || (T > 1 && ms[3] != 1)) return false;
             if (q->lazy) materialize(*q);
             const void *kdata = kt->data, *vdata = vh->data;
+            if (S != 1) {
+                const int ov = root.outputs[0];
+                const Shape oshape = {B, H, S, D};
+                Tensor& o = c.make(0, RMLK_F32, oshape);
+                // The result is laid out [B, S, H, D], what the Transpose behind the attention makes of it: that is then a view, and dense.
+                Shape ost = {H * S * D, S * D, D, 1};
+                if (!g.values[ov].is_output && binding_of_out[ov] < 0 && o.storage) {
+                    ost = {S * H * D, D, H * D, 1};
+                    Storage* keep = o.storage;
+                    set_strided(o, o.data, oshape, ost);
+                    o.storage = keep;
+                }
+                check_rc(rmlk_b200_gqa_prefill_attention(st, RMLK_F32, lk.outer, lk.fold, S, D, T, H / lk.fold, q->data, kdata, lk.sb, vdata, lv.sb, scale, mk->data, ms,
+                                                         o.data, ost.data(), status_ptr()));
+                status_dirty = true;
+                launches++;
+                return true;
+            }
             if (!attention_split && (lk.fold * D) % 64 == 0 && pairs_wanted(root.outputs[0], B, H * D, true)) {
                 const float* qd = static_cast<const float*>(q->data);
                 Tensor& o = make_pairs(root.outputs[0], Shape({B, H, 1, D}), B, H * D, static_cast<int>(lk.fold * D / 64));

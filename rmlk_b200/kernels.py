@@ -441,6 +441,27 @@ def rope_copy_batch(jobs) -> None:
     _check(lib().rmlk_b200_rope_copy_batch(_stream(), len(jobs), arr))
 
 
+def gqa_prefill_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale: float, mask: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """q [B, KV, G, S, 64]; k, v [B, KV, T, 64] as for gqa_decode_attention; mask [B, 1 or KV*G, S, T] or None -> [B, S, KV*G, 64]."""
+    _require_cuda(q, mask)
+    B, KV, G, S, D = q.shape
+    T = k.shape[2]
+    assert k.is_cuda and v.is_cuda and k.shape == v.shape == (B, KV, T, D) and q.is_contiguous()
+    assert k.stride(3) == 1 and k.stride(2) == D and v.stride(3) == 1 and v.stride(2) == D
+    assert k.stride(0) == KV * k.stride(1) and v.stride(0) == KV * v.stride(1)
+    out = torch.empty((B, S, KV * G, D), dtype=q.dtype, device=q.device)
+    ms = [0, 0, 0]
+    if mask is not None:
+        assert mask.dim() == 4 and mask.shape[0] == B and mask.shape[2] == S and mask.shape[3] == T and mask.stride(3) == 1
+        ms = [mask.stride(0), mask.stride(1) if mask.shape[1] > 1 else 0, mask.stride(2)]
+    _check(lib().rmlk_b200_gqa_prefill_attention(
+        _stream(), dt.from_torch(q.dtype), ctypes.c_int64(B * KV), ctypes.c_int64(G), ctypes.c_int64(S), ctypes.c_int64(D), ctypes.c_int64(T),
+        ctypes.c_int64(KV), _ptr(q), ctypes.c_void_p(k.data_ptr()), ctypes.c_int64(k.stride(1)), ctypes.c_void_p(v.data_ptr()),
+        ctypes.c_int64(v.stride(1)), ctypes.c_float(scale), ctypes.c_void_p(0 if mask is None else mask.data_ptr()), _i64(ms), _ptr(out),
+        _i64([out.stride(0), out.stride(2), out.stride(1)]), None))
+    return out
+
+
 def gqa_decode_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale: float, mask: Optional[torch.Tensor] = None,
                          split: bool = False, workspace: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """q [B, KV, G, D] (G <= 4 query heads per KV head, one token each); k, v [B, KV, T, D] views whose [T, D] blocks are
