@@ -153,21 +153,27 @@ __global__ void __launch_bounds__(SK_THREADS) skinny_kernel(SkinnyParams p) {
 // wide-strip small-M MatMul (M <= 16, rows of B 16-byte aligned): the decode GEMV
 // ---------------------------------------------------------------------------------------------
 // Memory-bound: B is read exactly once.  A CTA owns a strip of 128 columns (a warp-wide load is one 512-byte piece
-// of a row of B; 128-byte pieces stream a fifth slower) and a range of K; its 16 warps take rows k, k + 16, ... of the
-// range, each thread holding 8 independent 128-bit loads in flight (64 KB per CTA, two CTAs per SM).  A round covers 128 rows
-// of B: the loads go out first, then the 128 x MB block of A is staged in shared memory as [k][m] under them, then the FMAs.
+// of a row of B; 128-byte pieces stream a fifth slower) and a range of K; its W warps take rows k, k + W, ... of the
+// range, each thread holding 8 independent 128-bit loads in flight.  A round covers 8 W rows of B: the loads go out first,
+// then the 8 W x MB block of A is staged in shared memory as [k][m] under them, then the FMAs.  Up to 4 rows: 16 warps, two CTAs per SM;
+// more rows need the registers for their sums: 8 warps, three CTAs per SM, so that the FMAs of one run under the loads of the others (one CTA
+// of 16 warps: [8,4096] x [4096,14336] 82 us, this 60 us - what the tensor-core kernel takes, which has these rows where it can).
 // Weights that nothing in flight writes (b_static) are requested for the first round before the kernel waits for its
-// predecessor: the stream starts while that one drains.  K is split until the grid has about two CTAs per SM (the partial sums go
-// through the caller's scratch and a fixed-order sum); the 16 k-lanes are added by a tree through shared memory.
-// 8 warps and six CTAs per SM streamed as fast, but cut K into two to three times as many slabs for the reader to add.
+// predecessor: the stream starts while that one drains.  K is split until the grid fills the SMs; the k-lanes of a CTA are added by a tree
+// through shared memory.  Up to 8 splits form a thread-block cluster whose first CTA adds the others' sums out of their shared memory, in
+// order ([1,2048] x [2048,8192] 18.6 -> 12.4 us against a second kernel for the sum); more go through the caller's scratch and a fixed-order sum,
+// as do all of them for a caller that adds slabs itself (its kernel reads them as fast: a decode step is the same either way).
+// A staged for many rounds at a time, which takes the barriers out of the loop, measured 6 % slower in a decode step.
+// 8 warps and six CTAs per SM for one row streamed as fast, but cut K into two to three times as many slabs for the reader to add.
 constexpr int GW_COLS = 128;
 constexpr int GW_U = 8;                 // loads in flight per thread
-constexpr int GW_WARPS = 16;
-constexpr int GW_KR = GW_WARPS * GW_U;  // rows of B per round
-constexpr int GW_THREADS = 32 * GW_WARPS;
+constexpr int GW_CLUSTER = 8;           // largest portable cluster
+constexpr int gw_warps(int64_t mb) { return mb <= 4 ? 16 : 8; }
+constexpr int gw_ctas(int64_t mb) { return mb <= 4 ? 2 : mb <= 8 ? 3 : 2; }  // per SM
 
-template <int MB>
-__global__ void __launch_bounds__(GW_THREADS, MB <= 4 ? 2 : 1) gemv_wide_kernel(SkinnyParams p) {
+template <int MB, bool CLUSTER>
+__global__ void __launch_bounds__(32 * gw_warps(MB), gw_ctas(MB)) gemv_wide_kernel(SkinnyParams p) {
+    constexpr int GW_WARPS = gw_warps(MB), GW_THREADS = 32 * GW_WARPS, GW_KR = GW_WARPS * GW_U;
     dep_trigger();
     __shared__ __align__(16) float sA[GW_KR * MB];
     constexpr int SLOTS = MB <= 8 ? GW_WARPS / 2 : GW_WARPS / 4;  // warps whose sums are in shared memory at a time
@@ -259,24 +265,67 @@ __global__ void __launch_bounds__(GW_THREADS, MB <= 4 ? 2 : 1) gemv_wide_kernel(
             }
         }
     }
+    if constexpr (CLUSTER) {  // the K splits of the strip: blockIdx.y is the rank
+        if (warp == 0 && split > 0) {
+#pragma unroll
+            for (int m = 0; m < MB; m++)
+                *reinterpret_cast<float4*>(sRed + m * GW_COLS + lane * 4) = make_float4(acc[m][0], acc[m][1], acc[m][2], acc[m][3]);
+        }
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (warp == 0 && split == 0) {
+            const uint32_t mine = static_cast<uint32_t>(__cvta_generic_to_shared(sRed + lane * 4));
+            for (int r = 1; r < p.ksplit; r++) {
+                uint32_t from;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(from) : "r"(mine), "r"(r));
+#pragma unroll
+                for (int m = 0; m < MB; m++) {
+                    float4 t;
+                    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(t.x), "=f"(t.y), "=f"(t.z), "=f"(t.w) : "r"(from + m * GW_COLS * 4) : "memory");
+                    acc[m][0] += t.x; acc[m][1] += t.y; acc[m][2] += t.z; acc[m][3] += t.w;
+                }
+            }
+        }
+        // no CTA leaves while the first one may still read its shared memory
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (split > 0) return;
+    }
     if (warp == 0 && in_cols) {
-        float* __restrict__ C = p.c + (p.ksplit > 1 ? (static_cast<int64_t>(split) * gridDim.z + batch) * p.M * p.N : batch * p.sc);
+        float* __restrict__ C = p.c + (!CLUSTER && p.ksplit > 1 ? (static_cast<int64_t>(split) * gridDim.z + batch) * p.M * p.N : batch * p.sc);
 #pragma unroll
         for (int m = 0; m < MB; m++)
             if (m < p.M) *reinterpret_cast<float4*>(C + static_cast<int64_t>(m) * p.N + n0) = make_float4(acc[m][0], acc[m][1], acc[m][2], acc[m][3]);
     }
 }
 
-// K split of the wide-strip kernel: about two CTAs per SM, ranges that are multiples of a round.
+// K split of the wide-strip kernel: until the SMs are full, ranges that are multiples of a round.
 static int gemv_wide_plan(int64_t batch, int64_t m, int64_t n, int64_t k, int64_t* k_per_split) {
-    const int64_t strips = ceil_div64(n, GW_COLS) * batch;
-    const int64_t rounds = ceil_div64(k, GW_KR);
-    int64_t s = (m <= 4 ? 2ll : 1ll) * sm_count() / strips;
+    const int64_t strips = ceil_div64(n, GW_COLS) * batch, kr = gw_warps(m) * GW_U;
+    const int64_t rounds = ceil_div64(k, kr);
+    int64_t s = static_cast<int64_t>(gw_ctas(m)) * sm_count() / strips;
     if (s > rounds) s = rounds;
     if (s < 1) s = 1;
     if (s > 64) s = 64;
-    *k_per_split = ceil_div64(rounds, s) * GW_KR;
+    *k_per_split = ceil_div64(rounds, s) * kr;
     return static_cast<int>(ceil_div64(k, *k_per_split));
+}
+
+template <int MB>
+static cudaError_t gemv_wide_launch(cudaStream_t st, const SkinnyParams& p, dim3 grid, bool cluster) {
+    if (!cluster) return launch_dep(gemv_wide_kernel<MB, false>, grid, dim3(32 * gw_warps(MB)), 0, st, p);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(32 * gw_warps(MB));
+    cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 1;
+    at[0].val.clusterDim.y = grid.y;
+    at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = dep_launch_enabled() ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, gemv_wide_kernel<MB, true>, p);
 }
 
 // Many small problems with a short K (decode attention scores: batch x heads problems of [1, 64] x [64, T]).
@@ -846,7 +895,7 @@ static bool gemv_wide_takes(int64_t batch, int64_t m, int64_t n, int64_t k, cons
 }
 // Returns the number of K slabs left in `workspace` (1: c holds the result).
 static int gemv_wide(cudaStream_t st, int64_t batch, int64_t m, int64_t n, int64_t k, const void* a, int64_t sa, const void* b, int64_t sb, void* c, int64_t sc,
-                     void* workspace, size_t workspace_bytes, int flags) {
+                     void* workspace, size_t workspace_bytes, int flags, bool slabs = false) {
     SkinnyParams p;
     p.a = static_cast<const float*>(a);
     p.b = static_cast<const float*>(b);
@@ -857,19 +906,23 @@ static int gemv_wide(cudaStream_t st, int64_t batch, int64_t m, int64_t n, int64
     int64_t kps = k;
     int ksplit = gemv_wide_plan(batch, m, n, k, &kps);
     const size_t need = static_cast<size_t>(ksplit) * batch * m * n * sizeof(float);
-    if (ksplit > 1 && (!workspace || workspace_bytes < need || !aligned_to(workspace, 16))) {
-        ksplit = 1;
-        kps = k;
+    const bool scratch = workspace && workspace_bytes >= need && aligned_to(workspace, 16);
+    if (ksplit > GW_CLUSTER && !scratch) {  // as many splits as a cluster takes
+        const int64_t kr = gw_warps(m) * GW_U;
+        kps = ceil_div64(ceil_div64(k, kr), GW_CLUSTER) * kr;
+        ksplit = static_cast<int>(ceil_div64(k, kps));
     }
+    const bool cluster = ksplit > 1 && ksplit <= GW_CLUSTER && !(slabs && scratch);
     p.ksplit = ksplit;
     p.k_per_split = kps;
-    p.c = ksplit > 1 ? static_cast<float*>(workspace) : static_cast<float*>(c);
+    p.c = ksplit > 1 && !cluster ? static_cast<float*>(workspace) : static_cast<float*>(c);
     const dim3 grid(static_cast<unsigned>(ceil_div64(n, GW_COLS)), ksplit, static_cast<unsigned>(batch));
-    if (m == 1) launch_dep(gemv_wide_kernel<1>, grid, dim3(GW_THREADS), 0, st, p);
-    else if (m == 2) launch_dep(gemv_wide_kernel<2>, grid, dim3(GW_THREADS), 0, st, p);
-    else if (m <= 4) launch_dep(gemv_wide_kernel<4>, grid, dim3(GW_THREADS), 0, st, p);
-    else if (m <= 8) launch_dep(gemv_wide_kernel<8>, grid, dim3(GW_THREADS), 0, st, p);
-    else launch_dep(gemv_wide_kernel<16>, grid, dim3(GW_THREADS), 0, st, p);
+    if (m == 1) gemv_wide_launch<1>(st, p, grid, cluster);
+    else if (m == 2) gemv_wide_launch<2>(st, p, grid, cluster);
+    else if (m <= 4) gemv_wide_launch<4>(st, p, grid, cluster);
+    else if (m <= 8) gemv_wide_launch<8>(st, p, grid, cluster);
+    else gemv_wide_launch<16>(st, p, grid, cluster);
+    if (cluster) ksplit = 1;
     return ksplit;
 }
 
@@ -889,7 +942,7 @@ extern "C" int rmlk_b200_matmul_parts(rmlk_stream_t stream, int dtype, int64_t m
         return RMLK_OK;
     }
     if (dtype == RMLK_F32 && gemv_wide_takes(1, m, n, k, a, b, 0, c, 0)) {
-        *parts = gemv_wide(as_stream(stream), 1, m, n, k, a, 0, b, 0, c, 0, workspace, workspace_bytes, flags);
+        *parts = gemv_wide(as_stream(stream), 1, m, n, k, a, 0, b, 0, c, 0, workspace, workspace_bytes, flags, true);
         RMLK_CHECK_LAUNCH("gemv_wide_kernel");
         return RMLK_OK;
     }
