@@ -30,11 +30,16 @@ def size(code: int) -> int:
     return to_numpy(code).itemsize
 
 
+_FROM_TORCH = {}
+
+
 def from_torch(dt) -> int:
-    import torch
-    return {torch.float16: F16, torch.float32: F32, torch.float64: F64, torch.int32: I32, torch.int64: I64,
-            torch.uint8: U8, torch.int8: I8, torch.int16: I16, torch.bool: BOOL, torch.uint16: U16, torch.uint32: U32,
-            torch.uint64: U64}[dt]
+    if not _FROM_TORCH:  # (torch is imported by whoever has a torch dtype to ask about)
+        import torch
+        _FROM_TORCH.update({torch.float16: F16, torch.float32: F32, torch.float64: F64, torch.int32: I32, torch.int64: I64,
+                            torch.uint8: U8, torch.int8: I8, torch.int16: I16, torch.bool: BOOL, torch.uint16: U16, torch.uint32: U32,
+                            torch.uint64: U64})
+    return _FROM_TORCH[dt]
 
 
 def to_torch(code: int):
