@@ -8,11 +8,13 @@
 // come out of TMEM into its registers, the running maximum and sum and the 64 output sums stay in registers in fp32, and the
 // probabilities go back through shared memory as pairs.
 //
-// What bounds it: issue slots of the softmax (about 45 instructions per score for the two splits, mask, maximum and expf), not the MMAs.  Two
-// CTAs per SM (98 KB, 256 TMEM columns each), so that one computes while the other waits for its MMAs.
+// What bounds it: the chain of one block - mask and keys in, scores, softmax, probabilities, values - through which a CTA goes step by step; issue
+// slots are 32 % busy.  Two CTAs per SM (98 KB, 256 TMEM columns, 255 registers) overlap their chains.  [4, 32 heads, 512] queries over 512 keys
+// take 110 us, with 2-norm error 2.1e-7 (fp32 products and softmax op by op: 2.7e-7).
 // Prompts of 16 x 512 tokens 80.9 -> 60.5 ms, of 3 x 187 tokens 5.5 -> 5.2 ms.
 // A block of keys whose mask is the lowest fp32 value (or -inf) for every row of the tile contributes exactly zero once a row has seen a
-// score of ordinary size; such a block - half of a causal prompt - is passed over when all its values are finite and of ordinary size.
+// score of ordinary size; such a block is passed over when all its values are finite and of ordinary size.
+// (Fetching it costs most of what a block costs: the causal mask above measured no faster than one that hides nothing.)
 #include <mutex>
 
 #include "split_pair.cuh"
