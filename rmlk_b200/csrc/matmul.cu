@@ -824,7 +824,7 @@ static bool split_pays(int64_t m, int64_t n, int64_t k) {
 }
 static size_t round1k(size_t v) { return (v + 1023) & ~static_cast<size_t>(1023); }
 static size_t split_workspace(int64_t m, int64_t n, int64_t k) {
-    const int parts = umma_split_parts(m, n, k);
+    const int parts = std::max(umma_split_parts(m, n, k, false), umma_split_parts(m, n, k, true));
     return 1024 + round1k(split_weights_bytes(n, k)) + round1k(split_rows_bytes(m, k, 0)) + (parts > 1 ? static_cast<size_t>(parts) * m * n * sizeof(float) : 0);
 }
 
@@ -993,7 +993,7 @@ extern "C" int rmlk_b200_matmul_flags(rmlk_stream_t stream, int dtype, int64_t b
         if (int rc = split_rows_pack(st, static_cast<const float*>(a), k, x)) return rc;
         int parts = 1;
         const size_t left = workspace_bytes - static_cast<size_t>(ws - static_cast<char*>(workspace));
-        if (int rc = umma_split(st, x, w, static_cast<float*>(c), n, reinterpret_cast<float*>(ws), left, status, 0, &parts)) return rc;
+        if (int rc = umma_split(st, x, w, static_cast<float*>(c), n, reinterpret_cast<float*>(ws), left, status, 0, !tc_matmul_eligible(m, n, k, a, b, c), &parts)) return rc;
         if (parts > 1) return rmlk_b200_sum_parts(stream, dtype, parts, m * n, ws, c);
         return RMLK_OK;
     }

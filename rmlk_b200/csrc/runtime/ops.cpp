@@ -2700,8 +2700,10 @@ void Instance::packed_product(PackedWeights& pw, const SplitRows& x, int64_t n0,
     const SplitWeights w = n0 == 0 && n == pw.n_total ? pw.w : split_weights_window(pw.w, n0, n);
     float* sp = nullptr;
     size_t bytes = 0;
+    const bool short_sums = pw.n_total % 128 != 0 || pw.k % 32 != 0;
     if (parts) {
-        const int want = umma_split_parts(x.m, n, x.k);
+        // (rows that share a scale by chunks take the plan of short sums)
+        const int want = std::max(umma_split_parts(x.m, n, x.k, false), umma_split_parts(x.m, n, x.k, true));
         if (want > 1) {
             bytes = static_cast<size_t>(want) * x.m * n * sizeof(float);
             sp = static_cast<float*>(slabs->ensure(bytes));
@@ -2709,7 +2711,7 @@ void Instance::packed_product(PackedWeights& pw, const SplitRows& x, int64_t n0,
     }
     // from the run after the one that laid them out nothing in flight writes the weights
     const int flags = pw.packed_run < run_counter ? RMLK_MATMUL_B_STATIC : 0;
-    check_rc(umma_split(stream, x, w, out, ldc, sp, bytes, status_ptr(), flags, parts));
+    check_rc(umma_split(stream, x, w, out, ldc, sp, bytes, status_ptr(), flags, short_sums, parts));
     status_dirty = true;
     launches++;
 }

@@ -143,11 +143,14 @@ int umma_f16(cudaStream_t st, int64_t m, int64_t n, int64_t k, const void* a, co
     return dispatch<false, true>(st, pl, tmW, tmX, p);
 }
 
-int umma_split_parts(int64_t m, int64_t n, int64_t k) { return umma::plan_for(m, n, k, 3, true).ksplit; }
+int umma_split_parts(int64_t m, int64_t n, int64_t k, bool short_sums) { return umma::plan_for(m, n, k, 3, true, short_sums).ksplit; }
 
-int umma_split(cudaStream_t st, const SplitRows& x, const SplitWeights& w, float* out, int64_t ldc, float* slabs, size_t slab_bytes, int* status, int flags, int* parts) {
+constexpr int SHORT_BLOCKS = 4;
+int umma_split(cudaStream_t st, const SplitRows& x, const SplitWeights& w, float* out, int64_t ldc, float* slabs, size_t slab_bytes, int* status, int flags, bool short_sums,
+               int* parts) {
     using namespace umma;
-    const bool chunks = static_cast<int64_t>(x.chunk_blocks) * BK < x.k_pad;
+    const bool scales = static_cast<int64_t>(x.chunk_blocks) * BK < x.k_pad;  // a scale per chunk of a row
+    const bool chunks = scales || short_sums;
     Plan pl = plan_for(x.m, w.n, x.k, 3, parts != nullptr, chunks);
     if (pl.ksplit > 1 && slab_bytes < static_cast<size_t>(pl.ksplit) * x.m * w.n * sizeof(float)) pl = plan_for(x.m, w.n, x.k, 3, false, chunks);
     CUtensorMap tmW, tmX;
@@ -162,8 +165,8 @@ int umma_split(cudaStream_t st, const SplitRows& x, const SplitWeights& w, float
     p.x_lo_row = static_cast<int>(x.m_pad);
     p.w_scale = w.scale;
     p.x_scale = x.scale;
-    p.x_scale_pitch = x.scale_pitch;
-    p.chunk_blocks = x.chunk_blocks;
+    p.x_scale_pitch = scales ? x.scale_pitch : 0;  // one scale per row: every chunk reads the same one
+    p.chunk_blocks = scales || !short_sums ? x.chunk_blocks : SHORT_BLOCKS;
     p.w_static = (flags & RMLK_MATMUL_B_STATIC) ? 1 : 0;
     p.status = status;
     if (parts) *parts = p.ksplit;

@@ -109,3 +109,18 @@ def test_f32_split_non_finite_and_extreme(cuda, n, k):
     mag = torch.nan_to_num(a.double().abs(), posinf=0.0) @ torch.nan_to_num(b.double().abs(), posinf=0.0)
     bound = mag * (3 * 2.0 ** -22 + 2.0 ** -23 * (k / 16 + 2)) + 2.0 ** -125
     assert bool(((got - want).abs() <= bound)[fine].all())
+
+
+@pytest.mark.parametrize("m,k,n", [(1000, 777, 1003), (300, 4100, 260), (2048, 2050, 516), (512, 1025, 100)])
+def test_f32_split_ragged_accuracy(cuda, m, k, n):
+    """Sizes that FMA chains would otherwise take are no less accurate than those: 2-norm error at most that of fp32 sums over K."""
+    import torch
+    from rmlk_b200 import kernels as K
+    g = torch.Generator(device=cuda)
+    g.manual_seed(k)
+    a, b = torch.randn(m, k, device=cuda, generator=g), torch.randn(k, n, device=cuda, generator=g) * 0.02
+    ws = torch.empty(K.matmul_workspace_bytes(1, m, n, k), dtype=torch.uint8, device=cuda)
+    want = a.double() @ b.double()
+    # the same call without workspace runs on the FMA kernel
+    split, fma = K.matmul(a, b, workspace=ws).double(), K.matmul(a, b).double()
+    assert float((split - want).norm()) <= float((fma - want).norm())
