@@ -2643,10 +2643,18 @@ void Instance::find_pairs() {
     for (size_t v = 0; v < g.values.size(); v++) {
         int at = static_cast<int>(v);
         bool through = false;
-        // [B, heads, 1, D] -> Transpose -> Reshape -> [B, 1, heads D]
+        // [B, heads, 1, D] -> Transpose -> Reshape -> [B, 1, heads D]: pairs lie in the order of [B, heads, D], so the Transpose may move
+        // nothing but the one token, and its operand must be the four-dimensional value itself
         while (plain(at) && readers[at].size() == 1) {
             const NodeDef& n = g.nodes[readers[at][0]];
             if ((n.op != RMLK_OP_TRANSPOSE && n.op != RMLK_OP_RESHAPE) || n.inputs[0] != at || n.outputs.empty()) break;
+            if (n.op == RMLK_OP_TRANSPOSE) {
+                auto pa = n.attrs.find("perm");
+                if (through || pa == n.attrs.end() || pa->second.kind != Attr::INTS) break;
+                std::vector<int64_t> rest = pa->second.ints;
+                rest.erase(std::remove(rest.begin(), rest.end(), 2), rest.end());
+                if (pa->second.ints.size() != 4 || rest != std::vector<int64_t>({0, 1, 3})) break;
+            }
             at = n.outputs[0];
             through = true;
         }
