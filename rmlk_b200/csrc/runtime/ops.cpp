@@ -2106,7 +2106,9 @@ bool Instance::run_fused(const FusedGroup& fg) {
             int64_t pg = 0, pu = 0;
             const bool pitched = (gt->lazy || up->lazy) && !gt->shape.empty() && gt->shape.back() % 4 == 0 && as_rows(*gt, pg) && as_rows(*up, pu) &&
                                  pg % 4 == 0 && pu % 4 == 0 && reinterpret_cast<uintptr_t>(gt->data) % 16 == 0 && reinterpret_cast<uintptr_t>(up->data) % 16 == 0;
-            if (unsummed.y && gt->storage == unsummed.y && up->storage == unsummed.y && last_use[fg.v[0]] == fg.root && last_use[fg.v[1]] == fg.root &&
+            // (three references: gate, up and `unsummed` itself - any further member of the merged product still wants the sum)
+            if (unsummed.y && gt->storage == unsummed.y && up->storage == unsummed.y && fg.v[0] != fg.v[1] && unsummed.y->refs == 3 &&
+                last_use[fg.v[0]] == fg.root && last_use[fg.v[1]] == fg.root &&
                 pending_jobs.empty() && !gt->shape.empty() && gt->shape.back() % 4 == 0 && as_rows(*gt, pg) && as_rows(*up, pu) && pg % 4 == 0 && pu % 4 == 0 &&
                 unsummed.part_stride % 4 == 0) {
                 // the product's K slabs have not been added up and nothing else reads them: added here, as they are read

@@ -52,3 +52,29 @@ def test_transposed_attention_result(cuda, B, perm):
     got = inst.run(feeds)["y"]
     want = graph_cpu.run_graph(g, feeds)["y"]
     assert np.max(np.abs(got - want)) <= 1e-4 * np.max(np.abs(want))
+
+
+# one merged product of which SwiGLU reads two blocks, and another op a third one behind it; fp32 slabs (1, 4 rows) and pairs (8, 64)
+@pytest.mark.parametrize("rows", [1, 4, 8, 64])
+@pytest.mark.parametrize("third_first", [False, True])
+def test_third_reader_of_a_product_behind_swiglu(cuda, rows, third_first):
+    from rmlk_b200.runtime import ModelInstance
+    K, N = 2048, 512
+    g = GraphSpec()
+    g.input("x", np.float32, [0, K])
+    r = np.random.default_rng(rows)
+    names = ["third", "gate", "up"] if third_first else ["gate", "up", "third"]
+    for n in names:
+        g.const("w_" + n, (r.standard_normal((K, N)) * 0.03).astype(np.float32))
+    for n in names:
+        g.op("MatMul", ["x", "w_" + n], n)
+    g.op("Mul", [g.op("Mul", ["gate", g.op("Sigmoid", ["gate"])]), "up"], "act")
+    g.op("Neg", ["third"], "late")
+    g.output("act")
+    g.output("late")
+    inst = ModelInstance(g.to_runtime())
+    for _ in range(2):
+        x = r.standard_normal((rows, K), dtype=np.float32)
+        got, want = inst.run({"x": x}), graph_cpu.run_graph(g, {"x": x})
+        for n in ("act", "late"):
+            assert np.max(np.abs(got[n] - want[n])) <= 1e-4 * np.max(np.abs(want[n])), n
