@@ -113,10 +113,6 @@ RMLK_API int rmlk_instance_stream_output(rmlk_instance* inst, const char* name, 
 RMLK_API int rmlk_instance_wait_outputs(rmlk_instance* inst);
 /* Copies a value to host memory and waits for it (get_outputs, runtime/src/core/instance.rs:58-82). */
 RMLK_API int rmlk_instance_read(rmlk_instance* inst, const char* name, void* dst, size_t nbytes);
-/* Pinned host memory for results: rmlk_instance_read into it takes half as long as into pageable memory.  NULL when the
- * process-wide allowance (64 MB, blocks up to 8 MB) is in use; rmlk_host_free takes the size that was asked for. */
-RMLK_API void* rmlk_host_alloc(size_t nbytes);
-RMLK_API void rmlk_host_free(void* p, size_t nbytes);
 /* Number of kernels / async copies enqueued by the last run, and number of times it had to wait for
  * the device (0 when all small operands had host mirrors). */
 RMLK_API int64_t rmlk_instance_last_launches(const rmlk_instance* inst);

@@ -477,96 +477,6 @@ void HostBlock::release() {
     base = nullptr;
 }
 
-// Pinned buffers for results (rmlk_host_alloc): carved from slabs of 8 MB, reused by size, at most 64 MB in all.  A slab with nothing
-// handed out starts anew; one such slab is kept, any further one is given back.  (Pinning takes a millisecond, a result is wanted
-// every step.)
-namespace {
-struct ResultPool {
-    static constexpr size_t SLAB = size_t(8) << 20, SLABS_MOST = 8, UNIT = size_t(32) << 10;
-    struct Slab {
-        char* base;
-        size_t used = 0;  // carved so far
-        int live = 0;     // pieces handed out
-        std::multimap<size_t, char*> free_;
-    };
-    std::mutex mutex;
-    std::vector<Slab> slabs;
-    static size_t rounded(size_t bytes) { return round_up(std::max<size_t>(bytes, 1), UNIT); }
-    void* alloc(size_t bytes) {
-        if (bytes > SLAB) return nullptr;
-        const size_t n = rounded(bytes);
-        std::lock_guard<std::mutex> lock(mutex);
-        for (Slab& s : slabs) {
-            auto it = s.free_.find(n);
-            if (it == s.free_.end()) continue;
-            char* p = it->second;
-            s.free_.erase(it);
-            s.live++;
-            return p;
-        }
-        Slab* room = nullptr;
-        for (Slab& s : slabs)
-            if (SLAB - s.used >= n) room = &s;
-        if (!room) {
-            if (slabs.size() >= SLABS_MOST) return nullptr;
-            slabs.reserve(slabs.size() + 1);
-            void* p = nullptr;
-            if (cudaHostAlloc(&p, SLAB, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
-                cudaGetLastError();
-                return nullptr;
-            }
-            slabs.emplace_back();
-            room = &slabs.back();
-            room->base = static_cast<char*>(p);
-        }
-        char* p = room->base + room->used;
-        room->used += n;
-        room->live++;
-        return p;
-    }
-    void release(void* ptr, size_t bytes) {
-        char* p = static_cast<char*>(ptr);
-        std::lock_guard<std::mutex> lock(mutex);
-        size_t idle = 0, at = slabs.size();
-        for (size_t i = 0; i < slabs.size(); i++) {
-            Slab& s = slabs[i];
-            if (p >= s.base && p < s.base + SLAB) {
-                at = i;
-                if (--s.live == 0) {
-                    s.free_.clear();
-                    s.used = 0;
-                } else {
-                    s.free_.emplace(rounded(bytes), p);
-                }
-            }
-            idle += s.live == 0;
-        }
-        if (at < slabs.size() && slabs[at].live == 0 && idle > 1) {
-            cudaFreeHost(slabs[at].base);
-            slabs.erase(slabs.begin() + static_cast<ptrdiff_t>(at));
-        }
-    }
-};
-ResultPool& result_pool() {
-    static ResultPool* pool = new ResultPool();  // never destroyed: results may outlive every static object
-    return *pool;
-}
-}  // namespace
-void* host_result_alloc(size_t bytes) {
-    try {
-        return result_pool().alloc(bytes);
-    } catch (...) {  // no memory for the bookkeeping: as if the pool were used up
-        return nullptr;
-    }
-}
-void host_result_free(void* p, size_t bytes) {
-    if (!p) return;
-    try {
-        result_pool().release(p, bytes);
-    } catch (...) {  // the piece is reused when its slab starts anew
-    }
-}
-
 // Feeds host data to a device buffer of the instance (16-byte aligned).  Inputs up to 1 MB are copied to pinned memory and fetched by a
 // kernel when the run starts, those of more than 256 KB in pieces, each on its way while the next is copied.  What is larger, or pinned
 // already and worth its own transfer, goes to the copy engine as it is.  [64, 2048] floats (512 KB) are fed in 16 us of host time; a
@@ -1258,9 +1168,6 @@ extern "C" int rmlk_instance_read(rmlk_instance* inst, const char* name, void* d
     return RMLK_OK;
     RT_CATCH
 }
-
-extern "C" void* rmlk_host_alloc(size_t nbytes) { return rmlk::rt::host_result_alloc(nbytes); }
-extern "C" void rmlk_host_free(void* p, size_t nbytes) { rmlk::rt::host_result_free(p, nbytes); }
 
 extern "C" int rmlk_instance_stream_output(rmlk_instance* inst, const char* name, void* host_dst, size_t nbytes) {
     RT_TRY

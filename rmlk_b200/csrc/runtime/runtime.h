@@ -363,8 +363,6 @@ struct Instance {
 };
 
 size_t dtype_size_of(int dt);
-void* host_result_alloc(size_t bytes);
-void host_result_free(void* p, size_t bytes);
 
 std::string status_word_message(int word);  // text for a non-zero device status word
 void check_cuda_fn(cudaError_t e, const char* what);

@@ -17,7 +17,6 @@ from __future__ import annotations
 
 import ctypes
 import enum
-import weakref
 from typing import Dict, Optional, Sequence
 
 import numpy as np
@@ -150,34 +149,12 @@ def _setup(l):
     l.rmlk_instance_value_info.argtypes = [ctypes.c_void_p, ctypes.c_char_p, ctypes.c_void_p, ctypes.c_void_p,
                                            ctypes.c_void_p, ctypes.c_void_p]
     l.rmlk_instance_read.argtypes = [ctypes.c_void_p, ctypes.c_char_p, ctypes.c_void_p, ctypes.c_size_t]
-    l.rmlk_host_alloc.restype = ctypes.c_void_p
-    l.rmlk_host_alloc.argtypes = [ctypes.c_size_t]
-    l.rmlk_host_free.restype = None
-    l.rmlk_host_free.argtypes = [ctypes.c_void_p, ctypes.c_size_t]
     l._rt_ready = True
     return l
 
 
 def _rt():
     return _setup(lib())
-
-
-_PINNED_FROM, _PINNED_TO = 32 << 10, 8 << 20
-
-
-def _result_array(l, shape, dtype) -> np.ndarray:
-    """An uninitialised array for a result.  From 32 KB on its memory is pinned, so that the device writes into it directly; it goes back
-    to the library's pool with the array.  (The pool is bounded: an ordinary array when it is used up.)"""
-    n = dtype.itemsize
-    for v in shape:
-        n *= v
-    if _PINNED_FROM <= n <= _PINNED_TO:
-        ptr = l.rmlk_host_alloc(n)
-        if ptr:
-            buf = (ctypes.c_char * n).from_address(ptr)
-            weakref.finalize(buf, l.rmlk_host_free, ptr, n).atexit = False
-            return np.frombuffer(buf, dtype=dtype).reshape(shape)
-    return np.empty(shape, dtype=dtype)
 
 
 class OpHandle:
@@ -328,7 +305,7 @@ class ModelInstance:
         key = self._key(name)
         # (no device address: asking for one would give a value that only the host knows device memory)
         _check(self._l.rmlk_instance_value_info(self._h, key, self._info_refs[0], self._info_refs[1], dims, None))
-        out = _result_array(self._l, dims[: r.value], dt.to_numpy(d.value))
+        out = np.empty(dims[: r.value], dtype=dt.to_numpy(d.value))  # pageable: a caller may change or drop it at once after feeding it on
         _check(self._l.rmlk_instance_read(self._h, key, out.__array_interface__["data"][0], out.nbytes))
         return out
 
