@@ -477,16 +477,16 @@ void HostBlock::release() {
     base = nullptr;
 }
 
-// Feeds host data to a device buffer of the instance (16-byte aligned).  Inputs up to 1 MB are copied to pinned memory and fetched by a
-// kernel when the run starts, those of more than 256 KB in pieces, each on its way while the next is copied.  What is larger, or pinned
-// already and worth its own transfer, goes to the copy engine as it is.  [64, 2048] floats (512 KB) are fed in 16 us of host time; a
-// pageable cudaMemcpyAsync takes 21 us and the stream's next kernel waits 18 us more for the copy engine.
+// Feeds host data to a device buffer of the instance (16-byte aligned).  Pageable inputs up to 1 MB are copied to pinned memory and fetched
+// by a kernel when the run starts, those of more than 256 KB in pieces, each on its way while the next is copied.  Memory that CUDA knows
+// (pinned, managed) is read by the copy engine in stream order: what the stream writes there before is what is fed.  [64, 2048] floats (512 KB)
+// are fed in 16 us of host time; a pageable cudaMemcpyAsync takes 21 us and the stream's next kernel waits 18 us more for the copy engine.
 void Instance::feed_host(void* dst, const void* src, size_t bytes) {
-    constexpr size_t SMALL = size_t(32) << 10, LARGEST = size_t(1) << 20, PIECE = size_t(256) << 10;
+    constexpr size_t LARGEST = size_t(1) << 20, PIECE = size_t(256) << 10;
     bool direct = bytes > LARGEST;
-    if (!direct && bytes > SMALL) {
+    if (!direct) {
         cudaPointerAttributes at;
-        if (cudaPointerGetAttributes(&at, src) == cudaSuccess) direct = at.type == cudaMemoryTypeHost;
+        if (cudaPointerGetAttributes(&at, src) == cudaSuccess) direct = at.type != cudaMemoryTypeUnregistered;
         else cudaGetLastError();
     }
     if (direct) {

@@ -34,3 +34,22 @@ def test_results_may_be_changed_after_they_were_fed(cuda, rows):
     del y
     first.run({"x": x + 5})  # (takes the memory that was given back)
     assert np.array_equal(second.read("y"), 4 * x)
+
+
+@pytest.mark.parametrize("rows", [1, 8, 9, 200, 300])
+def test_pinned_input_is_read_in_stream_order(cuda, rows):
+    """What the stream writes into pinned memory before a run is what the run is fed, at every size."""
+    import torch
+    from rmlk_b200 import dtypes as dt
+    cols = 1024
+    stream = torch.cuda.Stream()
+    inst = _doubler(cols, stream.cuda_stream)
+    pinned = torch.zeros(rows, cols, pin_memory=True)
+    x = torch.randn(rows, cols, device=cuda)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        torch.cuda._sleep(20_000_000)
+        pinned.copy_(x, non_blocking=True)
+    inst.set_input_ptr("x", dt.F32, [rows, cols], pinned.data_ptr(), False)
+    inst.launch()
+    assert np.array_equal(inst.read("y"), 2 * x.cpu().numpy())
