@@ -1130,7 +1130,10 @@ extern "C" int rmlk_instance_value_info(rmlk_instance* inst, const char* name, i
     if (id < 0) raise(RMLK_ERR_INVALID_ARG, std::string("unknown value `") + name + "`");
     Tensor& t = I.values[id];
     if (!t.present) raise(RMLK_ERR_INVALID_ARG, std::string("value `") + name + "` has no data");
-    if (device_ptr) I.settle_host_only(t);
+    if (device_ptr && t.host_only) {
+        check_cuda(cudaSetDevice(I.device), "cudaSetDevice");  // kernels go to a stream of the current device only
+        I.settle_host_only(t);
+    }
     if (dtype) *dtype = t.dtype;
     if (rank) *rank = static_cast<int>(t.shape.size());
     if (dims)
@@ -1149,6 +1152,7 @@ extern "C" int rmlk_instance_read(rmlk_instance* inst, const char* name, void* d
     const Tensor& t = I.values[id];
     if (!t.present) raise(RMLK_ERR_INVALID_ARG, std::string("value `") + name + "` has no data");
     if (nbytes != t.nbytes()) raise(RMLK_ERR_INVALID_ARG, std::string("read of `") + name + "`: size mismatch");
+    check_cuda(cudaSetDevice(I.device), "cudaSetDevice");  // kernels go to a stream of the current device only
     const void* src = t.data;
     if (t.lazy && nbytes) {
         // a strided view (a cache kept in a buffer with spare room): gather it into a dense staging buffer first

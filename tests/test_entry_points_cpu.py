@@ -1,0 +1,26 @@
+"""Entry points of the runtime, as far as a host without a GPU can look at them."""
+import os
+import re
+
+import rmlk_b200
+
+CSRC = os.path.join(os.path.dirname(rmlk_b200.__file__), "csrc", "runtime", "runtime.cpp")
+
+
+def test_entry_points_that_launch_set_the_device():
+    """A kernel launch on a stream of another device fails; copies there do not, so an entry point that comes to launch one needs its device made
+    current.  (Two devices in one process: what is looked at here is the source.)"""
+    with open(CSRC) as f:
+        source = f.read()
+    bodies = dict(re.findall(r'extern "C" [\w \*]*?(rmlk_instance_\w+)\([^{]*\) \{(.*?)\n\}', source, re.S))
+    assert {"rmlk_instance_read", "rmlk_instance_value_info", "rmlk_instance_set_input", "rmlk_instance_run"} <= set(bodies)
+    launching = re.compile(r"strided_copy|settle_host_only|flush_uploads|read_to_host|feed_host|host_download|host_upload")
+    checked = 0
+    for name, body in bodies.items():
+        at = launching.search(body)
+        if at:
+            checked += 1
+            assert "cudaSetDevice" in body[: at.start()], name
+    assert checked >= 3
+    run = re.search(r"void Instance::run\(\) \{(.*?)\n\}", source, re.S).group(1)
+    assert run.index("cudaSetDevice") < run.index("flush_uploads")
