@@ -12,7 +12,11 @@ def test_entry_points_that_launch_set_the_device():
     current.  (Two devices in one process: what is looked at here is the source.)"""
     with open(CSRC) as f:
         source = f.read()
-    bodies = dict(re.findall(r'extern "C" [\w \*]*?(rmlk_instance_\w+)\([^{]*\) \{(.*?)\n\}', source, re.S))
+    bodies = {}
+    for part in source.split('extern "C" ')[1:]:
+        name = re.match(r"[\w \*]*?(rmlk_instance_\w+)\(", part)
+        if name:
+            bodies[name.group(1)] = part
     assert {"rmlk_instance_read", "rmlk_instance_value_info", "rmlk_instance_set_input", "rmlk_instance_run"} <= set(bodies)
     launching = re.compile(r"strided_copy|settle_host_only|flush_uploads|read_to_host|feed_host|host_download|host_upload")
     checked = 0
