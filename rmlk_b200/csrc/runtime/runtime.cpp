@@ -1116,6 +1116,10 @@ extern "C" int rmlk_instance_run(rmlk_instance* inst) {
 extern "C" int rmlk_instance_synchronize(rmlk_instance* inst) {
     RT_TRY
     if (!inst) raise(RMLK_ERR_INVALID_ARG, "NULL instance");
+    if (!inst->I.uploads.empty()) {
+        check_cuda(cudaSetDevice(inst->I.device), "cudaSetDevice");
+        inst->I.flush_uploads();
+    }
     check_cuda(cudaStreamSynchronize(inst->I.stream), "cudaStreamSynchronize");
     inst->I.check_status();
     return RMLK_OK;
@@ -1130,8 +1134,9 @@ extern "C" int rmlk_instance_value_info(rmlk_instance* inst, const char* name, i
     if (id < 0) raise(RMLK_ERR_INVALID_ARG, std::string("unknown value `") + name + "`");
     Tensor& t = I.values[id];
     if (!t.present) raise(RMLK_ERR_INVALID_ARG, std::string("value `") + name + "` has no data");
-    if (device_ptr && t.host_only) {
+    if (device_ptr && (t.host_only || !I.uploads.empty())) {
         check_cuda(cudaSetDevice(I.device), "cudaSetDevice");  // kernels go to a stream of the current device only
+        I.flush_uploads();                                     // (the address of an input fed since the last run)
         I.settle_host_only(t);
     }
     if (dtype) *dtype = t.dtype;

@@ -53,3 +53,27 @@ def test_pinned_input_is_read_in_stream_order(cuda, rows):
     inst.set_input_ptr("x", dt.F32, [rows, cols], pinned.data_ptr(), False)
     inst.launch()
     assert np.array_equal(inst.read("y"), 2 * x.cpu().numpy())
+
+
+@pytest.mark.parametrize("asked_for", ["value_info", "synchronize"])
+@pytest.mark.parametrize("rows", [1, 200])
+def test_fed_input_is_on_the_device_before_the_run(cuda, asked_for, rows):
+    """The address of an input that has just been fed: its data is there behind synchronize, and behind the stream's work once the address is out."""
+    import torch
+    cols = 1024
+    inst = _doubler(cols)
+    r = np.random.default_rng(rows)
+    inst.run({"x": r.standard_normal((rows, cols), dtype=np.float32)})
+    x = r.standard_normal((rows, cols), dtype=np.float32)
+    ptr = inst.value_info("x")[2]
+    inst.set_input("x", x)
+    if asked_for == "value_info":
+        ptr = inst.value_info("x")[2]
+        torch.cuda.synchronize()
+    else:
+        inst.synchronize()
+
+    class Array:
+        __cuda_array_interface__ = {"version": 3, "data": (ptr, True), "shape": x.shape, "typestr": "<f4", "strides": None}
+
+    assert np.array_equal(torch.as_tensor(Array(), device="cuda").cpu().numpy(), x)
