@@ -637,7 +637,10 @@ void Instance::run() {
         values[i].pairs = false;
         values[i].host_only = false;
     }
-    flush_uploads();
+    {
+        std::lock_guard<std::mutex> lock(io);
+        flush_uploads();
+    }
     parts_owner = -1;
     if (copies_pending) {
         // last run's block-wise copies read buffers that this run is about to hand out again
@@ -1051,6 +1054,7 @@ extern "C" int rmlk_instance_set_input(rmlk_instance* inst, const char* name, in
     for (int i = 0; i < rank; i++)
         if (d.dims[i] != 0 && d.dims[i] != dims[i]) raise(RMLK_ERR_INVALID_ARG, std::string("input `") + name + "`: dimensions mismatch");
     check_cuda(cudaSetDevice(I.device), "cudaSetDevice");
+    std::lock_guard<std::mutex> lock(I.io);
     Tensor& t = I.values[id];
     t = Tensor();
     t.dtype = dtype;
@@ -1116,9 +1120,12 @@ extern "C" int rmlk_instance_run(rmlk_instance* inst) {
 extern "C" int rmlk_instance_synchronize(rmlk_instance* inst) {
     RT_TRY
     if (!inst) raise(RMLK_ERR_INVALID_ARG, "NULL instance");
-    if (!inst->I.uploads.empty()) {
-        check_cuda(cudaSetDevice(inst->I.device), "cudaSetDevice");
-        inst->I.flush_uploads();
+    {
+        std::lock_guard<std::mutex> lock(inst->I.io);
+        if (!inst->I.uploads.empty()) {
+            check_cuda(cudaSetDevice(inst->I.device), "cudaSetDevice");
+            inst->I.flush_uploads();
+        }
     }
     check_cuda(cudaStreamSynchronize(inst->I.stream), "cudaStreamSynchronize");
     inst->I.check_status();
@@ -1130,6 +1137,7 @@ extern "C" int rmlk_instance_value_info(rmlk_instance* inst, const char* name, i
     RT_TRY
     if (!inst || !name) raise(RMLK_ERR_INVALID_ARG, "NULL argument");
     Instance& I = inst->I;
+    std::lock_guard<std::mutex> lock(I.io);
     const int id = I.g.find(name);
     if (id < 0) raise(RMLK_ERR_INVALID_ARG, std::string("unknown value `") + name + "`");
     Tensor& t = I.values[id];
@@ -1152,6 +1160,7 @@ extern "C" int rmlk_instance_read(rmlk_instance* inst, const char* name, void* d
     RT_TRY
     if (!inst || !name) raise(RMLK_ERR_INVALID_ARG, "NULL argument");
     Instance& I = inst->I;
+    std::lock_guard<std::mutex> lock(I.io);
     const int id = I.g.find(name);
     if (id < 0) raise(RMLK_ERR_INVALID_ARG, std::string("unknown value `") + name + "`");
     const Tensor& t = I.values[id];

@@ -7,6 +7,7 @@
 
 #include <map>
 #include <memory>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 #include <unordered_map>
@@ -284,6 +285,8 @@ struct Instance {
     size_t up_used = 0;              // bytes of the staging area that uploads not known to be finished occupy
     cudaEvent_t up_done = nullptr;   // behind the last upload
     uint32_t down_seq = 0;
+    // Held while the staging areas and the list of uploads are used: several threads may feed and read one instance.
+    std::mutex io;
     void feed_host(void* dst, const void* src, size_t bytes);
     void flush_uploads();
     void read_to_host(void* dst, const void* src, size_t bytes);

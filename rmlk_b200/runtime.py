@@ -17,6 +17,7 @@ from __future__ import annotations
 
 import ctypes
 import enum
+import threading
 from typing import Dict, Optional, Sequence
 
 import numpy as np
@@ -237,6 +238,19 @@ class GraphBuilder:
         return self
 
 
+_per_thread = threading.local()
+
+
+def _info():
+    """What rmlk_instance_value_info writes to, and the references to it: made once per thread (ctypes lets other threads run during a call)."""
+    try:
+        return _per_thread.info
+    except AttributeError:
+        vals = (ctypes.c_int(), ctypes.c_int(), (ctypes.c_int64 * 8)(), ctypes.c_void_p())
+        _per_thread.info = vals, tuple(ctypes.byref(x) if i != 2 else x for i, x in enumerate(vals))
+        return _per_thread.info
+
+
 class ModelInstance:
     """Builder::from_graph(graph).build() + ModelInstance (runtime/src/core/instance.rs:89-221)."""
 
@@ -249,8 +263,6 @@ class ModelInstance:
         self._keep = []
         self._l = _rt()
         self._names = {}           # name -> encoded, for the names used so far
-        self._info = (ctypes.c_int(), ctypes.c_int(), (ctypes.c_int64 * 8)(), ctypes.c_void_p())
-        self._info_refs = tuple(ctypes.byref(x) if i != 2 else x for i, x in enumerate(self._info))
 
     def _key(self, name: str) -> bytes:
         k = self._names.get(name)
@@ -296,15 +308,15 @@ class ModelInstance:
         _check(_rt().rmlk_instance_synchronize(self._h))
 
     def value_info(self, name: str):
-        d, r, dims, p = self._info
-        _check(self._l.rmlk_instance_value_info(self._h, self._key(name), *self._info_refs))
+        (d, r, dims, p), refs = _info()
+        _check(self._l.rmlk_instance_value_info(self._h, self._key(name), *refs))
         return d.value, dims[: r.value], p.value or 0
 
     def read(self, name: str) -> np.ndarray:
-        d, r, dims, _ = self._info
+        (d, r, dims, _), refs = _info()
         key = self._key(name)
         # (no device address: asking for one would give a value that only the host knows device memory)
-        _check(self._l.rmlk_instance_value_info(self._h, key, self._info_refs[0], self._info_refs[1], dims, None))
+        _check(self._l.rmlk_instance_value_info(self._h, key, refs[0], refs[1], dims, None))
         out = np.empty(dims[: r.value], dtype=dt.to_numpy(d.value))  # pageable: a caller may change or drop it at once after feeding it on
         _check(self._l.rmlk_instance_read(self._h, key, out.__array_interface__["data"][0], out.nbytes))
         return out

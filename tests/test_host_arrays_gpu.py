@@ -77,3 +77,26 @@ def test_fed_input_is_on_the_device_before_the_run(cuda, asked_for, rows):
         __cuda_array_interface__ = {"version": 3, "data": (ptr, True), "shape": x.shape, "typestr": "<f4", "strides": None}
 
     assert np.array_equal(torch.as_tensor(Array(), device="cuda").cpu().numpy(), x)
+
+
+def test_threads_read_one_instance(cuda):
+    """Two threads read outputs of different shapes, types and sizes of one instance at the same time."""
+    from concurrent.futures import ThreadPoolExecutor
+    from rmlk_b200.runtime import ModelInstance
+    g = GraphSpec()
+    g.input("x", np.float32, [0, 1024])
+    g.input("n", np.int64, [0])
+    g.op("Add", ["x", "x"], "y")
+    g.op("Add", ["n", "n"], "m")
+    g.output("y")
+    g.output("m")
+    inst = ModelInstance(g.to_runtime())
+    x, n = np.random.default_rng(1).standard_normal((150, 1024), dtype=np.float32), np.arange(3000, dtype=np.int64)
+    inst.run({"x": x, "n": n})
+
+    def reads(name, want):
+        return all((lambda got: got.dtype == want.dtype and np.array_equal(got, want))(inst.read(name)) for _ in range(300))
+
+    with ThreadPoolExecutor(4) as pool:
+        jobs = [pool.submit(reads, *a) for a in (("y", 2 * x), ("m", 2 * n), ("y", 2 * x), ("m", 2 * n))]
+        assert all(j.result() for j in jobs)
