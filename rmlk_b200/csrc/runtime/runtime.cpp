@@ -1179,9 +1179,10 @@ extern "C" int rmlk_instance_read(rmlk_instance* inst, const char* name, void* d
     if (t.host_only) {
         for (int64_t i = 0; i < t.numel(); i++)
             std::memcpy(static_cast<char*>(dst) + i * dtype_size_of(t.dtype), &t.mi[i], dtype_size_of(t.dtype));
-        return RMLK_OK;
+        check_cuda(cudaStreamSynchronize(I.stream), "cudaStreamSynchronize");  // a read waits for the run and reports its errors
+    } else {
+        I.read_to_host(dst, src, nbytes);
     }
-    I.read_to_host(dst, src, nbytes);
     I.check_status();
     return RMLK_OK;
     RT_CATCH

@@ -100,3 +100,26 @@ def test_threads_read_one_instance(cuda):
     with ThreadPoolExecutor(4) as pool:
         jobs = [pool.submit(reads, *a) for a in (("y", 2 * x), ("m", 2 * n), ("y", 2 * x), ("m", 2 * n))]
         assert all(j.result() for j in jobs)
+
+
+def test_reading_a_shape_reports_the_errors_of_the_run(cuda):
+    from rmlk_b200.runtime import InferenceError, ModelInstance
+    g = GraphSpec()
+    g.input("data", np.float32, [0, 4])
+    g.input("at", np.int64, [0])
+    g.op("Gather", ["data", "at"], "y", axis=0)
+    g.op("Shape", ["y"], "shape")
+    g.op("Reshape", ["y", "shape"], "z")
+    g.output("z")
+    inst = ModelInstance(g.to_runtime())
+    at = np.zeros(100, np.int64)
+    for name, value in (("data", np.zeros((8, 4), np.float32)), ("at", at)):
+        inst.set_input(name, value)
+    inst.launch()
+    assert inst.read("shape").tolist() == [100, 4]
+    at[70] = 9  # out of range: seen by the kernel, which writes nothing there
+    for name, value in (("data", np.zeros((8, 4), np.float32)), ("at", at)):
+        inst.set_input(name, value)
+    inst.launch()
+    with pytest.raises(InferenceError):
+        inst.read("shape")
