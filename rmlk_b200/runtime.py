@@ -106,7 +106,10 @@ _DIMS = [ctypes.c_int64 * max(n, 1) for n in range(9)]  # array types, made once
 
 def _i64(vals: Sequence[int]):
     n = len(vals)
-    return (_DIMS[n] if n < 9 else ctypes.c_int64 * n)(*vals)
+    try:
+        return (_DIMS[n] if n < 9 else ctypes.c_int64 * n)(*vals)
+    except TypeError:  # numpy integers and the like
+        return (ctypes.c_int64 * max(n, 1))(*[int(v) for v in vals])
 
 
 _NP_CODES = {np.dtype(dt.to_numpy(c)): c for c in dt.NAMES}  # dtype object -> code

@@ -28,3 +28,12 @@ def test_entry_points_that_launch_set_the_device():
     assert checked >= 3
     run = re.search(r"void Instance::run\(\) \{(.*?)\n\}", source, re.S).group(1)
     assert run.index("cudaSetDevice") < run.index("flush_uploads")
+
+
+def test_dims_of_any_integer_type():
+    import numpy as np
+    import torch
+    from rmlk_b200 import kernels, runtime
+    for make in (runtime._i64, kernels._i64):
+        for dims in ([], [3], (2, 5), list(range(12)), np.arange(4), [np.int32(7), 2], torch.Size([4, 6]), [torch.tensor(9), 1], [True, 2.0]):
+            assert list(make(dims))[: len(dims)] == [int(v) for v in dims]
