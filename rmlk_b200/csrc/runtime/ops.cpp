@@ -2207,7 +2207,18 @@ bool Instance::run_fused(const FusedGroup& fg) {
             const Shape sshape = {B, H, S, T};
             if (mk->shape.size() > 4 || mk->shape.empty() || mk->shape.back() != T || !bcast_strides(*mk, sshape, ms) || (T > 1 && ms[3] != 1)) return false;
             if (q->lazy) materialize(*q);
-            const void *kdata = kt->data, *vdata = vh->data;
+            const void *kdata = kt->data, *vdata = vh->data, *qdata = q->data;
+            struct Copy {
+                Arena& arena;
+                Storage* s = nullptr;
+                ~Copy() { arena.release(s); }
+            } copy{*arena};
+            if (reinterpret_cast<uintptr_t>(qdata) % 16) {  // a caller's buffer, used in place: the kernels read 16 bytes at a time
+                copy.s = arena->alloc(q->nbytes());
+                check_cuda(cudaMemcpyAsync(copy.s->ptr, qdata, q->nbytes(), cudaMemcpyDeviceToDevice, stream), "attention queries");
+                launches++;
+                qdata = copy.s->ptr;
+            }
             if (S != 1) {
                 const int ov = root.outputs[0];
                 const Shape oshape = {B, H, S, D};
@@ -2220,14 +2231,14 @@ bool Instance::run_fused(const FusedGroup& fg) {
                     set_strided(o, o.data, oshape, ost);
                     o.storage = keep;
                 }
-                check_rc(rmlk_b200_gqa_prefill_attention(st, RMLK_F32, lk.outer, lk.fold, S, D, T, H / lk.fold, q->data, kdata, lk.sb, vdata, lv.sb, scale, mk->data, ms,
+                check_rc(rmlk_b200_gqa_prefill_attention(st, RMLK_F32, lk.outer, lk.fold, S, D, T, H / lk.fold, qdata, kdata, lk.sb, vdata, lv.sb, scale, mk->data, ms,
                                                          o.data, ost.data(), status_ptr()));
                 status_dirty = true;
                 launches++;
                 return true;
             }
             if (!attention_split && (lk.fold * D) % 64 == 0 && pairs_wanted(root.outputs[0], B, H * D, true)) {
-                const float* qd = static_cast<const float*>(q->data);
+                const float* qd = static_cast<const float*>(qdata);
                 Tensor& o = make_pairs(root.outputs[0], Shape({B, H, 1, D}), B, H * D, static_cast<int>(lk.fold * D / 64));
                 check_rc(gqa_decode_attention_pairs(stream, lk.outer, lk.fold, D, T, H / lk.fold, qd, static_cast<const float*>(kdata), lk.sb,
                                                     static_cast<const float*>(vdata), lv.sb, scale, static_cast<const float*>(mk->data), ms[0], ms[1], o.split));
@@ -2253,7 +2264,7 @@ bool Instance::run_fused(const FusedGroup& fg) {
                 }
                 attn_ws_problems = lk.outer;
             }
-            check_rc(rmlk_b200_gqa_decode_attention_ws(st, RMLK_F32, lk.outer, lk.fold, D, T, H / lk.fold, q->data, kdata, lk.sb, vdata, lv.sb, scale,
+            check_rc(rmlk_b200_gqa_decode_attention_ws(st, RMLK_F32, lk.outer, lk.fold, D, T, H / lk.fold, qdata, kdata, lk.sb, vdata, lv.sb, scale,
                                                        mk->data, ms[0], ms[1], o.data, ws, ws_need));
             launches++;
             return true;
