@@ -21,13 +21,9 @@ def cuda():
     return torch.device("cuda:0")
 
 
-@pytest.hookimpl(wrapper=True)
-def pytest_runtest_call(item):
+@pytest.fixture(autouse=True)
+def _without_reference_kernels(monkeypatch):
     """The bit oracle is built from the reference's kernel sources; where they were not there to build it from, a test that asks for it is skipped."""
     from oracle import ref_cpu
-    try:
-        return (yield)
-    except OSError:
-        if ref_cpu.available():
-            raise
-        pytest.skip("reference kernels not built (oracle/Makefile)")
+    if not ref_cpu.available():
+        monkeypatch.setattr(ref_cpu, "lib", lambda: pytest.skip("reference kernels not built (oracle/Makefile)"))
