@@ -74,7 +74,7 @@ def test_fed_input_is_on_the_device_before_the_run(cuda, asked_for, rows):
         inst.synchronize()
 
     class Array:
-        __cuda_array_interface__ = {"version": 3, "data": (ptr, True), "shape": x.shape, "typestr": "<f4", "strides": None}
+        __cuda_array_interface__ = {"version": 3, "data": (ptr, False), "shape": x.shape, "typestr": "<f4", "strides": None}
 
     assert np.array_equal(torch.as_tensor(Array(), device="cuda").cpu().numpy(), x)
 
