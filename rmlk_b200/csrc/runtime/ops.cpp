@@ -2010,6 +2010,17 @@ static rmlk_batch_job rope_job(const Shape& oshape, const int64_t* xstr, const i
     return j;
 }
 
+// Several tokens: the one-launch kernel or the single operators.  The kernel gives a CTA 128 query rows of a KV head (`rows` in all) and walks its
+// keys 64 at a time, 5 us each, however few CTAs there are; the single operators use every SM, and up to 16 rows they stream the
+// keys.  Measured on 2 to 32 KV heads, 1 to 16 requests, 2 to 192 tokens behind 64 to 8192 keys of 64, kernel against single operators: 8 KV heads of 4
+// query heads, 2 tokens, 4096 keys 359 against 55 us; 16 tokens, 2048 keys 189 / 136; 16 requests of 16 tokens, 2048 keys 222 / 557; one prompt of
+// 256 tokens 112 / 150.  With the line below 15 of some 2400 sizes are slower than the single operators by more than 5 % (worst 331 / 229), and the
+// sizes left to these cost 2 % on average.
+static bool prompt_attention_pays(int64_t problems, int64_t rows, int64_t keys) {
+    const int64_t all = problems * rows;
+    return rows > 16 && (keys <= 128 || all >= 4096 || all * keys > (int64_t(1) << 22));
+}
+
 bool Instance::run_fused(const FusedGroup& fg) {
     const NodeDef& root = g.nodes[fg.root];
     Ctx c{*this, root};
@@ -2200,6 +2211,7 @@ bool Instance::run_fused(const FusedGroup& fg) {
             if (!analyze_lazy_b(*kt, D, T, lk) || !lk.transposed || !analyze_lazy_b(*vh, T, D, lv) || lv.transposed) return false;
             if (lk.fold != lv.fold || lk.outer != lv.outer || lk.outer * lk.fold != B * H || H % lk.fold) return false;
             if (S == 1 ? !rmlk_b200_gqa_decode_attention_supported(lk.fold, D, T) : !rmlk_b200_gqa_prefill_attention_supported(S, lk.fold, D, T)) return false;
+            if (S > 1 && !prompt_attention_pays(lk.outer, lk.fold * S, T)) return false;
             if (lk.outer > 1 && (lk.sb % 4 || lv.sb % 4)) return false;
             if (reinterpret_cast<uintptr_t>(kt->data) % 16 || reinterpret_cast<uintptr_t>(vh->data) % 16) return false;
             if (mk->lazy) materialize(*mk);

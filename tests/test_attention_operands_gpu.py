@@ -70,3 +70,30 @@ def test_queries_off_16_byte_boundaries(cuda, B, S, project):
     name = "y" if project else "ctx"
     got, want = inst.read(name), graph_cpu.run_graph(g, feeds)[name]
     assert np.max(np.abs(got - want)) <= 1e-4 * np.max(np.abs(want))
+
+
+# requests, new tokens, keys in the cache, one launch: few rows behind a long cache are shared out over the GPU by the single operators
+@pytest.mark.parametrize("B,S,T,one", [(1, 2, 600, False), (1, 16, 2000, False), (4, 4, 64, False), (1, 30, 90, True), (2, 64, 64, True), (8, 100, 30, True),
+                                       (8, 33, 1100, True)])
+def test_tokens_behind_a_cache(cuda, B, S, T, one):
+    import os
+    from rmlk_b200.runtime import ModelInstance
+    KV, G, D = 8, 4, 64
+    g = attention_graph(KV, G, D)
+    fused = ModelInstance(g.to_runtime())
+    os.environ["RMLK_B200_ATTENTION"] = "0"
+    try:
+        single = ModelInstance(g.to_runtime())
+    finally:
+        del os.environ["RMLK_B200_ATTENTION"]
+    r = np.random.default_rng(S)
+    feeds = {"q": r.standard_normal((B, KV * G, S, D), dtype=np.float32), "new_k": r.standard_normal((B, KV, S, D), dtype=np.float32),
+             "new_v": r.standard_normal((B, KV, S, D), dtype=np.float32), "past_k": r.standard_normal((B, KV, T, D), dtype=np.float32),
+             "past_v": r.standard_normal((B, KV, T, D), dtype=np.float32), "mask": np.zeros((B, 1, S, T + S), np.float32)}
+    outs = []
+    for inst in (fused, single):
+        inst.bind("present_k", "past_k")
+        inst.bind("present_v", "past_v")
+        outs.append(inst.run(feeds)["ctx"])
+    assert np.max(np.abs(outs[0] - outs[1])) <= 1e-5 * np.max(np.abs(outs[1]))
+    assert (fused.last_launches < single.last_launches) == one
