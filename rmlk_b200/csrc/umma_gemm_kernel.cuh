@@ -264,9 +264,8 @@ __global__ void __launch_bounds__(Layout<CG, SPLIT, MT, ST>::THREADS, 1) gemm_ke
                 if constexpr (SPLIT) {
                     if (4 * lane < HM) s4 = __ldg(reinterpret_cast<const float4*>(p.x_scale + c * p.x_scale_pitch + m_base) + lane);
                 }
-                ok = mbar_wait(acc_full(buf), acc_phase, abort_flag, p.status);
+                ok = __all_sync(0xffffffffu, mbar_wait(acc_full(buf), acc_phase, abort_flag, p.status));  // (one lane's limit may run out before another's)
                 if (!ok) break;
-                __syncwarp();
                 tc_fence_after();
                 const uint32_t d = tmem + lane_field + buf * L::D_COLS + part * HM;
                 if constexpr (!SPLIT || ONE_CHUNK) {
