@@ -671,27 +671,37 @@ __global__ void __launch_bounds__(FL_THREADS, LPR <= 16 ? 4 : 2) gqa_decode_flas
     }
     if (rank == 0) {
         const bool bad = *s_bad != 0;
-        uint32_t top = 0;
+        uint32_t top = 0, low = 0xffffffffu;
 #pragma unroll
         for (int q = 0; q < PER; q++) {
             const int i = threadIdx.x + q * FL_THREADS;
             A[q] = bad ? __int_as_float(0x7fc00000) : A[q] / Ls[q];
             if (i >= p.rows * D) continue;
-            if constexpr (PAIRS) top = max(top, finite_abs_bits(A[q]));
-            else p.out[prob * p.rows * D + i] = A[q];
+            if constexpr (PAIRS) {
+                top = max(top, finite_abs_bits(A[q]));
+                low = min(low, nonzero_low(A[q]));
+            } else p.out[prob * p.rows * D + i] = A[q];
         }
         if constexpr (PAIRS) {
             uint32_t* s_top = reinterpret_cast<uint32_t*>(s_m);  // every thread has read the statistics
             __syncthreads();
-            if (threadIdx.x == 0) *s_top = 0;
+            if (threadIdx.x == 0) {
+                s_top[0] = 0;
+                s_top[1] = 0xffffffffu;
+            }
             __syncthreads();
             top = __reduce_max_sync(0xffffffffu, top);
-            if (lane == 0) atomicMax(s_top, top);
+            low = __reduce_min_sync(0xffffffffu, low);
+            if (lane == 0) {
+                atomicMax(s_top, top);
+                atomicMin(s_top + 1, low);
+            }
             __syncthreads();
-            const int e = scale_exponent(*s_top);
+            const int e = scale_exponent(s_top[0]);
+            const bool hold = pairs_hold(s_top[0], s_top[1]);
             const float up = exp2_int(e);
             const int64_t b = prob / p.kv_heads, h = prob % p.kv_heads;
-            if (threadIdx.x == 0) p.pairs.scale[h * p.pairs.scale_pitch + b] = exp2_int(-e);
+            if (threadIdx.x == 0) p.pairs.scale[h * p.pairs.scale_pitch + b] = hold ? exp2_int(-e) : -exp2_int(-e);
             __half* o = static_cast<__half*>(p.pairs.data) + b * p.pairs.k_pad + h * p.rows * D;
 #pragma unroll
             for (int q = 0; q < PER; q++) {
@@ -701,6 +711,7 @@ __global__ void __launch_bounds__(FL_THREADS, LPR <= 16 ? 4 : 2) gqa_decode_flas
                 const __half hi = __float2half_rn(x);
                 o[i] = hi;
                 o[p.pairs.m_pad * p.pairs.k_pad + i] = __float2half_rn((x - __half2float(hi)) * SPLIT_LO);
+                if (!hold) p.pairs.full[b * p.pairs.full_ld + h * p.rows * D + i] = A[q];
             }
         }
     }

@@ -86,11 +86,41 @@ __global__ void __launch_bounds__(256) rmsnorm_f32_kernel(int64_t cols, float ex
     for (int64_t c = threadIdx.x; c < cols; c += 256) dst[c] = __fmul_rn(__fdiv_rn(row[c], sd), w[c]);
 }
 
-// Same, for rows of up to THREADS * 4 * NP elements with 16-byte alignment: the row is read once and held in registers.
+// Range of a row's magnitudes, as bits: of all values (an infinity or NaN shows in the largest, a zero in the smallest), and as pairs_hold takes it
+__device__ __forceinline__ void magnitude_range(float4 x, uint32_t& mx, uint32_t& mn) {
+    const uint32_t a = __float_as_uint(x.x) & 0x7fffffffu, b = __float_as_uint(x.y) & 0x7fffffffu, c = __float_as_uint(x.z) & 0x7fffffffu, d = __float_as_uint(x.w) & 0x7fffffffu;
+    mx = max(max(mx, max(a, b)), max(c, d));
+    mn = min(min(mn, min(a, b)), min(c, d));
+}
+__device__ __forceinline__ void plain_range(float4 x, uint32_t& mx, uint32_t& low) {
+    mx = max(max(mx, max(finite_abs_bits(x.x), finite_abs_bits(x.y))), max(finite_abs_bits(x.z), finite_abs_bits(x.w)));
+    low = min(min(low, min(nonzero_low(x.x), nonzero_low(x.y))), min(nonzero_low(x.z), nonzero_low(x.w)));
+}
+// over the CTA; a barrier lies between the two
+__device__ __forceinline__ void put_range(uint32_t mx, uint32_t mn, uint32_t* part_max, uint32_t* part_min) {
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    mn = __reduce_min_sync(0xffffffffu, mn);
+    if ((threadIdx.x & 31) == 0) {
+        part_max[threadIdx.x >> 5] = mx;
+        part_min[threadIdx.x >> 5] = mn;
+    }
+}
+template <int THREADS>
+__device__ __forceinline__ void get_range(uint32_t& mx, uint32_t& mn, const uint32_t* part_max, const uint32_t* part_min) {
+    mx = part_max[0];
+    mn = part_min[0];
+#pragma unroll
+    for (int i = 1; i < THREADS / 32; i++) {
+        mx = max(mx, part_max[i]);
+        mn = min(mn, part_min[i]);
+    }
+}
+
+// Same as above, for rows of up to THREADS * 4 * NP elements with 16-byte alignment: the row is read once and held in registers.
 // A few rows (a decode step: 64) take 512 or 1024 threads with one pack each, so that the row, the residual and all
 // split-K slabs of a pack are requested at once - one trip to memory instead of several; many rows take 256 threads.
-// PAIRS: the normalised row goes out as pairs of f16 for the tensor-core MatMul that reads it (its scale from the largest
-// |x w| / sd, found in the same pass as the sum) instead of as fp32.
+// PAIRS: the normalised row goes out as pairs of f16 for the tensor-core MatMul that reads it (its range from the largest and smallest
+// |x w|, found in the same pass as the sum) instead of as fp32; as fp32 too if pairs do not hold it.
 template <int NP, int THREADS, bool PAIRS>
 __global__ void __launch_bounds__(THREADS) rmsnorm_f32_regs_kernel(int cols, float exponent, float eps, const float* __restrict__ x,
                                                                   const float* __restrict__ w, float* __restrict__ out, SplitRows pairs, RowAdd ra) {
@@ -99,13 +129,13 @@ __global__ void __launch_bounds__(THREADS) rmsnorm_f32_regs_kernel(int cols, flo
     const int packs = cols / 4;
     dep_wait();
     __shared__ double part[THREADS / 32];
-    __shared__ uint32_t part_max[THREADS / 32];
+    __shared__ uint32_t part_max[THREADS / 32], part_min[THREADS / 32];
     const int64_t r0 = static_cast<int64_t>(blockIdx.x) * cols;
     const float4* row = reinterpret_cast<const float4*>(x + r0);
     float4* dst = reinterpret_cast<float4*>(out + r0);
     float4 v[NP];
     double acc = 0.0;
-    uint32_t mx = 0;
+    uint32_t mx = 0, mn = 0xffffffffu;  // bits of the largest and smallest |x w|
     const bool square = exponent == 2.0f;  // powf(v, 2) is v * v rounded once; the product is a tenth of the instructions
 #pragma unroll
     for (int i = 0; i < NP; i++) {
@@ -150,17 +180,13 @@ __global__ void __launch_bounds__(THREADS) rmsnorm_f32_regs_kernel(int cols, flo
             }
             if constexpr (PAIRS) {
                 const float4 g = wv[c];
-                mx = max(max(mx, max(finite_abs_bits(v[i].x * g.x), finite_abs_bits(v[i].y * g.y))),
-                         max(finite_abs_bits(v[i].z * g.z), finite_abs_bits(v[i].w * g.w)));
+                magnitude_range(make_float4(v[i].x * g.x, v[i].y * g.y, v[i].z * g.z, v[i].w * g.w), mx, mn);
             }
         }
     }
     acc = warp_sum_d(acc);
-    if constexpr (PAIRS) mx = __reduce_max_sync(0xffffffffu, mx);
-    if ((threadIdx.x & 31) == 0) {
-        part[threadIdx.x >> 5] = acc;
-        if constexpr (PAIRS) part_max[threadIdx.x >> 5] = mx;
-    }
+    if constexpr (PAIRS) put_range(mx, mn, part_max, part_min);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
     __syncthreads();
     double total = 0.0;
 #pragma unroll
@@ -168,13 +194,34 @@ __global__ void __launch_bounds__(THREADS) rmsnorm_f32_regs_kernel(int cols, flo
     const float mean = static_cast<float>(total / static_cast<double>(cols));
     const float sd = sqrtf(__fadd_rn(mean, eps));
     float scale = 1.f;
+    bool hold = true;
     if constexpr (PAIRS) {
-        uint32_t top = 0;
+        get_range<THREADS>(mx, mn, part_max, part_min);
+        uint32_t top = finite_abs_bits(__fdiv_rn(__uint_as_float(mx), sd)), low = mn - 1u;
+        if (mx >= 0x7f800000u || mn == 0 || mx < 0x12800000u) {
+            // infinities, NaNs or zeros among the products, or all of them below 2^-90: x w may have left the range of fp32 where (x / sd) w has
+            // not, so the values themselves are looked at
+            __syncthreads();
+            mx = 0;
+            low = 0xffffffffu;
 #pragma unroll
-        for (int i = 0; i < THREADS / 32; i++) top = max(top, part_max[i]);
-        const int e = scale_exponent(finite_abs_bits(__fdiv_rn(__uint_as_float(top), sd)));
+            for (int i = 0; i < NP; i++) {
+                const int c = threadIdx.x + THREADS * i;
+                if (c < packs) {
+                    const float4 g = wv[c];
+                    plain_range(make_float4(__fmul_rn(__fdiv_rn(v[i].x, sd), g.x), __fmul_rn(__fdiv_rn(v[i].y, sd), g.y), __fmul_rn(__fdiv_rn(v[i].z, sd), g.z),
+                                            __fmul_rn(__fdiv_rn(v[i].w, sd), g.w)), mx, low);
+                }
+            }
+            put_range(mx, low, part_max, part_min);
+            __syncthreads();
+            get_range<THREADS>(mx, low, part_max, part_min);
+            top = mx;
+        }
+        hold = pairs_hold(mx, low);
+        const int e = scale_exponent(top);
         scale = exp2_int(e);
-        if (threadIdx.x == 0) pairs.scale[blockIdx.x] = exp2_int(-e);
+        if (threadIdx.x == 0) pairs.scale[blockIdx.x] = hold ? exp2_int(-e) : -exp2_int(-e);
     }
 #pragma unroll
     for (int i = 0; i < NP; i++) {
@@ -186,8 +233,12 @@ __global__ void __launch_bounds__(THREADS) rmsnorm_f32_regs_kernel(int cols, flo
             r.y = __fmul_rn(__fdiv_rn(v[i].y, sd), g.y);
             r.z = __fmul_rn(__fdiv_rn(v[i].z, sd), g.z);
             r.w = __fmul_rn(__fdiv_rn(v[i].w, sd), g.w);
-            if constexpr (PAIRS) store_pairs4(pairs, blockIdx.x, 4 * c, r, scale);
-            else dst[c] = r;
+            if constexpr (PAIRS) {
+                store_pairs4(pairs, blockIdx.x, 4 * c, r, scale);
+                if (!hold) store_full4(pairs, blockIdx.x, 4 * c, r);
+            } else {
+                dst[c] = r;
+            }
         }
     }
 }
@@ -441,7 +492,7 @@ __global__ void __launch_bounds__(128) swiglu_slabs_kernel(int64_t rows, int64_t
 template <int NP, int THREADS>
 __global__ void __launch_bounds__(THREADS) swiglu_pairs_kernel(int cols, const float* __restrict__ g, int64_t ldg, const float* __restrict__ u, int64_t ldu, SplitRows pairs) {
     dep_sync();
-    __shared__ uint32_t part_max[THREADS / 32];
+    __shared__ uint32_t part_max[THREADS / 32], part_min[THREADS / 32];
     const int64_t row = blockIdx.x;
     const float4* gr = reinterpret_cast<const float4*>(g + row * ldg);
     const float4* ur = reinterpret_cast<const float4*>(u + row * ldu);
@@ -455,7 +506,7 @@ __global__ void __launch_bounds__(THREADS) swiglu_pairs_kernel(int cols, const f
             b[i] = ur[c];
         }
     }
-    uint32_t mx = 0;
+    uint32_t mx = 0, mn = 0xffffffffu;
 #pragma unroll
     for (int i = 0; i < NP; i++) {
         if (threadIdx.x + THREADS * i < packs) {
@@ -464,22 +515,35 @@ __global__ void __launch_bounds__(THREADS) swiglu_pairs_kernel(int cols, const f
             r.y = __fmul_rn(__fmul_rn(r.y, 1.0f / (1.0f + expf(-r.y))), b[i].y);
             r.z = __fmul_rn(__fmul_rn(r.z, 1.0f / (1.0f + expf(-r.z))), b[i].z);
             r.w = __fmul_rn(__fmul_rn(r.w, 1.0f / (1.0f + expf(-r.w))), b[i].w);
-            mx = max(max(mx, max(finite_abs_bits(r.x), finite_abs_bits(r.y))), max(finite_abs_bits(r.z), finite_abs_bits(r.w)));
+            magnitude_range(r, mx, mn);
         }
     }
-    mx = __reduce_max_sync(0xffffffffu, mx);
-    if ((threadIdx.x & 31) == 0) part_max[threadIdx.x >> 5] = mx;
+    put_range(mx, mn, part_max, part_min);
     __syncthreads();
-    uint32_t top = 0;
+    get_range<THREADS>(mx, mn, part_max, part_min);
+    uint32_t low = mn - 1u;
+    if (mx >= 0x7f800000u || mn == 0) {  // infinities, NaNs and zeros are left out of the range
+        __syncthreads();
+        mx = 0;
+        low = 0xffffffffu;
 #pragma unroll
-    for (int i = 0; i < THREADS / 32; i++) top = max(top, part_max[i]);
-    const int e = scale_exponent(top);
+        for (int i = 0; i < NP; i++)
+            if (threadIdx.x + THREADS * i < packs) plain_range(a[i], mx, low);
+        put_range(mx, low, part_max, part_min);
+        __syncthreads();
+        get_range<THREADS>(mx, low, part_max, part_min);
+    }
+    const int e = scale_exponent(mx);
     const float scale = exp2_int(e);
-    if (threadIdx.x == 0) pairs.scale[row] = exp2_int(-e);
+    const bool hold = pairs_hold(mx, low);
+    if (threadIdx.x == 0) pairs.scale[row] = hold ? exp2_int(-e) : -exp2_int(-e);
 #pragma unroll
     for (int i = 0; i < NP; i++) {
         const int c = threadIdx.x + THREADS * i;
-        if (c < packs) store_pairs4(pairs, row, 4 * c, a[i], scale);
+        if (c < packs) {
+            store_pairs4(pairs, row, 4 * c, a[i], scale);
+            if (!hold) store_full4(pairs, row, 4 * c, a[i]);
+        }
     }
 }
 

@@ -825,7 +825,7 @@ static bool split_pays(int64_t m, int64_t n, int64_t k) {
 static size_t round1k(size_t v) { return (v + 1023) & ~static_cast<size_t>(1023); }
 static size_t split_workspace(int64_t m, int64_t n, int64_t k) {
     const int parts = std::max(umma_split_parts(m, n, k, false), umma_split_parts(m, n, k, true));
-    return 1024 + round1k(split_weights_bytes(n, k)) + round1k(split_rows_bytes(m, k, 0)) + (parts > 1 ? static_cast<size_t>(parts) * m * n * sizeof(float) : 0);
+    return 1024 + round1k(split_weights_bytes(n, k)) + round1k(split_rows_bytes(m, k, 0, false)) + (parts > 1 ? static_cast<size_t>(parts) * m * n * sizeof(float) : 0);
 }
 
 // Least scratch of a shape (what the kernels without a splitting pass need)
@@ -980,10 +980,10 @@ extern "C" int rmlk_b200_matmul_flags(rmlk_stream_t stream, int dtype, int64_t b
     const bool b_rows_aligned = (n % 4 == 0) && aligned_to(b, 16) && (b_batch_stride % 4 == 0);
     if (batch == 1 && split_pays(m, n, k) && workspace && workspace_bytes >= split_workspace(m, n, k)) {
         char* ws = reinterpret_cast<char*>(round1k(reinterpret_cast<uintptr_t>(workspace)));
-        const SplitWeights w = split_weights_at(ws, n, k);
+        SplitWeights w = split_weights_at(ws, n, k);
         ws += round1k(split_weights_bytes(n, k));
-        const SplitRows x = split_rows_at(ws, m, k, 0);
-        ws += round1k(split_rows_bytes(m, k, 0));
+        SplitRows x = split_rows_at(ws, m, k, 0, false);
+        ws += round1k(split_rows_bytes(m, k, 0, false));
         WeightSources src = {};
         src.count = 1;
         src.w[0] = static_cast<const float*>(b);

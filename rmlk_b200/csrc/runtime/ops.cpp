@@ -2709,9 +2709,9 @@ Tensor& Instance::make_pairs(int value_id, const std::vector<int64_t>& shape, in
     o = Tensor();
     o.dtype = RMLK_F32;
     o.shape = shape;
-    o.storage = arena->alloc(split_rows_bytes(rows, k, chunk_blocks));
+    o.storage = arena->alloc(split_rows_bytes(rows, k, chunk_blocks, true));
     o.data = o.storage->ptr;
-    o.split = split_rows_at(o.data, rows, k, chunk_blocks);
+    o.split = split_rows_at(o.data, rows, k, chunk_blocks, true);
     o.pairs = true;
     o.present = true;
     return o;
@@ -2723,7 +2723,7 @@ SplitRows Instance::split_left_operand(const Tensor& t, int64_t rows, int64_t k)
         return t.split;
     }
     const float* a = static_cast<const float*>(t.data);
-    const SplitRows x = split_rows_at(x_split.ensure(split_rows_bytes(rows, k, 0)), rows, k, 0);
+    SplitRows x = split_rows_at(x_split.ensure(split_rows_bytes(rows, k, 0, false)), rows, k, 0, false);
     check_rc(split_rows_pack(stream, a, k, x));
     launches++;
     return x;

@@ -19,6 +19,15 @@ __device__ __forceinline__ int scale_exponent(uint32_t max_bits) {
 }
 __device__ __forceinline__ float exp2_int(int e) { return __int_as_float((e + 127) << 23); }
 
+// Low end of a group's range: the smallest of `nonzero_low` over its values is the bits of the smallest magnitude that is not zero, less one.
+__device__ __forceinline__ uint32_t nonzero_low(float x) { return (__float_as_uint(x) & 0x7fffffffu) - 1u; }
+// Do pairs under one scale hold every value of the group?  Down to 2^-28 of the largest they keep at least 22 bits; below, a value is off by up to
+// 2^-50 of the largest.  Where not, the scale that is stored is negative, and sums that this could show in are formed again from the fp32
+// operands (umma_gemm_kernel.cuh, repair).
+__device__ __forceinline__ bool pairs_hold(uint32_t max_bits, uint32_t low) {
+    return low == 0xffffffffu || __uint_as_float(low + 1u) * 268435456.f >= __uint_as_float(max_bits);
+}
+
 // two scaled values -> their high and low parts
 __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo) {
     const __half2 h = __floats2half2_rn(a, b);
@@ -42,5 +51,7 @@ __device__ __forceinline__ void store_pairs4(const SplitRows& d, int64_t m, int6
     *reinterpret_cast<uint2*>(p) = hi;
     *reinterpret_cast<uint2*>(p + d.m_pad * d.k_pad) = lo;
 }
+// the same values in fp32, for a row that pairs do not hold
+__device__ __forceinline__ void store_full4(const SplitRows& d, int64_t m, int64_t k, float4 v) { *reinterpret_cast<float4*>(d.full + m * d.full_ld + k) = v; }
 
 }  // namespace rmlk

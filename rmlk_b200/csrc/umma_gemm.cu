@@ -165,6 +165,15 @@ int umma_split(cudaStream_t st, const SplitRows& x, const SplitWeights& w, float
     p.x_lo_row = static_cast<int>(x.m_pad);
     p.w_scale = w.scale;
     p.x_scale = x.scale;
+    p.K = x.k;
+    p.w_src = w.src;
+    p.w_col0 = w.col0;
+    p.x_full = x.full;
+    p.x_full_ld = x.full_ld;
+    p.x_full_all = x.full_all ? 1 : 0;
+    p.x_pairs = x.data;
+    p.x_k_pad = x.k_pad;
+    p.x_low = x.m_pad * x.k_pad;
     p.x_scale_pitch = scales ? x.scale_pitch : 0;  // one scale per row: every chunk reads the same one
     p.chunk_blocks = scales || !short_sums ? x.chunk_blocks : SHORT_BLOCKS;
     p.w_static = (flags & RMLK_MATMUL_B_STATIC) ? 1 : 0;

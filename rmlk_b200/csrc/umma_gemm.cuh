@@ -2,6 +2,7 @@
 #pragma once
 
 #include "matmul_tc.cuh"
+#include "umma_gemm.h"
 
 namespace rmlk {
 namespace umma {
@@ -85,10 +86,17 @@ struct Params {
     int k_blocks, k_per_split, ksplit;
     int w_rows_per_tile;     // packed weights: rows of the tile map per block of 128 columns
     int x_lo_row;            // split activations: row of the low part of row 0 in the activation map
-    const float* w_scale;    // split operands: per column / [chunk][x_scale_pitch] per row, exact powers of two; NULL: none
-    const float* x_scale;
+    const float* w_scale;    // split operands: per column / [chunk][x_scale_pitch] per row, exact powers of two, negative where
+    const float* x_scale;    // pairs do not hold the column / the row; NULL: none
     int64_t x_scale_pitch;
     int chunk_blocks;        // k-blocks that share a row scale
+    int64_t K;               // split operands as they are, for the sums that are formed again (repair): W in its sources, X as fp32 rows
+    WeightSources w_src;     // (all of them, or those that pairs do not hold) and as pairs
+    int64_t w_col0;
+    const float* x_full;
+    int64_t x_full_ld, x_k_pad, x_low;
+    int x_full_all;
+    const void* x_pairs;
     int w_static;            // nothing in flight writes the weights: their first loads may go out before the previous kernel has finished
     int* status;
 };
@@ -99,6 +107,8 @@ struct Layout {
     // Epilogue warps, two or four for each group of 32 TMEM lanes: at most 64 sums per thread, so that nothing spills.
     static constexpr int EPI_WARPS = MT >= 192 ? 16 : 8;
     static constexpr int THREADS = 64 + 32 * EPI_WARPS;  // TMA warp, MMA warp, epilogue warps
+    // Small tiles leave registers for the CTAs of the kernels before and behind, which overlap with this one: those of as many threads.
+    static constexpr int REGS_FOR = !SPLIT || MT > 64 ? THREADS : MT == 64 ? 512 : 640;
     static constexpr int XR = MT / CG;  // activation rows that this CTA loads
     static constexpr uint32_t W_BYTES = W_TILE * (SPLIT ? 2 : 1);
     static constexpr uint32_t X_TILE = XR * BK * 2;

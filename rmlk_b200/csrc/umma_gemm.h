@@ -28,23 +28,29 @@ struct WeightSources {
 };
 struct SplitWeights {
     void* tiles;   // [n_blocks][k_blocks][2][16 KB]
-    float* scale;  // per column, padded to whole blocks; behind it the scratch of the packing kernels
+    float* scale;  // per column, padded to whole blocks, negative where pairs do not hold the column; behind it the scratch of the packing kernels
     int64_t n, k, n_blocks, k_blocks;
+    WeightSources src;  // the fp32 matrices, which have to stay: a column that pairs do not hold is read from them
+    int64_t col0;       // first column of a window
 };
 size_t split_weights_bytes(int64_t n, int64_t k);
 SplitWeights split_weights_at(void* buf, int64_t n, int64_t k);  // buf: 1 KB aligned
 SplitWeights split_weights_window(const SplitWeights& w, int64_t n0, int64_t n);  // columns [n0, n0 + n), n0 a multiple of 128
-int split_weights_pack(cudaStream_t st, const WeightSources& src, const SplitWeights& w);
+int split_weights_pack(cudaStream_t st, const WeightSources& src, SplitWeights& w);
 
 struct SplitRows {
     void* data;    // f16 [2][m_pad][k_pad]: high parts over low parts; rows behind m are never read into a result
-    float* scale;  // [chunks][scale_pitch]
+    float* scale;  // [chunks][scale_pitch], negative where pairs do not hold the values of the row in the chunk
     int64_t m, k, m_pad, k_pad, scale_pitch;
     int chunk_blocks;  // blocks of 64 k that share a scale
+    float* full;       // rows of k fp32 values, full_ld apart: all of them (full_all), or those that pairs do not hold
+    int64_t full_ld;
+    bool full_all;
 };
-size_t split_rows_bytes(int64_t m, int64_t k, int chunk_blocks);  // chunk_blocks 0: one scale per row
-SplitRows split_rows_at(void* buf, int64_t m, int64_t k, int chunk_blocks);
-int split_rows_pack(cudaStream_t st, const float* x, int64_t ldx, const SplitRows& dst);  // one scale per row
+// chunk_blocks 0: one scale per row.  keep_full: with room for the fp32 values of rows that pairs do not hold, for a producer to write.
+size_t split_rows_bytes(int64_t m, int64_t k, int chunk_blocks, bool keep_full);
+SplitRows split_rows_at(void* buf, int64_t m, int64_t k, int chunk_blocks, bool keep_full);
+int split_rows_pack(cudaStream_t st, const float* x, int64_t ldx, SplitRows& dst);  // one scale per row; x has to stay, it is dst.full
 
 // out[m, n] = x w.  With `parts` the K splits may be left as f32 slabs [*parts][m][n] in `slabs` (*parts = 1: out holds the result);
 // without it, or without room for the slabs, K is not split.

@@ -63,8 +63,115 @@ __device__ __forceinline__ Item item_at(int w, const Params& p) {
     return it;
 }
 
+// Pairs keep an element of a row or column to 2^-50 of its largest at worst.  With Xmax < 2^15 sx and Wmax < 2^15 sw a sum over k terms is off
+// by less than 2^-20 k sx sw through that: by 2^-21 of itself where it is 2 k sx sw or more, which ordinary sums are (they measure in the tens of
+// millions of sx sw, so that one in a million falls below).  Tiles with a marked row or column keep the smallest of their sums, chunk by chunk, as
+// they come out of TMEM, and look closer where it falls below: at the sums of the marked rows and columns.  Where one of those does - a column of a table whose largest entry no row asks for, a row whose large values meet zeros - the
+// sums that small are formed again here from the fp32 operands.  One warp, columns n of its lanes, rows m_base .. m_base + HM; behind all tiles,
+// so that nothing waits for it.
+// (Few registers: what it needs is added to what the product's kernel needs.)
+__device__ __noinline__ void repair(const Params& p, int rows, int split, int64_t m_base, int64_t n) {
+    constexpr int R = 4;
+    const int lane = threadIdx.x & 31;
+    const int kb0 = split * p.k_per_split, nk = min(p.k_per_split, p.k_blocks - kb0);
+    const int k0 = kb0 * BK, k1 = static_cast<int>(min(p.K, static_cast<int64_t>(k0) + nk * BK));
+    const bool in = n < p.N;
+    const float ws = in ? p.w_scale[n] : 1.f;
+    const bool any_col = __any_sync(0xffffffffu, in && ws < 0.f);
+    float* out = static_cast<float*>(p.out) + (p.ksplit > 1 ? static_cast<int64_t>(split) * p.M * p.N : 0) + n;
+    const float* w = nullptr;  // column n of W in fp32, ldw apart
+    int64_t ldw = 0;
+    if (in) {
+        const int64_t c = n + p.w_col0;
+        int j = 0;
+        while (j + 1 < p.w_src.count && c >= p.w_src.col0[j + 1]) j++;
+        w = p.w_src.w[j] + c - p.w_src.col0[j];
+        ldw = p.w_src.n[j];
+    }
+    auto chunk_at = [&](int k) { return k / BK / p.chunk_blocks * p.x_scale_pitch; };
+    auto x_at = [&](int64_t m, int k, int64_t chunk) {
+        const float s = p.x_scale[chunk + m];
+        if (p.x_full_all || s < 0.f) return p.x_full[m * p.x_full_ld + k];
+        const __half* h = static_cast<const __half*>(p.x_pairs) + m * p.x_k_pad + k;
+        return fmaf(__half2float(h[p.x_low]), 1.f / LO_SCALE, __half2float(h[0])) * s;
+    };
+    rows = static_cast<int>(min(static_cast<int64_t>(rows), p.M - m_base));
+#pragma unroll 1
+    for (int j0 = 0; j0 < rows; j0 += R) {
+        uint32_t lanes[R];
+        int total = 0;
+#pragma unroll
+        for (int j = 0; j < R; j++) {
+            lanes[j] = 0;
+            if (j0 + j >= rows) continue;
+            const int64_t m = m_base + j0 + j;
+            float most = 0.f;
+            bool wide = any_col;
+#pragma unroll 1
+            for (int c = kb0 / p.chunk_blocks; c <= (kb0 + nk - 1) / p.chunk_blocks; c++) {
+                const float s = p.x_scale[c * p.x_scale_pitch + m];
+                most = fmaxf(most, fabsf(s));
+                wide = wide || s < 0.f;
+            }
+            if (!wide) continue;
+            const float v = in ? out[m * p.ldc] : 0.f;
+            lanes[j] = __ballot_sync(0xffffffffu, in && fabsf(v) < 2.f * static_cast<float>(k1 - k0) * most * fabsf(ws));
+            total += __popc(lanes[j]);
+        }
+        if (total == 0) continue;
+        if (total <= 12) {  // a sum at a time, the lanes along k
+#pragma unroll 1
+            for (int j = 0; j < R; j++) {
+                const int64_t m = m_base + j0 + j;
+                for (uint32_t left = j == 0 ? lanes[0] : j == 1 ? lanes[1] : j == 2 ? lanes[2] : lanes[3]; left; left &= left - 1) {
+                    const int l = __ffs(left) - 1;
+                    const float* wl = reinterpret_cast<const float*>(__shfl_sync(0xffffffffu, reinterpret_cast<uint64_t>(w), l));
+                    const int64_t ld = __shfl_sync(0xffffffffu, ldw, l);
+                    float sum = 0.f;
+#pragma unroll 2
+                    for (int k = k0 + lane; k < k1; k += 32) sum = fmaf(x_at(m, k, chunk_at(k)), wl[k * ld], sum);
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+                    if (lane == l) out[m * p.ldc] = sum;
+                }
+            }
+            continue;
+        }
+        // a column per lane, four rows
+        float sum[R] = {0.f, 0.f, 0.f, 0.f};
+        int k = k0;
+        if (p.x_full_all) {
+            const float* x = p.x_full + (m_base + j0) * p.x_full_ld;
+            const int64_t last = rows - 1 - j0;
+#pragma unroll 1
+            for (; k + 4 <= k1; k += 4) {
+                float wv[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) wv[i] = in ? w[(k + i) * ldw] : 0.f;
+#pragma unroll
+                for (int j = 0; j < R; j++) {
+                    const float* row = x + min(static_cast<int64_t>(j), last) * p.x_full_ld + k;
+#pragma unroll
+                    for (int i = 0; i < 4; i++) sum[j] = fmaf(row[i], wv[i], sum[j]);
+                }
+            }
+        }
+#pragma unroll 1
+        for (; k < k1; k++) {
+            const float wv = in ? w[k * ldw] : 0.f;
+#pragma unroll
+            for (int j = 0; j < R; j++)
+                if (lanes[j]) sum[j] = fmaf(x_at(m_base + j0 + j, k, chunk_at(k)), wv, sum[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < R; j++)
+            if (lanes[j] >> lane & 1) out[(m_base + j0 + j) * p.ldc] = sum[j];
+    }
+}
+
 template <int CG, bool SPLIT, int MT, int ST, bool OUT16>
-__global__ void __launch_bounds__(Layout<CG, SPLIT, MT, ST>::THREADS, 1) gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, Params p) {
+__global__ void __launch_bounds__(Layout<CG, SPLIT, MT, ST>::REGS_FOR, 1) gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX,
+                                                                                     const __grid_constant__ Params p) {
     using L = Layout<CG, SPLIT, MT, ST>;
     dep_trigger();
     extern __shared__ uint8_t smem_raw[];
@@ -244,14 +351,20 @@ __global__ void __launch_bounds__(Layout<CG, SPLIT, MT, ST>::THREADS, 1) gemm_ke
         dep_wait();  // scales and outputs may belong to kernels before this one
         int buf = 0;
         uint32_t acc_phase = 0;
-        bool ok = true;
+        bool ok = true, again = false;  // again: a sum of this thread has to be formed again (repair)
         for (int w = first; w < items && ok; w += stride) {
             const Item it = item_at(w, p);
             const int kb0 = it.split * p.k_per_split, nk = min(p.k_per_split, p.k_blocks - kb0);
             const int64_t n = (static_cast<int64_t>(it.n_tile) * CG + rank) * BN + sub * 32 + lane;
             const bool in = n < p.N;
             float ws = 0.f;
-            if constexpr (SPLIT && !ONE_CHUNK) ws = in ? __ldg(p.w_scale + n) : 0.f;
+            float low = INFINITY;       // smallest sum over a chunk, rows behind the last one among them
+            bool col_marked = false, row_marked = false;  // this column; one of the tile's rows that this lane has the scale of
+            if constexpr (SPLIT) {
+                const float w_scale = in ? __ldg(p.w_scale + n) : 0.f;
+                col_marked = w_scale < 0.f;
+                if constexpr (!ONE_CHUNK) ws = fabsf(w_scale);
+            }
             const int64_t m_base = static_cast<int64_t>(it.m_tile) * MT + part * HM;
             float acc[HM];
             float4 s4 = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -262,7 +375,11 @@ __global__ void __launch_bounds__(Layout<CG, SPLIT, MT, ST>::THREADS, 1) gemm_ke
             for (int c = c_first; c <= c_last && ok; c++) {
                 // the scales of this warp's rows, four per lane, handed round by shuffles when they are needed
                 if constexpr (SPLIT) {
-                    if (4 * lane < HM) s4 = __ldg(reinterpret_cast<const float4*>(p.x_scale + c * p.x_scale_pitch + m_base) + lane);
+                    if (4 * lane < HM) {
+                        s4 = __ldg(reinterpret_cast<const float4*>(p.x_scale + c * p.x_scale_pitch + m_base) + lane);
+                        const int64_t left = p.M - m_base - 4 * lane;  // (what lies behind the last row is no scale)
+                        row_marked = row_marked || (s4.x < 0.f && left > 0) || (s4.y < 0.f && left > 1) || (s4.z < 0.f && left > 2) || (s4.w < 0.f && left > 3);
+                    }
                 }
                 ok = __all_sync(0xffffffffu, mbar_wait(acc_full(buf), acc_phase, abort_flag, p.status));  // (one lane's limit may run out before another's)
                 if (!ok) break;
@@ -279,7 +396,10 @@ __global__ void __launch_bounds__(Layout<CG, SPLIT, MT, ST>::THREADS, 1) gemm_ke
                             tmem_ld<STEP>(d + MT + j0, q);
                             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                            for (int j = 0; j < STEP; j++) acc[j0 + j] = add_low(acc[j0 + j], __uint_as_float(q[j]));
+                            for (int j = 0; j < STEP; j++) {
+                                acc[j0 + j] = add_low(acc[j0 + j], __uint_as_float(q[j]));
+                                low = fminf(low, fabsf(acc[j0 + j]));
+                            }
                         }
                     }
                 } else {
@@ -291,7 +411,9 @@ __global__ void __launch_bounds__(Layout<CG, SPLIT, MT, ST>::THREADS, 1) gemm_ke
                         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
                         for (int j = 0; j < STEP; j++) {
-                            const float v = unscale(add_low(__uint_as_float(r[j]), __uint_as_float(q[j])), row_scale(j0 + j), ws);
+                            float v = add_low(__uint_as_float(r[j]), __uint_as_float(q[j]));
+                            low = fminf(low, fabsf(v));
+                            v = unscale(v, fabsf(row_scale(j0 + j)), ws);
                             acc[j0 + j] = c == c_first ? v : acc[j0 + j] + v;
                         }
                     }
@@ -308,14 +430,28 @@ __global__ void __launch_bounds__(Layout<CG, SPLIT, MT, ST>::THREADS, 1) gemm_ke
                 }
             }
             if (!ok) break;
-            if constexpr (SPLIT && ONE_CHUNK) ws = in ? __ldg(p.w_scale + n) : 0.f;
+            if constexpr (SPLIT && ONE_CHUNK) ws = in ? fabsf(__ldg(p.w_scale + n)) : 0.f;
+            if constexpr (SPLIT) {
+                const float least = 2.f * BK * min(p.chunk_blocks, nk);
+                if (__any_sync(0xffffffffu, col_marked || row_marked) && __any_sync(0xffffffffu, in && low < least)) {
+                    if (c_first < c_last) {
+                        again = true;
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < HM; j++) {
+                            const float xs = row_scale(j);
+                            again = again || (in && m_base + j < p.M && (col_marked || xs < 0.f) && fabsf(acc[j]) < (ONE_CHUNK ? least : least * fabsf(xs) * ws));
+                        }
+                    }
+                }
+            }
             using Out = typename std::conditional<OUT16, __half, float>::type;
             Out* o = static_cast<Out*>(p.out) + (p.ksplit > 1 ? static_cast<int64_t>(it.split) * p.M * p.N : 0) + m_base * p.ldc + n;
             const int64_t rows = in ? p.M - m_base : 0;
 #pragma unroll
             for (int j = 0; j < HM; j++) {
                 float v = acc[j];
-                if constexpr (SPLIT && ONE_CHUNK) v = unscale(v, row_scale(j), ws);
+                if constexpr (SPLIT && ONE_CHUNK) v = unscale(v, fabsf(row_scale(j)), ws);
                 if (j < rows) {
                     if constexpr (OUT16) *o = __float2half_rn(v);
                     else *o = v;
@@ -324,6 +460,12 @@ __global__ void __launch_bounds__(Layout<CG, SPLIT, MT, ST>::THREADS, 1) gemm_ke
                 asm volatile("" : "+l"(o)::"memory");  // one row after the other: addresses and scales of all 128 rows would not fit in registers beside the sums
             }
         }
+        if constexpr (SPLIT)
+            if (ok && __any_sync(0xffffffffu, again))
+                for (int w = first; w < items; w += stride) {
+                    const Item it = item_at(w, p);
+                    repair(p, HM, it.split, static_cast<int64_t>(it.m_tile) * MT + part * HM, (static_cast<int64_t>(it.n_tile) * CG + rank) * BN + sub * 32 + lane);
+                }
     }
     tc_fence_before();
     if constexpr (CG == 2) cluster_sync_all();  // no CTA of the pair leaves while the other may still signal its barriers or read its tiles
