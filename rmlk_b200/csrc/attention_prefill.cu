@@ -29,8 +29,12 @@ constexpr int D = 64;          // head size
 constexpr int QT = 128;        // query rows per CTA = MMA M = threads
 constexpr int KT = 64;         // keys per block
 constexpr uint32_t QH = 0, QL = 16384, KH = 32768, VH = 49152, PH = 65536, PL = 81920;  // low tiles of K and V lie 8 KB behind the high ones
-constexpr uint32_t ROW_OFF = 98304, RED = ROW_OFF + QT * 8, BARS = RED + 4 * 16, TOTAL = BARS + 32 + 1024;
+constexpr uint32_t ROW_OFF = 98304, RED = ROW_OFF + QT * 8, BARS = RED + 4 * 16 + 16, TOTAL = BARS + 32 + 1024;
 constexpr float P_SCALE = 16384.f;  // probabilities are at most 1
+// Queries of a tile share a scale, keys of a block do, values of a block do.  Values far below the largest are held to 2^-50 of that:
+// Scores are off by less than 2^-43 |q|max |k|max scale through it, less than a rounding of the exponent's argument up to here; above, or where the
+// values of the blocks span more than pairs hold and a result is too small to hide it, the tile is left to rows_in_fp32.
+constexpr float SCORES_MOST = 65536.f;
 
 struct Params {
     const float *q, *k, *v, *mask;
@@ -78,12 +82,63 @@ __device__ __forceinline__ float joined(uint32_t high, uint32_t low) {
     return fabsf(h) < INFINITY ? fmaf(__uint_as_float(low), 1.f / LO_SCALE, h) : h;
 }
 
+// The tile's rows one per thread in fp32.  512 keys: one tile 353 us (58 us on pairs), all tiles of [4, 32 heads, 512] queries 876 us (107 us).
+__device__ __noinline__ void rows_in_fp32(const Params& p, int64_t prob, int row0, int64_t mask_row) {
+    const int row = row0 + threadIdx.x;
+    if (row >= p.rows) return;
+    const int64_t b = prob / p.kv_heads;
+    const int g = row / p.S, s_at = row - g * p.S;
+    const int64_t h = (prob - b * p.kv_heads) * p.G + g;
+    const float4* Q = reinterpret_cast<const float4*>(p.q + (prob * p.rows + row) * D);
+    const float4* K = reinterpret_cast<const float4*>(p.k + prob * p.kb);
+    const float4* V = reinterpret_cast<const float4*>(p.v + prob * p.vb);
+    float4 q[D / 4], acc[D / 4];
+#pragma unroll
+    for (int j = 0; j < D / 4; j++) {
+        q[j] = Q[j];
+        acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float top = -INFINITY, sum = 0.f;
+#pragma unroll 1
+    for (int64_t t = 0; t < p.T; t++) {
+        float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int j = 0; j < D / 4; j++) {
+            const float4 k = K[t * (D / 4) + j];
+            d.x = fmaf(q[j].x, k.x, d.x);
+            d.y = fmaf(q[j].y, k.y, d.y);
+            d.z = fmaf(q[j].z, k.z, d.z);
+            d.w = fmaf(q[j].w, k.w, d.w);
+        }
+        float x = __fmul_rn((d.x + d.y) + (d.z + d.w), p.scale);
+        if (p.mask) x = __fadd_rn(x, p.mask[mask_row + t]);
+        if (x > top) {
+            const float corr = top == -INFINITY ? 0.f : expf(top - x);
+            top = x;
+            sum *= corr;
+#pragma unroll
+            for (int j = 0; j < D / 4; j++) acc[j] = make_float4(acc[j].x * corr, acc[j].y * corr, acc[j].z * corr, acc[j].w * corr);
+        }
+        const float e = expf(x - (top == -INFINITY ? 0.f : top));
+        sum += e;
+#pragma unroll
+        for (int j = 0; j < D / 4; j++) {
+            const float4 v = V[t * (D / 4) + j];
+            acc[j] = make_float4(fmaf(e, v.x, acc[j].x), fmaf(e, v.y, acc[j].y), fmaf(e, v.z, acc[j].z), fmaf(e, v.w, acc[j].w));
+        }
+    }
+    float4* o = reinterpret_cast<float4*>(p.out + b * p.os_b + h * p.os_h + s_at * p.os_s);
+#pragma unroll
+    for (int j = 0; j < D / 4; j++) o[j] = make_float4(acc[j].x / sum, acc[j].y / sum, acc[j].z / sum, acc[j].w / sum);
+}
+
 __global__ void __launch_bounds__(QT, 2) attention_kernel(const __grid_constant__ Params p) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* sm = smem_raw + (base - smem_u32(smem_raw));
     int64_t* s_row = reinterpret_cast<int64_t*>(sm + ROW_OFF);
     uint4* s_red = reinterpret_cast<uint4*>(sm + RED);
+    uint32_t* s_low = reinterpret_cast<uint32_t*>(sm + RED + 64);
     const uint32_t bar_s = base + BARS, bar_o = bar_s + 8;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sm + BARS + 16);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(sm + BARS + 20);
@@ -118,6 +173,7 @@ __global__ void __launch_bounds__(QT, 2) attention_kernel(const __grid_constant_
     // ---- queries ----
     int qe;
     bool q_plain;
+    float k_most;  // scores stay below SCORES_MOST with keys up to this
     {
         float4 x[16];
         const float* Qp = p.q + (prob * p.rows + row0) * D;
@@ -141,6 +197,7 @@ __global__ void __launch_bounds__(QT, 2) attention_kernel(const __grid_constant_
         }
         qe = scale_exponent(m.finite);
         q_plain = m.any < 0x58800000u;  // 2^50
+        k_most = SCORES_MOST / (__uint_as_float(m.finite) * fabsf(p.scale));  // (infinite where all queries are zero)
         const float up = exp2_int(qe);
 #pragma unroll
         for (int i = 0; i < 16; i++) put_pairs(sm + QH, QL - QH, r8 + 8 * i, c4, x[i], up);
@@ -173,7 +230,8 @@ __global__ void __launch_bounds__(QT, 2) attention_kernel(const __grid_constant_
     for (int j = 0; j < D; j++) acc[j] = 0.f;
     float top = -INFINITY, sum = 0.f;
     uint32_t phase = 0;
-    bool ok = true;
+    bool ok = true, plain = true;  // plain: pairs do
+    uint32_t v_max = 0, v_low = 0xffffffffu;
     for (int key0 = 0; key0 < p.T; key0 += KT) {
         // The mask of the block goes where the probabilities will be: the row's first 32 values into its 128 bytes of the high tile, the others into
         // the low tile's, so that a thread overwrites nothing but what it has read.
@@ -195,14 +253,20 @@ __global__ void __launch_bounds__(QT, 2) attention_kernel(const __grid_constant_
             }
         }
         Mags km = {0, 0}, vm = {0, 0};
+        uint32_t low = 0xffffffffu;
 #pragma unroll
         for (int i = 0; i < 8; i++) {
             km.add(kx[i]);
             vm.add(vx[i]);
+            low = min(min(low, min(nonzero_low(vx[i].x), nonzero_low(vx[i].y))), min(nonzero_low(vx[i].z), nonzero_low(vx[i].w)));
         }
         km.warp_max();
         vm.warp_max();
-        if (lane == 0) s_red[warp] = make_uint4(km.finite, km.any, vm.finite, vm.any);
+        low = __reduce_min_sync(0xffffffffu, low);
+        if (lane == 0) {
+            s_red[warp] = make_uint4(km.finite, km.any, vm.finite, vm.any);
+            s_low[warp] = low;
+        }
         asm volatile("cp.async.wait_all;" ::: "memory");
         if (__syncthreads_or(!ok)) {
             ok = false;
@@ -215,6 +279,7 @@ __global__ void __launch_bounds__(QT, 2) attention_kernel(const __grid_constant_
             km.any = max(km.any, x.y);
             vm.finite = max(vm.finite, x.z);
             vm.any = max(vm.any, x.w);
+            low = min(low, s_low[w]);
         }
         if (key0 > 0 && p.mask) {
             float most = -INFINITY;
@@ -233,6 +298,12 @@ __global__ void __launch_bounds__(QT, 2) attention_kernel(const __grid_constant_
                 load_kv(key0 + KT);
                 continue;
             }
+        }
+        v_max = max(v_max, vm.finite);
+        v_low = min(v_low, low);
+        if (!(__uint_as_float(km.finite) <= k_most)) {
+            plain = false;
+            break;
         }
         const int ke = scale_exponent(km.finite), ve = scale_exponent(vm.finite);
         {
@@ -332,7 +403,17 @@ __global__ void __launch_bounds__(QT, 2) attention_kernel(const __grid_constant_
         phase ^= 1;
     }
     const bool bad = __syncthreads_or(!ok);
-    if (row < p.rows) {
+    if (plain && !pairs_hold(v_max, v_low)) {  // the same in every thread
+        // each block's share is off by less than 2^-43 of the largest value: by 2^-21 of a result that is not below this
+        const float least = __uint_as_float(v_max) * (1.f / 4194304.f) * static_cast<float>(p.T / KT + 1);
+        bool small = false;
+#pragma unroll
+        for (int j = 0; j < D; j++) small = small || fabsf(acc[j]) < least;
+        plain = !__syncthreads_or(small && row < p.rows);
+    }
+    if (!plain && !bad) {
+        rows_in_fp32(p, prob, row0, s_row[tid]);
+    } else if (row < p.rows) {
         float4* o = reinterpret_cast<float4*>(p.out + b * p.os_b + h * p.os_h + s_at * p.os_s);
         const float nan = __int_as_float(0x7fc00000);
 #pragma unroll

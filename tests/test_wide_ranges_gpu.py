@@ -200,3 +200,56 @@ def test_attention_rows(cuda, B, T):
     p = e / e.sum(-1, keepdims=True)
     want, mag = (p @ v).reshape(B, H * D) @ sel, (p @ np.abs(v)).reshape(B, H * D) @ sel
     assert (np.abs(got[:, 0] - want) <= 2e-5 * mag).all()
+
+
+def _attention_cases():
+    def value_behind(q, k, v):  # a finite, very large value at a key that the later rows see and the earlier ones do not
+        v[0, 0, 100] = 1e30
+        v[0, 1, 101, 7] = LOWEST
+
+    def values_apart(q, k, v):  # blocks of values 2^60 apart, dims 2^45 apart
+        v[:, 0, 64:128] *= 2.0 ** 60
+        v[:, 1, :, ::3] *= 2.0 ** -45
+
+    def faint_giant(q, k, v):  # a huge value under a weight of 2^-50 beside ordinary ones under weights of 1
+        k[:, :, 5] = 0
+        q[:, :, :, :, 0] = 8.0
+        k[:, :, :, 0] = 0
+        k[:, :, 5, 0] = -35.0
+        v[:, :, 5] *= 2.0 ** 45
+
+    def keys_apart(q, k, v):  # scores far beyond what one scale for queries and keys holds
+        k[0, 0, 30] *= 1e20
+        q[0, 1, 0, 9] *= 1e12
+
+    def query_apart(q, k, v):  # one row of the tile 2^60 above the others, with scores of ordinary size
+        q[:, :, :, 3] *= 2.0 ** 60
+        q[:, :, :, 3, 1:] = 0
+        k[:, :, :, 0] *= 2.0 ** -60
+        q[:, :, :, 4:, 1:] *= 4.0
+
+    return {f.__name__: f for f in (value_behind, values_apart, faint_giant, keys_apart, query_apart)}
+
+
+@pytest.mark.parametrize("case", sorted(_attention_cases()))
+@pytest.mark.parametrize("B,KV,G,S", [(1, 2, 1, 130), (1, 2, 4, 150)])
+def test_prompt_attention(cuda, case, B, KV, G, S):
+    import torch
+    from rmlk_b200 import kernels as K
+    gen = torch.Generator(device=cuda)
+    gen.manual_seed(S)
+    q, k, v = (torch.randn(B, KV, *x, 64, device=cuda, generator=gen) for x in ((G, S), (S,), (S,)))
+    _attention_cases()[case](q, k, v)
+    mask = torch.zeros(B, 1, S, S, device=cuda).masked_fill(torch.arange(S, device=cuda)[None] > torch.arange(S, device=cuda)[:, None], LOWEST)
+    got = K.gqa_prefill_attention(q, k, v, 0.125, mask).double()
+    s = torch.einsum("bkgsd,bktd->bkgst", q.double(), k.double()) * 0.125
+    # (what fp32 products of this size round to: a score is off by 2^-22 of its terms, a weight by that much of itself)
+    slack = (torch.einsum("bkgsd,bktd->bkgst", q.double().abs(), k.double().abs()) * 0.125 * 2.0 ** -22).amax(-1, keepdim=True)
+    p = torch.softmax(s + mask.double()[:, :, None], -1)
+    want = torch.einsum("bkgst,bktd->bkgsd", p, v.double())
+    mag = torch.einsum("bkgst,bktd->bkgsd", p, v.double().abs()) * (2e-6 + 2 * slack.clamp(max=1.0))
+    lay = lambda x: x.permute(0, 3, 1, 2, 4).reshape(B, S, KV * G, 64)  # noqa: E731
+    off, bound = (got - lay(want)).abs(), lay(mag)
+    settled = (lay(slack.expand_as(want)) < 0.1)  # (rows of scores beyond 2^20 are one-hot up to rounding: only that they are numbers)
+    assert bool((off <= bound)[settled].all()), float((off / bound)[settled].max())
+    assert bool(torch.isfinite(got).all())
