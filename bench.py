@@ -220,8 +220,53 @@ def time_graph(fn_of_i, n=16, replays=4):
 # dram__bytes_read.sum + dram__bytes_write.sum per launch of the kernel named by DOMINANT, from one ncu capture of that
 # kernel on this shape (a cross-check of the algorithmic bytes, not a live measurement: it goes stale when the kernel changes)
 DOMINANT = "matmul_gate_up"
-NCU_TRAFFIC_BYTES = {"matmul_gate_up": 134_809_600 + 3_740_416}
-NCU_TRAFFIC_SOURCE = "ncu --set full capture of tc_gemm_kernel on [64,2048]x[2048,16384] (read 134.81 MB + write 3.74 MB per launch)"
+NCU_TRAFFIC_BYTES = {"matmul_gate_up": 134_876_928 + 3_592_448}
+NCU_TRAFFIC_SOURCE = "ncu capture of umma::gemm_kernel on [64,2048]x[2048,16384] (read 134.88 MB + write 3.59 MB per launch)"
+
+
+def time_packed_products(m, k, weights):
+    """Milliseconds per product of one [m, k] operand with each of the constant weights, and launches per product: a graph in which one producer
+    writes the operand (RMSNorm, or SwiGLU where rows are long) and a MatMul per weight reads it, so that the producer's
+    launch is a small share.  The weights together are larger than L2."""
+    import torch
+    from rmlk_b200 import dtypes as dt
+    from rmlk_b200.graphspec import GraphSpec
+    from rmlk_b200.runtime import ModelInstance
+    g = GraphSpec()
+    g.input("x", np.float32, [0, k])
+    g.input("u", np.float32, [0, k])
+    if k <= 4096:
+        for name, value in (("two", 2.0), ("eps", 1e-5)):
+            g.const(name, np.array(value, np.float32))
+        g.const("scale", np.ones(k, np.float32))
+        mean = g.op("ReduceMean", [g.op("Pow", ["x", "two"])], axes=[-1], keepdims=1)
+        a = g.op("Mul", [g.op("Div", ["x", g.op("Sqrt", [g.op("Add", [mean, "eps"])])]), "scale"])
+    else:
+        a = g.op("Mul", [g.op("Mul", ["x", g.op("Sigmoid", ["x"])]), "u"])
+    for i, w in enumerate(weights):
+        g.const_device(f"w{i}", w)
+        g.op("MatMul", [a, f"w{i}"], f"y{i}")
+        g.output(f"y{i}")
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    inst = ModelInstance(g.to_runtime(), stream=stream.cuda_stream)
+    x = torch.randn(m, k, device="cuda")
+    best = None
+    for r in range(6):
+        for name in ("x", "u"):
+            inst.set_input_ptr(name, dt.F32, [m, k], x.data_ptr(), True)
+        torch.cuda.synchronize()
+        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        with torch.cuda.stream(stream):
+            torch.cuda._sleep(400_000)  # the host runs ahead, so that the products follow one another without gaps
+            e0.record(stream)
+            inst.launch()
+            e1.record(stream)
+        stream.synchronize()
+        if r >= 3:
+            ms = e0.elapsed_time(e1)
+            best = ms if best is None else min(best, ms)
+    return best / len(weights), inst.last_launches / len(weights)
 
 
 def kernel_rooflines(batch, ctx, peak_gbs, peak_kind):
@@ -236,8 +281,8 @@ def kernel_rooflines(batch, ctx, peak_gbs, peak_kind):
     def ring(make, nbytes_each):
         return [make() for _ in range(max(2, min(6, (252 << 20) // max(nbytes_each, 1) + 1)))]
 
-    def add(name, kernel, fn, algo_bytes, shape, flops=0):
-        ms = time_graph(fn)
+    def add(name, kernel, fn, algo_bytes, shape, flops=0, ms=None):
+        ms = time_graph(fn) if ms is None else ms
         ach = algo_bytes / (ms * 1e-3) / 1e9
         e = {"bound": "hbm", "achieved": ach, "peak": peak_gbs, "unit": "GB/s", "frac": ach / peak_gbs,
              "traffic": NCU_TRAFFIC_BYTES.get(name), "traffic_source": NCU_TRAFFIC_SOURCE if name in NCU_TRAFFIC_BYTES else None, "kernel": kernel, "shape": shape,
@@ -255,18 +300,21 @@ def kernel_rooflines(batch, ctx, peak_gbs, peak_kind):
     add("attention", "gqa_decode_flash_kernel<16>", lambda i: K.gqa_decode_attention(q, kc[i % len(kc)], kc[(i + 1) % len(kc)], 0.125, mask=mask, out=cx),
         4 * B * 8 * (2 * 64 * T + 2 * 4 * 64) + 4 * B * T, [B * 8, 4, 64, T], flops=4 * B * 32 * 64 * T)
     del kc, q, mask, cx
-    # weight-streaming MatMul at the FFN gate/up shape and at the lm_head
-    # gate | up projections as the runtime runs them (one MatMul on the concatenated weights), the down projection, the lm_head
+    # the products of a step as the runtime runs them: gate | up and q | k | v (one product each on the weights side by side), down, lm_head
     for name, (m, k, n) in (("matmul_gate_up", (B, 2048, 16384)), ("matmul_qkv", (B, 2048, 3072)), ("matmul_down", (B, 8192, 2048)),
                             ("matmul_lm_head", (B, 2048, 128256))):
-        w = ring(lambda: torch.randn(k, n, device=dev) * 0.02, 4 * k * n)
-        x = torch.randn(m, k, device=dev)
-        y = torch.empty(m, n, device=dev)
-        wsb = K.matmul_workspace_bytes(1, m, n, k)
-        ws = torch.empty(max(wsb // 4, 1), device=dev) if wsb else None
-        add(name, "tc_gemm_kernel (tcgen05 3xTF32)" if m > 16 else "skinny_kernel",
-            lambda i: K.matmul(x, w[i % len(w)], out=y, workspace=ws), 4 * (m * k + k * n + m * n), [m, k, n], flops=2 * m * k * n)
-        del w, x, y, ws
+        algo, shape, flops = 4 * (m * k + k * n + m * n), [m, k, n], 2 * m * k * n
+        count = max(2, min(8, (400 << 20) // (4 * k * n)))
+        w = [torch.randn(k, n, device=dev) * 0.02 for _ in range(count)]
+        if m > 4:
+            ms, launches = time_packed_products(m, k, w)
+            add(name, "umma::gemm_kernel (tcgen05 kind::f16 on pairs)", None, algo, shape, flops=flops, ms=ms)
+            out[name]["launches_per_product"] = launches
+        else:
+            x, y = torch.randn(m, k, device=dev), torch.empty(m, n, device=dev)
+            ws = torch.empty(max(K.matmul_workspace_bytes(1, m, n, k) // 4, 4), device=dev)
+            add(name, "gemv_wide_kernel", lambda i: K.matmul(x, w[i % len(w)], out=y, workspace=ws), algo, shape, flops=flops)
+        del w
     torch.cuda.empty_cache()
     return out
 

@@ -264,8 +264,9 @@ RMLK_API int rmlk_b200_matmul_ex(rmlk_stream_t stream, int dtype, int64_t batch,
                         int64_t c_batch_stride, void* workspace, size_t workspace_bytes, int* status);
 /* Same, with hints.  RMLK_MATMUL_B_STATIC: nothing still in flight on the device writes B (model weights).  The
  * kernels of this library let the next kernel of a stream be scheduled while the previous one drains, each waiting for
- * its predecessor before it touches memory; with this flag the tensor-core kernel requests its first tiles of B
- * before that wait, so the weight stream starts under the tail of the previous kernel.  flags = 0: as _ex. */
+ * its predecessor before it touches memory; with this flag the tensor-core kernel and the kernel for a few rows request
+ * their first tiles of B before that wait, so the weight stream starts under the tail of the previous kernel.
+ * flags = 0: as _ex. */
 #define RMLK_MATMUL_B_STATIC 1
 RMLK_API int rmlk_b200_matmul_flags(rmlk_stream_t stream, int dtype, int64_t batch, int64_t m, int64_t n, int64_t k,
                            const void* a, int64_t a_batch_stride, const void* b, int64_t b_batch_stride, void* c,
@@ -273,15 +274,16 @@ RMLK_API int rmlk_b200_matmul_flags(rmlk_stream_t stream, int dtype, int64_t bat
 /* C[:, 0:n] = A x B[:, 0:n] on a block of n columns: b and c point at the block's first column inside matrices whose rows
  * are ld elements apart.  A wide product (the logits of a language model, [64, 2048] x [2048, 128256]) can so be issued
  * block by block and each block copied to the host while the next is computed.  Only for shapes the tensor-core kernel
- * runs without a K split (rmlk_b200_matmul_window_supported); same kernel, same values as rmlk_b200_matmul_ex. */
+ * runs without a K split (rmlk_b200_matmul_window_supported); same kernel and values as rmlk_b200_matmul_ex without a
+ * workspace.  (With the full workspace and 256 rows or more, _ex takes another kernel, whose sums round differently.) */
 RMLK_API int rmlk_b200_matmul_window(rmlk_stream_t stream, int dtype, int64_t m, int64_t n, int64_t k, const void* a, const void* b,
                             void* c, int64_t ld, int* status, int flags);
 RMLK_API int rmlk_b200_matmul_window_supported(int64_t m, int64_t n, int64_t k, int64_t ld);
 /* Unbatched MatMul for a caller that adds split-K partial sums in its own next kernel (rmlk_b200_add_rmsnorm does).
  * When the kernel plan for the shape splits K through the workspace, the [*parts][m*n] slabs are left in `workspace`
  * (to be added in slab order starting from 0.f - the order rmlk_b200_matmul uses) and c is NOT written; otherwise c
- * holds the result and *parts = 1.  Same kernels as rmlk_b200_matmul_ex (cuda/src/kernels/gemm.rs:206-231 in the
- * reference has no such form: cuBLAS reduces internally). */
+ * holds the result and *parts = 1.  Up to 255 rows the same kernels as rmlk_b200_matmul_ex (cuda/src/kernels/gemm.rs:206-231
+ * in the reference has no such form: cuBLAS reduces internally). */
 RMLK_API int rmlk_b200_matmul_parts(rmlk_stream_t stream, int dtype, int64_t m, int64_t n, int64_t k, const void* a, const void* b,
                            void* c, void* workspace, size_t workspace_bytes, int* status, int flags, int* parts);
 /* dst[i] = 0.f + src[0][i] + ... + src[parts-1][i] (slabs of n floats, dense): the split-K reduction that
@@ -317,6 +319,10 @@ RMLK_API int rmlk_b200_matmul_static(rmlk_stream_t stream, int dtype, int64_t ba
 RMLK_API size_t rmlk_b200_matmul_static_scratch_bytes(void);
 /* 1 if rmlk_b200_matmul_static takes the shape (its least scratch need fits the built-in array), 0 if it would be rejected. */
 RMLK_API int rmlk_b200_matmul_static_supported(int dtype, int64_t batch, int64_t m, int64_t n, int64_t k);
+/* Scratch that lets rmlk_b200_matmul take the fastest kernel for a shape; 16-byte aligned.  Less, or NULL, selects a kernel that needs less.
+ * fp32, unbatched, 256 rows or more: room for both operands as pairs of f16 under one power of two per row and column - about the
+ * size of the operands, 300 MB for [4096,4096] x [4096,14336].  Rows and columns whose values span more than such pairs hold (2^28)
+ * come out no less accurate: where it could show, sums are formed again from the fp32 operands (slowly, if that is most of them). */
 RMLK_API size_t rmlk_b200_matmul_workspace_bytes(int dtype, int64_t batch, int64_t m, int64_t n, int64_t k);
 
 /* y[m, n] = alpha * y + beta * c, in place, c read through element strides (0 broadcasts a dimension; c = NULL: y = alpha * y).

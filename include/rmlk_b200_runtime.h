@@ -54,7 +54,10 @@ RMLK_API int rmlk_graph_input(rmlk_graph* g, const char* name, int dtype, int ra
 RMLK_API int rmlk_graph_constant(rmlk_graph* g, const char* name, int dtype, int rank, const int64_t* dims,
                                  const void* data, size_t nbytes);
 /* An initializer that already lives in device memory (weights loaded by another component): used in
- * place, never copied or freed; it must stay valid for as long as any instance built from the graph. */
+ * place, never freed; it must stay valid, and keep its values, for as long as any instance built from the graph.
+ * An instance keeps right operands of MatMul in other layouts as well, made once: weights of products that share their
+ * left operand side by side, and, from the first run with 5 rows on, fp32 weights as pairs of f16 (as many bytes again;
+ * without memory for them the weights are used as they are). */
 RMLK_API int rmlk_graph_constant_device(rmlk_graph* g, const char* name, int dtype, int rank, const int64_t* dims,
                                         const void* device_data);
 /* An intermediate or output value. */

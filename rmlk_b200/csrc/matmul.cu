@@ -1,20 +1,23 @@
 // fp32 MatMul: C[b] = A[b] x B[b], row-major, fp32 accumulate.
 //
-// Two kernels, chosen by shape in rmlk_b200_matmul:
+// The SIMT kernels, and the choice between them and the tensor-core kernels (rmlk_b200_matmul_flags):
 //
-//  skinny_kernel   M <= 16 (decode GEMV / small-batch decode).  Memory-bound: every element of B is
-//                  read exactly once with 128-bit loads along N; a CTA owns a 32-column strip and its
-//                  256 threads are 8 column-quads x 32 k-lanes, 8 independent 128-bit loads in flight
-//                  per thread.  The A rows of the current k-chunk are staged in shared memory as
-//                  [k][m] so one LDS.128 feeds four FMAs rows.  When the strip count cannot fill the
-//                  GPU, K is also split across CTAs into a caller-provided scratch buffer that a
-//                  second kernel sums in a fixed order (deterministic, no atomics).
+//  gemv_wide_kernel  M <= 4, and M <= 16 where no tensor-core kernel applies, against rows of B on 16-byte boundaries: the decode GEMV.
+//                    Memory-bound, B is read once in strips of 128 columns; K splits are added in a cluster, through scratch, or by the reader.
+//  skinny_kernel     M <= 16 otherwise.  Every element of B is read exactly once with 128-bit loads along N where the rows allow; a CTA
+//                    owns a 32-column strip and its 256 threads are 8 column-quads x 32 k-lanes, 8 independent loads in flight per
+//                    thread.  The A rows of the current k-chunk are staged in shared memory as [k][m].  When the strips cannot fill the
+//                    GPU, K is also split across CTAs into a caller-provided scratch buffer that a second kernel sums in a fixed
+//                    order (deterministic, no atomics).
+//  small-K kernels   many small problems (attention products of a decode step): one thread or CTA per problem and block of columns.
+//  gemm_kernel       everything else.  Shared-memory tiled SIMT GEMM (BM x BN x 16, 256 threads, register micro-tiles, double-buffered)
+//                    with guarded edges, any M / N / K.
+//  matmul_tc.cu      from 5 rows on, N % 128 == 0 and K % 32 == 0: 3xTF32 on tcgen05, split in flight.
+//  umma_gemm.cu      from 256 rows on with the workspace that rmlk_b200_matmul_workspace_bytes asks for, any N and K from 64 on: both operands
+//                    split into pairs of f16 first.
 //
-//  gemm_kernel     everything else.  Shared-memory tiled SIMT GEMM (BM x BN x 16, 256 threads,
-//                  register micro-tiles, double-buffered) with guarded edges, any M/N/K.
-//
-// The reference calls cublasGemmStridedBatchedEx with CUBLAS_COMPUTE_32F
-// (cuda/src/kernels/gemm.rs:206-231); both kernels accumulate in fp32 with FMA.
+// The reference calls cublasGemmStridedBatchedEx with CUBLAS_COMPUTE_32F (cuda/src/kernels/gemm.rs:206-231).  The kernels here accumulate
+// in fp32 with FMA; the tensor cores' fp32 accumulators truncate.
 #include <algorithm>
 #include <atomic>
 
