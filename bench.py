@@ -250,11 +250,11 @@ def time_packed_products(m, k, weights):
     stream = torch.cuda.Stream()
     torch.cuda.synchronize()
     inst = ModelInstance(g.to_runtime(), stream=stream.cuda_stream)
-    x = torch.randn(m, k, device="cuda")
+    feeds = {"x": torch.randn(m, k, device="cuda"), "u": torch.randn(m, k, device="cuda")}
     best = None
     for r in range(6):
-        for name in ("x", "u"):
-            inst.set_input_ptr(name, dt.F32, [m, k], x.data_ptr(), True)
+        for name, t in feeds.items():
+            inst.set_input_ptr(name, dt.F32, [m, k], t.data_ptr(), True)
         torch.cuda.synchronize()
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         with torch.cuda.stream(stream):

@@ -699,6 +699,7 @@ __global__ void __launch_bounds__(FL_THREADS, LPR <= 16 ? 4 : 2) gqa_decode_flas
             __syncthreads();
             const int e = scale_exponent(s_top[0]);
             const bool hold = pairs_hold(s_top[0], s_top[1]);
+            int lossy = 0;
             const float up = exp2_int(e);
             const int64_t b = prob / p.kv_heads, h = prob % p.kv_heads;
             if (threadIdx.x == 0) p.pairs.scale[h * p.pairs.scale_pitch + b] = hold ? exp2_int(-e) : -exp2_int(-e);
@@ -711,7 +712,19 @@ __global__ void __launch_bounds__(FL_THREADS, LPR <= 16 ? 4 : 2) gqa_decode_flas
                 const __half hi = __float2half_rn(x);
                 o[i] = hi;
                 o[p.pairs.m_pad * p.pairs.k_pad + i] = __float2half_rn((x - __half2float(hi)) * SPLIT_LO);
-                if (!hold) p.pairs.full[b * p.pairs.full_ld + h * p.rows * D + i] = A[q];
+                if (!hold) {
+                    p.pairs.full[b * p.pairs.full_ld + h * p.rows * D + i] = A[q];
+                    lossy += is_lossy(x);
+                }
+            }
+            if (!hold) {  // the same in every thread
+                __syncthreads();
+                if (threadIdx.x == 0) s_top[0] = 0;
+                __syncthreads();
+                lossy = __reduce_add_sync(0xffffffffu, lossy);
+                if (lane == 0) atomicAdd(s_top, lossy);
+                __syncthreads();
+                if (threadIdx.x == 0) p.pairs.scale[p.pairs.count + h * p.pairs.scale_pitch + b] = static_cast<float>(s_top[0]);
             }
         }
     }

@@ -107,12 +107,21 @@ __device__ __forceinline__ void put_range(uint32_t mx, uint32_t mn, uint32_t* pa
 }
 template <int THREADS>
 __device__ __forceinline__ void get_range(uint32_t& mx, uint32_t& mn, const uint32_t* part_max, const uint32_t* part_min) {
-    mx = part_max[0];
-    mn = part_min[0];
-#pragma unroll
-    for (int i = 1; i < THREADS / 32; i++) {
-        mx = max(mx, part_max[i]);
-        mn = min(mn, part_min[i]);
+    const int lane = threadIdx.x & (THREADS / 32 - 1);  // (a number of warps that is a power of two)
+    mx = __reduce_max_sync(0xffffffffu, part_max[lane]);
+    mn = __reduce_min_sync(0xffffffffu, part_min[lane]);
+}
+
+// how many values of a row pairs do not hold; `part`: shared memory that every thread has read
+template <int THREADS>
+__device__ __forceinline__ void put_count(const SplitRows& d, int64_t row, int lossy, uint32_t* part) {
+    __syncthreads();
+    lossy = __reduce_add_sync(0xffffffffu, lossy);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = lossy;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 1; i < THREADS / 32; i++) lossy += part[i];
+        d.scale[d.count + row] = static_cast<float>(lossy);
     }
 }
 
@@ -223,6 +232,7 @@ __global__ void __launch_bounds__(THREADS) rmsnorm_f32_regs_kernel(int cols, flo
         scale = exp2_int(e);
         if (threadIdx.x == 0) pairs.scale[blockIdx.x] = hold ? exp2_int(-e) : -exp2_int(-e);
     }
+    int lossy = 0;
 #pragma unroll
     for (int i = 0; i < NP; i++) {
         const int c = threadIdx.x + THREADS * i;
@@ -235,12 +245,17 @@ __global__ void __launch_bounds__(THREADS) rmsnorm_f32_regs_kernel(int cols, flo
             r.w = __fmul_rn(__fdiv_rn(v[i].w, sd), g.w);
             if constexpr (PAIRS) {
                 store_pairs4(pairs, blockIdx.x, 4 * c, r, scale);
-                if (!hold) store_full4(pairs, blockIdx.x, 4 * c, r);
+                if (!hold) {
+                    store_full4(pairs, blockIdx.x, 4 * c, r);
+                    lossy += lossy4(r, scale);
+                }
             } else {
                 dst[c] = r;
             }
         }
     }
+    if constexpr (PAIRS)
+        if (!hold) put_count<THREADS>(pairs, blockIdx.x, lossy, part_max);
 }
 
 // 0.f + slab 0 + slab 1 + ... of four consecutive elements: up to eight slabs are asked for at a time, added in slab order
@@ -537,14 +552,19 @@ __global__ void __launch_bounds__(THREADS) swiglu_pairs_kernel(int cols, const f
     const float scale = exp2_int(e);
     const bool hold = pairs_hold(mx, low);
     if (threadIdx.x == 0) pairs.scale[row] = hold ? exp2_int(-e) : -exp2_int(-e);
+    int lossy = 0;
 #pragma unroll
     for (int i = 0; i < NP; i++) {
         const int c = threadIdx.x + THREADS * i;
         if (c < packs) {
             store_pairs4(pairs, row, 4 * c, a[i], scale);
-            if (!hold) store_full4(pairs, row, 4 * c, a[i]);
+            if (!hold) {
+                store_full4(pairs, row, 4 * c, a[i]);
+                lossy += lossy4(a[i], scale);
+            }
         }
     }
+    if (!hold) put_count<THREADS>(pairs, row, lossy, part_max);
 }
 
 struct MaskParams {

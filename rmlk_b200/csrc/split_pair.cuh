@@ -22,10 +22,16 @@ __device__ __forceinline__ float exp2_int(int e) { return __int_as_float((e + 12
 // Low end of a group's range: the smallest of `nonzero_low` over its values is the bits of the smallest magnitude that is not zero, less one.
 __device__ __forceinline__ uint32_t nonzero_low(float x) { return (__float_as_uint(x) & 0x7fffffffu) - 1u; }
 // Do pairs under one scale hold every value of the group?  Down to 2^-28 of the largest they keep at least 22 bits; below, a value is off by up to
-// 2^-50 of the largest.  Where not, the scale that is stored is negative, and sums that this could show in are formed again from the fp32
-// operands (umma_gemm_kernel.cuh, repair).
+// 2^-50 of the largest.  Where not, the scale that is stored is negative, the number of such values is stored as well, and sums that they could
+// show in are formed again from the fp32 operands (umma_gemm_kernel.cuh, repair).
 __device__ __forceinline__ bool pairs_hold(uint32_t max_bits, uint32_t low) {
     return low == 0xffffffffu || __uint_as_float(low + 1u) * 268435456.f >= __uint_as_float(max_bits);
+}
+
+// a scaled value that pairs do not hold to 22 bits
+__device__ __forceinline__ int is_lossy(float scaled) { return scaled != 0.f && fabsf(scaled) < 6.103515625e-5f ? 1 : 0; }  // 2^-14
+__device__ __forceinline__ int lossy4(float4 v, float scale) {
+    return is_lossy(v.x * scale) + is_lossy(v.y * scale) + is_lossy(v.z * scale) + is_lossy(v.w * scale);
 }
 
 // two scaled values -> their high and low parts

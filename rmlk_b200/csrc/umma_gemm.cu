@@ -168,6 +168,8 @@ int umma_split(cudaStream_t st, const SplitRows& x, const SplitWeights& w, float
     p.K = x.k;
     p.w_src = w.src;
     p.w_col0 = w.col0;
+    p.w_count = w.count;
+    p.x_count = x.count;
     p.x_full = x.full;
     p.x_full_ld = x.full_ld;
     p.x_full_all = x.full_all ? 1 : 0;

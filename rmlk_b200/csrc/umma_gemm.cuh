@@ -90,15 +90,16 @@ struct Params {
     const float* x_scale;    // pairs do not hold the column / the row; NULL: none
     int64_t x_scale_pitch;
     int chunk_blocks;        // k-blocks that share a row scale
+    int w_static;            // nothing in flight writes the weights: their first loads may go out before the previous kernel has finished
+    int* status;
+    // Behind what every launch reads:
     int64_t K;               // split operands as they are, for the sums that are formed again (repair): W in its sources, X as fp32 rows
     WeightSources w_src;     // (all of them, or those that pairs do not hold) and as pairs
-    int64_t w_col0;
+    int64_t w_col0, w_count, x_count;  // w_scale[w_count + ..], x_scale[x_count + ..]: how many values of a marked column, row are not held
     const float* x_full;
     int64_t x_full_ld, x_k_pad, x_low;
     int x_full_all;
     const void* x_pairs;
-    int w_static;            // nothing in flight writes the weights: their first loads may go out before the previous kernel has finished
-    int* status;
 };
 
 // CG: CTAs per tile (a pair shares one tile of 256 columns); SPLIT: operands are (high, low) pairs of f16; MT: activation rows per tile; ST: stages

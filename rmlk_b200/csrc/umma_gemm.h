@@ -32,6 +32,7 @@ struct SplitWeights {
     int64_t n, k, n_blocks, k_blocks;
     WeightSources src;  // the fp32 matrices, which have to stay: a column that pairs do not hold is read from them
     int64_t col0;       // first column of a window
+    int64_t count;      // scale[count + n]: values of a marked column that pairs do not hold, as a float
 };
 size_t split_weights_bytes(int64_t n, int64_t k);
 SplitWeights split_weights_at(void* buf, int64_t n, int64_t k);  // buf: 1 KB aligned
@@ -43,6 +44,7 @@ struct SplitRows {
     float* scale;  // [chunks][scale_pitch], negative where pairs do not hold the values of the row in the chunk
     int64_t m, k, m_pad, k_pad, scale_pitch;
     int chunk_blocks;  // blocks of 64 k that share a scale
+    int64_t count;     // scale[count + ...]: for a negative scale, the values that pairs do not hold, as a float
     float* full;       // rows of k fp32 values, full_ld apart: all of them (full_all), or those that pairs do not hold
     int64_t full_ld;
     bool full_all;

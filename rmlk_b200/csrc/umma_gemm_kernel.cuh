@@ -63,21 +63,23 @@ __device__ __forceinline__ Item item_at(int w, const Params& p) {
     return it;
 }
 
-// Pairs keep an element of a row or column to 2^-50 of its largest at worst.  With Xmax < 2^15 sx and Wmax < 2^15 sw a sum over k terms is off
-// by less than 2^-20 k sx sw through that: by 2^-21 of itself where it is 2 k sx sw or more, which ordinary sums are (they measure in the tens of
-// millions of sx sw, so that one in a million falls below).  Tiles with a marked row or column keep the smallest of their sums, chunk by chunk, as
-// they come out of TMEM, and look closer where it falls below: at the sums of the marked rows and columns.  Where one of those does - a column of a table whose largest entry no row asks for, a row whose large values meet zeros - the
-// sums that small are formed again here from the fp32 operands.  One warp, columns n of its lanes, rows m_base .. m_base + HM; behind all tiles,
-// so that nothing waits for it.
-// (Few registers: what it needs is added to what the product's kernel needs.)
+// Pairs keep an element of a row or column to 2^-50 of its largest at worst: of the lossy ones, lx in the row and lw in the column, each moves
+// a sum by less than 2^-36 2^15 sx sw (largest values are below 2^15 sx, 2^15 sw).  That is 2^-21 of the sum where it is lx + lw of sx sw or more,
+// which ordinary sums are (they measure in the tens of millions).  The smallest sum of a thread's tile is kept, chunk by chunk, as the sums come out
+// of TMEM; where a tile has a marked row or column and a sum below the line - a column of a table whose largest entry no row asks for, a row
+// whose large values meet zeros - such sums are formed again here from the fp32 operands.  One warp, columns n of its lanes, rows m_base ..
+// m_base + rows; behind all tiles, so that nothing waits for it.  (Few registers: what it needs is added to what the product's kernel needs.  A
+// look at every sum inside the epilogue cost each product 0.6 us, by its mere size.)  64 rows whose every row is marked (SwiGLU of two
+// equal operands) x [8192, 2048]: 20.0 us, 19.3 with ordinary rows; [4096,4096] x [4096,4096] with nearly every sum below the line: 31 ms, 0.35.
 __device__ __noinline__ void repair(const Params& p, int rows, int split, int64_t m_base, int64_t n) {
     constexpr int R = 4;
     const int lane = threadIdx.x & 31;
     const int kb0 = split * p.k_per_split, nk = min(p.k_per_split, p.k_blocks - kb0);
     const int k0 = kb0 * BK, k1 = static_cast<int>(min(p.K, static_cast<int64_t>(k0) + nk * BK));
+    const int c_first = p.x_scale_pitch ? kb0 / p.chunk_blocks : 0, c_last = p.x_scale_pitch ? (kb0 + nk - 1) / p.chunk_blocks : 0;
     const bool in = n < p.N;
     const float ws = in ? p.w_scale[n] : 1.f;
-    const bool any_col = __any_sync(0xffffffffu, in && ws < 0.f);
+    const float lw = in && ws < 0.f ? fminf(p.w_scale[p.w_count + n], static_cast<float>(k1 - k0)) : 0.f;
     float* out = static_cast<float*>(p.out) + (p.ksplit > 1 ? static_cast<int64_t>(split) * p.M * p.N : 0) + n;
     const float* w = nullptr;  // column n of W in fp32, ldw apart
     int64_t ldw = 0;
@@ -88,7 +90,7 @@ __device__ __noinline__ void repair(const Params& p, int rows, int split, int64_
         w = p.w_src.w[j] + c - p.w_src.col0[j];
         ldw = p.w_src.n[j];
     }
-    auto chunk_at = [&](int k) { return k / BK / p.chunk_blocks * p.x_scale_pitch; };
+    auto chunk_at = [&](int k) { return p.x_scale_pitch ? k / BK / p.chunk_blocks * p.x_scale_pitch : 0; };
     auto x_at = [&](int64_t m, int k, int64_t chunk) {
         const float s = p.x_scale[chunk + m];
         if (p.x_full_all || s < 0.f) return p.x_full[m * p.x_full_ld + k];
@@ -96,26 +98,38 @@ __device__ __noinline__ void repair(const Params& p, int rows, int split, int64_
         return fmaf(__half2float(h[p.x_low]), 1.f / LO_SCALE, __half2float(h[0])) * s;
     };
     rows = static_cast<int>(min(static_cast<int64_t>(rows), p.M - m_base));
+    uint64_t which = 0;  // rows to look at: the marked ones, or all of them where the column of a lane is marked
+    const bool any_col = __any_sync(0xffffffffu, lw > 0.f);
+    for (int h = 0; h < 64; h += 32) {
+        bool marked = false;
+        if (h + lane < rows)
+            for (int c = c_first; c <= c_last; c++) marked = marked || any_col || p.x_scale[c * p.x_scale_pitch + m_base + h + lane] < 0.f;
+        which |= static_cast<uint64_t>(__ballot_sync(0xffffffffu, marked)) << h;
+    }
 #pragma unroll 1
     for (int j0 = 0; j0 < rows; j0 += R) {
+        if ((which >> j0 & 15) == 0) continue;
+        float v[R], most[R], lx[R];
+#pragma unroll
+        for (int j = 0; j < R; j++) {
+            most[j] = lx[j] = 0.f;
+            v[j] = in && j0 + j < rows ? out[(m_base + j0 + j) * p.ldc] : 0.f;
+        }
+#pragma unroll 1
+        for (int c = c_first; c <= c_last; c++) {
+#pragma unroll
+            for (int j = 0; j < R; j++) {
+                const int64_t at = c * p.x_scale_pitch + m_base + min(j0 + j, rows - 1);
+                const float s = p.x_scale[at];
+                most[j] = fmaxf(most[j], fabsf(s));
+                if (s < 0.f) lx[j] -= s * fminf(p.x_scale[p.x_count + at], static_cast<float>(k1 - k0));
+            }
+        }
         uint32_t lanes[R];
         int total = 0;
 #pragma unroll
         for (int j = 0; j < R; j++) {
-            lanes[j] = 0;
-            if (j0 + j >= rows) continue;
-            const int64_t m = m_base + j0 + j;
-            float most = 0.f;
-            bool wide = any_col;
-#pragma unroll 1
-            for (int c = kb0 / p.chunk_blocks; c <= (kb0 + nk - 1) / p.chunk_blocks; c++) {
-                const float s = p.x_scale[c * p.x_scale_pitch + m];
-                most = fmaxf(most, fabsf(s));
-                wide = wide || s < 0.f;
-            }
-            if (!wide) continue;
-            const float v = in ? out[m * p.ldc] : 0.f;
-            lanes[j] = __ballot_sync(0xffffffffu, in && fabsf(v) < 2.f * static_cast<float>(k1 - k0) * most * fabsf(ws));
+            lanes[j] = __ballot_sync(0xffffffffu, in && j0 + j < rows && fabsf(v[j]) < (lx[j] + lw * most[j]) * fabsf(ws));
             total += __popc(lanes[j]);
         }
         if (total == 0) continue;
@@ -128,7 +142,7 @@ __device__ __noinline__ void repair(const Params& p, int rows, int split, int64_
                     const float* wl = reinterpret_cast<const float*>(__shfl_sync(0xffffffffu, reinterpret_cast<uint64_t>(w), l));
                     const int64_t ld = __shfl_sync(0xffffffffu, ldw, l);
                     float sum = 0.f;
-#pragma unroll 2
+#pragma unroll 4
                     for (int k = k0 + lane; k < k1; k += 32) sum = fmaf(x_at(m, k, chunk_at(k)), wl[k * ld], sum);
 #pragma unroll
                     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
@@ -142,7 +156,7 @@ __device__ __noinline__ void repair(const Params& p, int rows, int split, int64_
         int k = k0;
         if (p.x_full_all) {
             const float* x = p.x_full + (m_base + j0) * p.x_full_ld;
-            const int64_t last = rows - 1 - j0;
+            const int64_t last = p.M - 1 - (m_base + j0);
 #pragma unroll 1
             for (; k + 4 <= k1; k += 4) {
                 float wv[4];
@@ -351,7 +365,8 @@ __global__ void __launch_bounds__(Layout<CG, SPLIT, MT, ST>::REGS_FOR, 1) gemm_k
         dep_wait();  // scales and outputs may belong to kernels before this one
         int buf = 0;
         uint32_t acc_phase = 0;
-        bool ok = true, again = false;  // again: a sum of this thread has to be formed again (repair)
+        bool ok = true;
+        int again_at = -1;  // tile with sums that have to be formed again (repair), -2: several
         for (int w = first; w < items && ok; w += stride) {
             const Item it = item_at(w, p);
             const int kb0 = it.split * p.k_per_split, nk = min(p.k_per_split, p.k_blocks - kb0);
@@ -377,7 +392,7 @@ __global__ void __launch_bounds__(Layout<CG, SPLIT, MT, ST>::REGS_FOR, 1) gemm_k
                 if constexpr (SPLIT) {
                     if (4 * lane < HM) {
                         s4 = __ldg(reinterpret_cast<const float4*>(p.x_scale + c * p.x_scale_pitch + m_base) + lane);
-                        const int64_t left = p.M - m_base - 4 * lane;  // (what lies behind the last row is no scale)
+                        const int left = static_cast<int>(p.M - m_base) - 4 * lane;  // (what lies behind the last row is no scale)
                         row_marked = row_marked || (s4.x < 0.f && left > 0) || (s4.y < 0.f && left > 1) || (s4.z < 0.f && left > 2) || (s4.w < 0.f && left > 3);
                     }
                 }
@@ -432,17 +447,17 @@ __global__ void __launch_bounds__(Layout<CG, SPLIT, MT, ST>::REGS_FOR, 1) gemm_k
             if (!ok) break;
             if constexpr (SPLIT && ONE_CHUNK) ws = in ? fabsf(__ldg(p.w_scale + n)) : 0.f;
             if constexpr (SPLIT) {
-                const float least = 2.f * BK * min(p.chunk_blocks, nk);
-                if (__any_sync(0xffffffffu, col_marked || row_marked) && __any_sync(0xffffffffu, in && low < least)) {
-                    if (c_first < c_last) {
-                        again = true;
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < HM; j++) {
-                            const float xs = row_scale(j);
-                            again = again || (in && m_base + j < p.M && (col_marked || xs < 0.f) && fabsf(acc[j]) < (ONE_CHUNK ? least : least * fabsf(xs) * ws));
-                        }
+                if (__any_sync(0xffffffffu, col_marked || row_marked)) {
+                    const float all = static_cast<float>(BK * min(p.chunk_blocks, nk));
+                    float line = c_first < c_last ? all : 0.f;
+                    if (row_marked && c_first == c_last) {
+                        const float* count = p.x_scale + p.x_count + c_first * p.x_scale_pitch + m_base + 4 * lane;
+                        line = fmaxf(fmaxf(s4.x < 0.f ? count[0] : 0.f, s4.y < 0.f ? count[1] : 0.f), fmaxf(s4.z < 0.f ? count[2] : 0.f, s4.w < 0.f ? count[3] : 0.f));
+                        line = fminf(fmaxf(line, 1.f), all);
                     }
+                    line = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(line)));
+                    if (col_marked) line += fminf(p.w_scale[p.w_count + n], all);
+                    if (__any_sync(0xffffffffu, in && low < line)) again_at = again_at == -1 ? w : -2;
                 }
             }
             using Out = typename std::conditional<OUT16, __half, float>::type;
@@ -461,11 +476,12 @@ __global__ void __launch_bounds__(Layout<CG, SPLIT, MT, ST>::REGS_FOR, 1) gemm_k
             }
         }
         if constexpr (SPLIT)
-            if (ok && __any_sync(0xffffffffu, again))
-                for (int w = first; w < items; w += stride) {
+            if (ok && again_at != -1) {
+                for (int w = again_at >= 0 ? again_at : first; w < items; w = again_at >= 0 ? items : w + stride) {
                     const Item it = item_at(w, p);
                     repair(p, HM, it.split, static_cast<int64_t>(it.m_tile) * MT + part * HM, (static_cast<int64_t>(it.n_tile) * CG + rank) * BN + sub * 32 + lane);
                 }
+            }
     }
     tc_fence_before();
     if constexpr (CG == 2) cluster_sync_all();  // no CTA of the pair leaves while the other may still signal its barriers or read its tiles

@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(256) column_range_kernel(WeightSources s, int6
 
 // Grid: blocks of 128 columns x blocks of 64 rows.
 __global__ void __launch_bounds__(256) pack_weights_kernel(WeightSources s, int64_t K, const uint32_t* __restrict__ colmax, const uint32_t* __restrict__ collow,
-                                                           uint8_t* __restrict__ tiles, float* __restrict__ w_scale) {
+                                                           float* __restrict__ colcount, uint8_t* __restrict__ tiles, float* __restrict__ w_scale) {
     dep_sync();
     const int c8 = threadIdx.x & 15, r0 = threadIdx.x >> 4;
     const int64_t nb = blockIdx.x, n0 = nb * 128 + c8 * 8;
@@ -92,9 +92,12 @@ __global__ void __launch_bounds__(256) pack_weights_kernel(WeightSources s, int6
     int e[8];
 #pragma unroll
     for (int i = 0; i < 8; i++) e[i] = scale_exponent(colmax[n0 + i]);
+    uint32_t marked = 0;
+#pragma unroll
+    for (int i = 0; i < 8; i++) marked |= pairs_hold(colmax[n0 + i], ~collow[n0 + i]) ? 0u : 1u << i;
     if (kb == 0 && r0 == 0) {
 #pragma unroll
-        for (int i = 0; i < 8; i++) w_scale[n0 + i] = pairs_hold(colmax[n0 + i], ~collow[n0 + i]) ? exp2_int(-e[i]) : -exp2_int(-e[i]);
+        for (int i = 0; i < 8; i++) w_scale[n0 + i] = marked >> i & 1 ? -exp2_int(-e[i]) : exp2_int(-e[i]);
     }
 #pragma unroll
     for (int p = 0; p < 4; p++) {
@@ -109,6 +112,11 @@ __global__ void __launch_bounds__(256) pack_weights_kernel(WeightSources s, int6
         }
 #pragma unroll
         for (int i = 0; i < 8; i++) x[i] *= exp2_int(e[i]);
+        if (marked) {
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+                if ((marked >> i & 1) && is_lossy(x[i])) atomicAdd(colcount + n0 + i, 1.f);
+        }
         uint4 hi, lo;
         split8(x, 1.f, hi, lo);
         const uint32_t off = (c8 >> 3) * 8192 + r * 128 + (((c8 & 7) ^ (r & 7)) << 4);
@@ -119,7 +127,7 @@ __global__ void __launch_bounds__(256) pack_weights_kernel(WeightSources s, int6
 
 // One CTA per row: its largest magnitude, then both parts.  A row is read twice, the second time from L1 / L2.
 __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ x, int64_t ldx, int64_t K, int64_t k_pad, int64_t m_pad, __half* __restrict__ out,
-                                                         float* __restrict__ x_scale, int vec) {
+                                                         float* __restrict__ x_scale, int64_t count, int vec) {
     dep_sync();
     __shared__ uint32_t sm, sl;
     const int64_t m = blockIdx.x;
@@ -151,7 +159,9 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict
     __syncthreads();
     const int e = scale_exponent(sm);
     const float scale = exp2_int(e);
-    if (threadIdx.x == 0) x_scale[m] = pairs_hold(sm, sl) ? exp2_int(-e) : -exp2_int(-e);
+    const bool hold = pairs_hold(sm, sl);
+    if (threadIdx.x == 0) x_scale[m] = hold ? exp2_int(-e) : -exp2_int(-e);
+    int lossy = 0;
     __half* hrow = out + m * k_pad;
     __half* lrow = hrow + m_pad * k_pad;
     for (int64_t k = threadIdx.x * 8; k < k_pad; k += 2048) {
@@ -168,6 +178,19 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict
         split8(v, scale, hi, lo);
         *reinterpret_cast<uint4*>(hrow + k) = hi;
         *reinterpret_cast<uint4*>(lrow + k) = lo;
+        if (!hold) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) lossy += is_lossy(v[i] * scale);
+        }
+    }
+    if (!hold) {  // the same in every thread
+        __shared__ int total;
+        if (threadIdx.x == 0) total = 0;
+        __syncthreads();
+        lossy = __reduce_add_sync(0xffffffffu, lossy);
+        if ((threadIdx.x & 31) == 0) atomicAdd(&total, lossy);
+        __syncthreads();
+        if (threadIdx.x == 0) x_scale[count + m] = static_cast<float>(total);
     }
 }
 
@@ -177,7 +200,7 @@ static int64_t pad_to(int64_t v, int64_t a) { return (v + a - 1) / a * a; }
 
 size_t split_weights_bytes(int64_t n, int64_t k) {
     const int64_t nb = ceil_div64(n, 128), kb = ceil_div64(k, 64);
-    return static_cast<size_t>(nb) * kb * 32768 + static_cast<size_t>(nb) * 128 * 12;
+    return static_cast<size_t>(nb) * kb * 32768 + static_cast<size_t>(nb) * 128 * 16;
 }
 
 SplitWeights split_weights_at(void* buf, int64_t n, int64_t k) {
@@ -188,6 +211,7 @@ SplitWeights split_weights_at(void* buf, int64_t n, int64_t k) {
     w.k_blocks = ceil_div64(k, 64);
     w.tiles = buf;
     w.scale = reinterpret_cast<float*>(static_cast<char*>(buf) + static_cast<size_t>(w.n_blocks) * w.k_blocks * 32768);
+    w.count = 3 * w.n_blocks * 128;
     return w;
 }
 
@@ -206,7 +230,7 @@ int split_weights_pack(cudaStream_t st, const WeightSources& src, SplitWeights& 
     w.src = src;
     uint32_t* colmax = reinterpret_cast<uint32_t*>(w.scale + w.n_blocks * 128);
     uint32_t* collow = colmax + w.n_blocks * 128;
-    RMLK_CUDA(cudaMemsetAsync(colmax, 0, static_cast<size_t>(w.n_blocks) * 1024, st));
+    RMLK_CUDA(cudaMemsetAsync(colmax, 0, static_cast<size_t>(w.n_blocks) * 1536, st));
     // about 8 CTAs per SM
     int64_t ranges = std::max<int64_t>(1, std::min<int64_t>(ceil_div64(8ll * sm_count(), w.n_blocks), ceil_div64(w.k, 64)));
     const int64_t rows = ceil_div64(w.k, ranges);
@@ -214,7 +238,7 @@ int split_weights_pack(cudaStream_t st, const WeightSources& src, SplitWeights& 
     launch_dep(umma::column_range_kernel, dim3(static_cast<unsigned>(w.n_blocks), static_cast<unsigned>(ranges)), dim3(256), 0, st, src, w.k, rows, colmax, collow);
     RMLK_CHECK_LAUNCH("column_range_kernel");
     launch_dep(umma::pack_weights_kernel, dim3(static_cast<unsigned>(w.n_blocks), static_cast<unsigned>(w.k_blocks)), dim3(256), 0, st, src, w.k,
-               static_cast<const uint32_t*>(colmax), static_cast<const uint32_t*>(collow), static_cast<uint8_t*>(w.tiles), w.scale);
+               static_cast<const uint32_t*>(colmax), static_cast<const uint32_t*>(collow), w.scale + w.count, static_cast<uint8_t*>(w.tiles), w.scale);
     RMLK_CHECK_LAUNCH("pack_weights_kernel");
     return RMLK_OK;
 }
@@ -229,8 +253,9 @@ SplitRows split_rows_at(void* buf, int64_t m, int64_t k, int chunk_blocks, bool 
     x.scale_pitch = x.m_pad + 256;  // a tile of up to 256 rows may read scales behind the last row
     x.data = buf;
     x.scale = reinterpret_cast<float*>(static_cast<char*>(buf) + static_cast<size_t>(x.m_pad) * x.k_pad * 4);
+    x.count = ceil_div64(x.k_pad / 64, x.chunk_blocks) * x.scale_pitch;
     if (keep_full) {
-        x.full = x.scale + ceil_div64(x.k_pad / 64, x.chunk_blocks) * x.scale_pitch;
+        x.full = x.scale + 2 * x.count;
         x.full_ld = k;
     }
     return x;
@@ -238,7 +263,7 @@ SplitRows split_rows_at(void* buf, int64_t m, int64_t k, int chunk_blocks, bool 
 
 size_t split_rows_bytes(int64_t m, int64_t k, int chunk_blocks, bool keep_full) {
     const SplitRows x = split_rows_at(nullptr, m, k, chunk_blocks, keep_full);
-    return static_cast<size_t>(x.m_pad) * x.k_pad * 4 + static_cast<size_t>(ceil_div64(x.k_pad / 64, x.chunk_blocks)) * x.scale_pitch * 4 +
+    return static_cast<size_t>(x.m_pad) * x.k_pad * 4 + static_cast<size_t>(x.count) * 8 +
            (keep_full ? static_cast<size_t>(m) * k * 4 : 0);
 }
 
@@ -249,7 +274,7 @@ int split_rows_pack(cudaStream_t st, const float* x, int64_t ldx, SplitRows& dst
     if (dst.m > 0x7fffffffll) return fail(RMLK_ERR_INVALID_ARG, "matmul: too many rows");
     const int vec = aligned_to(x, 16) && ldx % 4 == 0 && dst.k % 4 == 0;
     launch_dep(umma::split_rows_kernel, dim3(static_cast<unsigned>(dst.m)), dim3(256), 0, st, x, ldx, dst.k, dst.k_pad, dst.m_pad, static_cast<__half*>(dst.data),
-               dst.scale, vec);
+               dst.scale, dst.count, vec);
     RMLK_CHECK_LAUNCH("split_rows_kernel");
     return RMLK_OK;
 }
