@@ -153,6 +153,8 @@ def _setup(l):
     l.rmlk_instance_value_info.argtypes = [ctypes.c_void_p, ctypes.c_char_p, ctypes.c_void_p, ctypes.c_void_p,
                                            ctypes.c_void_p, ctypes.c_void_p]
     l.rmlk_instance_read.argtypes = [ctypes.c_void_p, ctypes.c_char_p, ctypes.c_void_p, ctypes.c_size_t]
+    l.rmlk_instance_stream_output.argtypes = [ctypes.c_void_p, ctypes.c_char_p, ctypes.c_void_p, ctypes.c_size_t]
+    l.rmlk_instance_wait_outputs.argtypes = [ctypes.c_void_p]
     l._rt_ready = True
     return l
 

@@ -37,3 +37,14 @@ def test_dims_of_any_integer_type():
     for make in (runtime._i64, kernels._i64):
         for dims in ([], [3], (2, 5), list(range(12)), np.arange(4), [np.int32(7), 2], torch.Size([4, 6]), [torch.tensor(9), 1], [True, 2.0]):
             assert list(make(dims))[: len(dims)] == [int(v) for v in dims]
+
+
+def test_every_handle_is_passed_whole():
+    """ctypes cuts an int argument of a function without argtypes to 32 bits: a handle that lies higher would arrive broken."""
+    import inspect
+    from rmlk_b200 import runtime
+    library = runtime._rt()
+    names = set(re.findall(r"\.(rmlk_(?:graph|instance)_\w+)\(", inspect.getsource(runtime)))
+    assert "rmlk_instance_stream_output" in names
+    for name in names - {"rmlk_graph_create"}:
+        assert getattr(library, name).argtypes, name
