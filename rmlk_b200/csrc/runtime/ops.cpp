@@ -2013,8 +2013,8 @@ static rmlk_batch_job rope_job(const Shape& oshape, const int64_t* xstr, const i
 // Several tokens: the one-launch kernel or the single operators.  The kernel gives a CTA 128 query rows of a KV head (`rows` in all) and walks its
 // keys 64 at a time, 5 us each, however few CTAs there are; the single operators use every SM, and up to 16 rows they stream the
 // keys.  Measured on 2 to 32 KV heads, 1 to 16 requests, 2 to 192 tokens behind 64 to 8192 keys of 64, kernel against single operators: 8 KV heads of 4
-// query heads, 2 tokens, 4096 keys 359 against 55 us; 16 tokens, 2048 keys 189 / 136; 16 requests of 16 tokens, 2048 keys 222 / 557; one prompt of
-// 256 tokens 112 / 150.  With the line below 15 of some 2400 sizes are slower than the single operators by more than 5 % (worst 331 / 229), and the
+// query heads, 2 tokens, 4096 keys 359 against 55 us; 16 tokens, 2048 keys 189 / 136; 16 requests of 16 tokens, 2048 keys 357 / 682; 192 tokens,
+// 256 keys 42 / 58.  With the line below 15 of some 2400 sizes are slower than the single operators by more than 5 % (worst 331 / 229), and the
 // sizes left to these cost 2 % on average.
 static bool prompt_attention_pays(int64_t problems, int64_t rows, int64_t keys) {
     const int64_t all = problems * rows;
