@@ -70,7 +70,7 @@ __device__ __forceinline__ Item item_at(int w, const Params& p) {
 // whose large values meet zeros - such sums are formed again here from the fp32 operands.  One warp, columns n of its lanes, rows m_base ..
 // m_base + rows; behind all tiles, so that nothing waits for it.  (Few registers: what it needs is added to what the product's kernel needs.  A
 // look at every sum inside the epilogue cost each product 0.6 us, by its mere size.)  64 rows whose every row is marked (SwiGLU of two
-// equal operands) x [8192, 2048]: 20.0 us, 19.3 with ordinary rows; [4096,4096] x [4096,4096] with nearly every sum below the line: 31 ms, 0.35.
+// equal operands) x [8192, 2048]: 20.0 us, 19.6 with ordinary rows; [4096,4096] x [4096,4096] with nearly every sum below the line: 31 ms, 0.35.
 __device__ __noinline__ void repair(const Params& p, int rows, int split, int64_t m_base, int64_t n) {
     constexpr int R = 4;
     const int lane = threadIdx.x & 31;
@@ -373,7 +373,7 @@ __global__ void __launch_bounds__(Layout<CG, SPLIT, MT, ST>::REGS_FOR, 1) gemm_k
             const int64_t n = (static_cast<int64_t>(it.n_tile) * CG + rank) * BN + sub * 32 + lane;
             const bool in = n < p.N;
             float ws = 0.f;
-            float low = INFINITY;       // smallest sum over a chunk, rows behind the last one among them
+            float low = INFINITY;       // smallest sum over a chunk
             bool col_marked = false, row_marked = false;  // this column; one of the tile's rows that this lane has the scale of
             if constexpr (SPLIT) {
                 const float w_scale = in ? __ldg(p.w_scale + n) : 0.f;
@@ -381,6 +381,7 @@ __global__ void __launch_bounds__(Layout<CG, SPLIT, MT, ST>::REGS_FOR, 1) gemm_k
                 if constexpr (!ONE_CHUNK) ws = fabsf(w_scale);
             }
             const int64_t m_base = static_cast<int64_t>(it.m_tile) * MT + part * HM;
+            const int valid = static_cast<int>(min(static_cast<int64_t>(HM), p.M - m_base));  // rows of this warp (what lies behind them is no data)
             float acc[HM];
             float4 s4 = make_float4(0.f, 0.f, 0.f, 0.f);
             auto row_scale = [&](int j) {
@@ -392,8 +393,9 @@ __global__ void __launch_bounds__(Layout<CG, SPLIT, MT, ST>::REGS_FOR, 1) gemm_k
                 if constexpr (SPLIT) {
                     if (4 * lane < HM) {
                         s4 = __ldg(reinterpret_cast<const float4*>(p.x_scale + c * p.x_scale_pitch + m_base) + lane);
-                        const int left = static_cast<int>(p.M - m_base) - 4 * lane;  // (what lies behind the last row is no scale)
-                        row_marked = row_marked || (s4.x < 0.f && left > 0) || (s4.y < 0.f && left > 1) || (s4.z < 0.f && left > 2) || (s4.w < 0.f && left > 3);
+                        const int left = valid - 4 * lane;
+                        if (left < 4) s4 = make_float4(left > 0 ? s4.x : 1.f, left > 1 ? s4.y : 1.f, left > 2 ? s4.z : 1.f, 1.f);
+                        row_marked = row_marked || fminf(fminf(s4.x, s4.y), fminf(s4.z, s4.w)) < 0.f;
                     }
                 }
                 ok = __all_sync(0xffffffffu, mbar_wait(acc_full(buf), acc_phase, abort_flag, p.status));  // (one lane's limit may run out before another's)
@@ -413,7 +415,7 @@ __global__ void __launch_bounds__(Layout<CG, SPLIT, MT, ST>::REGS_FOR, 1) gemm_k
 #pragma unroll
                             for (int j = 0; j < STEP; j++) {
                                 acc[j0 + j] = add_low(acc[j0 + j], __uint_as_float(q[j]));
-                                low = fminf(low, fabsf(acc[j0 + j]));
+                                if (j0 + j < valid) low = fminf(low, fabsf(acc[j0 + j]));
                             }
                         }
                     }
@@ -427,7 +429,7 @@ __global__ void __launch_bounds__(Layout<CG, SPLIT, MT, ST>::REGS_FOR, 1) gemm_k
 #pragma unroll
                         for (int j = 0; j < STEP; j++) {
                             float v = add_low(__uint_as_float(r[j]), __uint_as_float(q[j]));
-                            low = fminf(low, fabsf(v));
+                            if (j0 + j < valid) low = fminf(low, fabsf(v));
                             v = unscale(v, fabsf(row_scale(j0 + j)), ws);
                             acc[j0 + j] = c == c_first ? v : acc[j0 + j] + v;
                         }
